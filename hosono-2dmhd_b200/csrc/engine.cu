@@ -132,6 +132,16 @@ class Engine::Rec {
         if (r != cudaSuccess) return e_->fail(HOSONO_ECUDA, "conditional handle: %s", cudaGetErrorString(r));
         return HOSONO_OK;
     }
+    // IF(flag) body.  Eager: the host reads the flag the preceding kernel wrote.
+    template <class Body>
+    int branch(cudaGraphConditionalHandle h, int BatchFlags::*field, Body&& body) {
+        if (!g_) {
+            TRYE(e_->sync());
+            afterKernel_ = false;
+            return e_->h_flags_->*field ? body(*this) : HOSONO_OK;
+        }
+        return node(h, cudaGraphCondTypeIf, body);
+    }
     // WHILE(flag) body.  Eager: the host reads the flag the preceding
     // condition kernel wrote.  Graph: a conditional WHILE node.
     template <class Body>
@@ -147,11 +157,24 @@ class Engine::Rec {
             }
             return HOSONO_OK;
         }
+        return node(h, cudaGraphCondTypeWhile, body);
+    }
+    template <class H>
+    int host(H&& h) {
+        if (g_) return HOSONO_OK;
+        TRYE(e_->sync());
+        afterKernel_ = false;  // h may queue copies
+        return h();
+    }
+
+  private:
+    template <class Body>
+    int node(cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, Body&& body) {
         TRYE(end());
         cudaGraphNodeParams p = {};
         p.type = cudaGraphNodeTypeConditional;
         p.conditional.handle = h;
-        p.conditional.type = cudaGraphCondTypeWhile;
+        p.conditional.type = type;
         p.conditional.size = 1;
         cudaGraphNode_t node;
         cudaError_t r = cudaGraphAddNode(&node, g_, deps_.empty() ? nullptr : deps_.data(), deps_.size(), &p);
@@ -163,15 +186,6 @@ class Engine::Rec {
         afterKernel_ = false;
         return HOSONO_OK;
     }
-    template <class H>
-    int host(H&& h) {
-        if (g_) return HOSONO_OK;
-        TRYE(e_->sync());
-        afterKernel_ = false;  // h may queue copies
-        return h();
-    }
-
-  private:
     Engine* e_;
     cudaGraph_t g_;
     std::vector<cudaGraphNode_t> deps_;
@@ -402,7 +416,8 @@ int Engine::autotune(int trials, bool force, hosono_tune_report* rep) {
         {
             const hosono_tuning t = cands[c];
             tune_ = t;
-            const Batch B = batch();
+            Batch B = batch();
+            B.p1Init = 0;  // the instances are between steps: their scheme stays
             float ms = 0.f;
             for (int k = 0; k <= trials; k++) {
                 if (k == 1) cudaEventRecord(e0, s_);
@@ -449,6 +464,8 @@ Batch Engine::batch() const {
     B.p1Radii = radii_;
     B.p1First = 0;
     B.p1End = INT_MAX;
+    B.p1Init = 1;
+    B.mcMax = trace || tune_.later_passes == HOSONO_LATER_PERSISTENT ? -1 : kClusterCells;
     B.ctStaged = tune_.update_staging == HOSONO_STAGE_TMA ? 1 : 0;
     B.dev = d_dev_;
     B.st = d_st_;
@@ -644,8 +661,8 @@ int Engine::add(const hosono_params& p, const double* pv, const double* qw, int*
     sl.dev.scheme[0] = (int8_t*)b;
     sl.dev.scheme[1] = (int8_t*)(b + plane);
     b += 2 * plane;
-    uint8_t** bp[] = {&sl.dev.rec, &sl.dev.recF, &sl.dev.rrRec, &sl.dev.fail, &sl.dev.failX,
-                      &sl.dev.failY, &sl.dev.nextPass, &sl.dev.dirty, &sl.dev.lowered, &sl.dev.innerCount,
+    uint8_t** bp[] = {&sl.dev.rec, &sl.dev.recF, &sl.dev.rrRec, &sl.dev.fail, &sl.dev.recB,
+                      &sl.dev.recFB, &sl.dev.nextPass, &sl.dev.dirty, &sl.dev.lowered, &sl.dev.innerCount,
                       &sl.dev.detMask};
     for (uint8_t** pp : bp) {
         *pp = b;
@@ -783,8 +800,6 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     CUE(cudaStreamWaitEvent(sCopy_, bandEv_[HOSONO_UPLOAD_BANDS_MAX], 0));
     const size_t rowBytes = (size_t)G.nxt * NCONS * sizeof(double), rowDoubles = (size_t)G.nxt * NCONS;
     const Batch B = batch();
-    K_->stage_init(B, s_);
-    launches++;
     const int base = instTiles_[slot].x;
     // band by band: the copy on sCopy_, then on the main stream the wait,
     // the conversion and pass 1 on the band's tile rows.  Interleaved, so
@@ -800,7 +815,7 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
         CUE(cudaEventRecord(bandEv_[b], sCopy_));
         CUE(cudaStreamWaitEvent(s_, bandEv_[b], 0));
         launch_aos_to_soa_rows(G, staging_, sl.dev.U[st.parity], NCONS, r0, r1, s_);
-        if (b > 0) CUE(cudaMemsetAsync(d_flags_->p1Next, 0, sizeof d_flags_->p1Next, s_));
+        CUE(cudaMemsetAsync(d_flags_->p1Next, 0, sizeof d_flags_->p1Next, s_));
         Batch Bb = B;
         Bb.p1First = base + tr0 * tilesPerRow;
         Bb.p1End = base + tr1 * tilesPerRow;
@@ -941,16 +956,15 @@ int Engine::record_stage(Rec& r, int uin, int uout, cudaEvent_t ev0, cudaEvent_t
     const Batch B = batch();
     const KernelSet* K = K_;
     const long long cap = (long long)INT_MAX;
+    // the cluster kernels are left out where the host looks at every pass (the
+    // trace) and where the persistent form of the later passes is asked for
+    const bool chainOnly = B.mcMax < 0;
     if (head) {
-        TRYE(r.k([&](cudaStream_t s) { K->stage_init(B, s); }));
         if (ev0) TRYE(r.event(ev0));
         TRYE(r.k([&](cudaStream_t s) { K->face_pass1(B, uin, s); }));
         if (!r.graph()) launches += radii_held() - 1;  // one pass-1 kernel per radius held
         if (ev1) TRYE(r.event(ev1));
     }
-    cudaGraphConditionalHandle hc1, hm;
-    TRYE(r.cond(&hc1, 0));
-    TRYE(r.k([&](cudaStream_t s) { K->cascade_cond(B, hc1, s); }));
     auto cascade_body = [&](cudaGraphConditionalHandle hc, int later) {
         return [&, hc, later](Rec& c) -> int {
             TRYE(c.k([&](cudaStream_t s) { K->cascade_lower(B, later, s); }));
@@ -960,19 +974,42 @@ int Engine::record_stage(Rec& r, int uin, int uout, cudaEvent_t ev0, cudaEvent_t
             return HOSONO_OK;
         };
     };
-    TRYE(r.loop(hc1, &BatchFlags::anyFail, cap, cascade_body(hc1, 0)));
-    TRYE(r.k([&](cudaStream_t s) { K->compact_dirty(B, s); }));
-    TRYE(r.k([&](cudaStream_t s) { K->flux_list(B, uin, s); }));
+    cudaGraphConditionalHandle ha;
+    TRYE(r.cond(&ha, 0));
+    TRYE(r.k([&](cudaStream_t s) { K->mood_faces(B, uin, ha, s); }));
+    TRYE(r.branch(ha, &BatchFlags::anyCasc, [&](Rec& b) -> int {
+        cudaGraphConditionalHandle hc1;
+        TRYE(b.cond(&hc1, 0));
+        TRYE(b.k([&](cudaStream_t s) { K->cascade_cond(B, hc1, s); }));
+        TRYE(b.loop(hc1, &BatchFlags::anyFail, cap, cascade_body(hc1, 0)));
+        TRYE(b.k([&](cudaStream_t s) { K->compact_dirty(B, s); }));
+        TRYE(b.k([&](cudaStream_t s) { K->flux_list(B, uin, s); }));
+        return HOSONO_OK;
+    }));
     TRYE(r.k([&](cudaStream_t s) { K->ct_update_detect(B, uin, uout, s); }));
+    if (chainOnly) return record_chain(r, B, uin, uout, cascade_body);
+    cudaGraphConditionalHandle hb;
+    TRYE(r.cond(&hb, 0));
+    TRYE(r.k([&](cudaStream_t s) { K->mood_passes(B, uin, uout, hb, s); }));
+    return r.branch(hb, &BatchFlags::anyMood, [&](Rec& b) -> int { return record_chain(b, B, uin, uout, cascade_body); });
+}
+
+// The end of pass 1 and the later MOOD passes as a chain of grid-wide
+// kernels, for the instances the cluster kernels left (InstState::big).
+template <class Cascade>
+int Engine::record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cascade_body) {
+    const KernelSet* K = K_;
+    const long long cap = (long long)INT_MAX;
     TRYE(r.k([&](cudaStream_t s) { K->mood_flags(B, MOOD_FLAGS_DENSE, s); }));
     if (trace) TRYE(r.host([&] { return trace_snapshot(); }));
-    TRYE(r.k([&](cudaStream_t s) { K->clear_low(B, s); }));
+    TRYE(r.k([&](cudaStream_t s) { K->clear_low_pass1(B, s); }));
     if (tune_.later_passes == HOSONO_LATER_PERSISTENT && !trace) {
         // the later passes as one persistent launch (it reads anyActive itself)
         TRYE(r.k([&](cudaStream_t s) { K->pass_end(B, 0, 1, s); }));
         TRYE(r.k([&](cudaStream_t s) { K->mood_rest(B, uin, uout, s); }));
         return HOSONO_OK;
     }
+    cudaGraphConditionalHandle hm;
     TRYE(r.cond(&hm, 0));
     TRYE(r.k([&](cudaStream_t s) { K->pass_end(B, hm, 1, s); }));
     if (trace) TRYE(r.host([&] { return trace_after_pass(); }));

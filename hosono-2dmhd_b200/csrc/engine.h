@@ -53,10 +53,10 @@ struct InstDev {
     int8_t* scheme[2];  // double-buffered MOOD scheme (GP radius per cell)
     uint8_t* rec;       // blk%recompute
     uint8_t* recF;      // blk%recomputeFLICD
+    uint8_t* recB;      // second recompute / recomputeFLICD planes of the cluster form of the later
+    uint8_t* recFB;     // passes (a pass reads one pair, its flag rebuild sets the other)
     uint8_t* rrRec;     // radius each face was last reconstructed at (2 bits x 4 faces)
-    uint8_t* fail;      // cell failed face CAD/PAD (inner cascade)
-    uint8_t* failX;     // bit0: E side of (i-1,j) failed, bit1: W side of (i,j)
-    uint8_t* failY;     // bit0: N side of (i,j-1) failed, bit1: S side of (i,j)
+    uint8_t* fail;      // cell failed face CAD/PAD (pass 1, inner cascade)
     uint8_t* nextPass;  // reconstructNextPass
     uint8_t* dirty;     // re-reconstructed by the pass-1 cascade
     uint8_t* lowered;   // lowered by detect in this pass
@@ -87,13 +87,17 @@ struct InstState {
     int stageActive;  // MOOD loop of the current stage still running
     int anyFail;     // face cascade: some cell failed CAD/PAD since the last check
     int nextIter;    // face cascade: this instance runs the next inner iteration
-    int cascaded;    // face cascade ran in the current pass
-    int cascadeMode;  // CASCADE_FROM_FACES after pass 1's fused kernel, else FROM_CELLS
+    int cascaded;    // face cascade ran in the current pass (kernel-chain form)
+    int big;         // this stage's work lists are too long for one cluster: the kernel chain takes it
+    int cFail;       // cells that failed CAD/PAD in pass 1 (its list of them)
+    int nCasc;       // cells on the cluster form's cascade-lowered list
+    int mc[8];       // the cluster form's list counters (mood_cluster.cuh MC_*)
     int nInner, nDetect;  // lowerings in the current pass
     int lastInner, lastDetect;  // lowerings of the last finished pass
     int passes;      // MOOD passes in the current stage
     int passCap;     // pass limit of a stage (HOSONO_MOOD_CAP_DEFAULT, or set by the caller)
     int maxPasses, stages, cascadeIters, passesTotal;
+    int chainPasses, chainIters;  // of passesTotal / cascadeIters: those the kernel chain ran
     long long innerTotal, detectTotal;
     unsigned long long cflbits[2];
 };
@@ -107,7 +111,10 @@ struct BatchFlags {
     int stepsLeft;   // step budget of the current run launch
     int radii;       // bit R set when a live instance has GP radius R (per-radius kernels of absent radii exit)
     int recSel;      // which recompute list the current MOOD pass reads (0: Lists::rec, 1: rec2)
-    int p1Next[4];   // pass 1 with the dynamic schedule: next tile index per radius (zeroed by stage_init)
+    int p1Next[4];   // pass 1 with the dynamic schedule: next tile index per radius (zeroed by mood_faces)
+    int anyCasc;     // some instance's pass-1 face cascade is left to the kernel chain
+    int anyMood;     // some instance's later passes are left to the kernel chain
+    int mcDone, mcBig;  // clusters finished in the running cluster launch; whether one left work to the chain
 };
 
 // Roles of the three U buffers: the state lives in U[parity]; A in
@@ -150,6 +157,8 @@ struct Batch {
     int p1Radii;         // bit R: the host launches the radius-R pass-1 kernel (radii held)
     int p1First, p1End;  // pass 1 covers tiles [p1First, min(p1End, ntiles)) of the tile list
     int ctStaged;        // the pass-1 update reads TMA-staged boxes (1) or the planes (0)
+    int p1Init;          // pass 1 also resets the stage's MOOD planes (0: the autotuner's timing launches)
+    int mcMax;           // most listed cells the cluster kernels take per instance (-1: everything to the chain)
     int maxTiles;        // capacity of the tile list
     int maxInst;         // capacity (slots)
     const int2* instTiles;  // per slot: first tile in the tile list, tile count (0: not live)
@@ -166,7 +175,6 @@ struct Batch {
     int* casInfo;
 };
 
-enum : int { CASCADE_FROM_FACES = 0, CASCADE_FROM_CELLS = 1 };
 enum : int { MOOD_FLAGS_LISTS = 0, MOOD_FLAGS_DENSE = 1, MOOD_FLAGS_LISTS_CLEAR = 2 };
 
 // Buffers of the per-module entry points (the reference's block arrays the
@@ -209,8 +217,13 @@ struct KernelSet {
     void (*step_begin)(const Batch&, int use_host_dt, cudaStream_t);
     void (*step_end)(const Batch&, cudaGraphConditionalHandle run_cond, cudaStream_t);
     // forward-Euler stage
-    void (*stage_init)(const Batch&, cudaStream_t);
     void (*face_pass1)(const Batch&, int uin, cudaStream_t);
+    // one cluster per instance: the stage scalars, and pass 1's face cascade
+    // with the fluxes it changes; h: some instance is left to the chain
+    void (*mood_faces)(const Batch&, int uin, cudaGraphConditionalHandle h, cudaStream_t);
+    // one cluster per instance: the end of pass 1 and every later pass of the
+    // stage; h: some instance is left to the chain
+    void (*mood_passes)(const Batch&, int uin, int uout, cudaGraphConditionalHandle h, cudaStream_t);
     void (*cascade_cond)(const Batch&, cudaGraphConditionalHandle h, cudaStream_t);
     // face cascade: the kernels walk the tiles of the instances in the
     // current iteration (Batch::casRange); `later` marks a later MOOD pass
@@ -228,7 +241,8 @@ struct KernelSet {
     void (*compact_dirty)(const Batch&, cudaStream_t);  // pass-1 faces next to re-reconstructed cells
     void (*flux_list)(const Batch&, int uin, cudaStream_t);
     void (*ct_list)(const Batch&, int uin, int uout, cudaStream_t);
-    void (*clear_low)(const Batch&, cudaStream_t);
+    void (*clear_low)(const Batch&, cudaStream_t);        // a later pass's lowered cells
+    void (*clear_low_pass1)(const Batch&, cudaStream_t);  // pass 1's, of the chain's instances
     // RK3 combines and boundary conditions
     void (*bc_fill)(const Batch&, int role, cudaStream_t);
     void (*rk_combine2)(const Batch&, cudaStream_t);

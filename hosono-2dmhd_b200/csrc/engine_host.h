@@ -22,6 +22,10 @@ struct DeviceAllocator {
     virtual void release(void* p) = 0;
 };
 
+// Most listed cells (pass 1's failing cells, then the cells detect lowered in
+// it) an instance may have for one cluster to take its stage.
+constexpr int kClusterCells = 2000;
+
 class Engine {
   public:
     Engine() = default;
@@ -153,6 +157,8 @@ class Engine {
     }
     // head = false leaves out the stage's set-up and pass 1 (run before, by the banded upload)
     int record_stage(Rec& r, int uin, int uout, cudaEvent_t ev0, cudaEvent_t ev1, bool head = true);
+    template <class Cascade>
+    int record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cascade_body);
     int record_step(Rec& r, bool host_dt, cudaGraphConditionalHandle run_cond, bool profile,
                     bool first_head = true);
     int build_graphs();

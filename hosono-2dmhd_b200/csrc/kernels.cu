@@ -197,9 +197,15 @@ __device__ __forceinline__ int rec_count(const Batch& B, bool next) { return rec
 // + getFluxes_ fused.  A thread owns the x-face between (i-1,j) and (i,j) and
 // the y-face between (i,j-1) and (i,j).  Face values are recomputed per
 // quadrature point and never stored.  A cell fails when any of its four
-// faces fails; the verdicts are kept per face side in failX / failY and
-// combined by cascade_lower.  Fluxes next to a cell the cascade
-// re-reconstructs are recomputed after it (compact_dirty + flux_list).
+// faces fails: the first failing face side marks it in `fail` and puts it on
+// the instance's list of failing cells.  Fluxes next to a cell the cascade
+// re-reconstructs are recomputed after it (mood_faces; compact_dirty +
+// flux_list in the chain).  The tile's MOOD planes are reset on the way
+// (timeStep_forwardEuler, timeStep.f90:79-81: scheme = R; recompute and
+// recomputeFLICD are true everywhere in pass 1, which its kernels know, so
+// the planes start clear for the flags of the later passes): eight bytes a
+// cell beside 144 of fluxes, in a kernel far from HBM's rate, instead of a
+// launch of its own.
 //
 // The block stages its tile's stencil box -- x in [x0-4, x0+36), y in
 // [y0-1-R, y0+9+R), all 8 planes -- in shared memory (16-byte vector loads,
@@ -290,10 +296,18 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
     return bits;
 }
 
+// a face side of cell c failed CAD/PAD in pass 1 (rare: kept out of line); the
+// byte is set through its 32-bit word, so exactly one thread lists the cell
+__device__ __noinline__ void pass1_fail(uint8_t* fail, int* list, int* count, int c) {
+    const unsigned sh = 8u * (unsigned)(c & 3);
+    const unsigned old = atomicOr(reinterpret_cast<unsigned*>(fail + (c - (c & 3))), 1u << sh);
+    if (((old >> sh) & 0xffu) == 0) list[atomicAdd(count, 1)] = c;
+}
+
 // the x- and y-faces of one cell of the staged tile (sim_forceHydro fixed at
-// compile time); returns whether any face state failed CAD/PAD
+// compile time)
 template <int R, int FH>
-__device__ __forceinline__ bool pass1_tile(const InstDev& d, const double* __restrict__ sU,
+__device__ __forceinline__ void pass1_tile(const Batch& B, const InstDev& d, const double* __restrict__ sU,
                                            const double* __restrict__ sPv, const Cell& c, double* acc) {
     using Box = P1Box<R>;
     const Geo& G = d.geo;
@@ -304,18 +318,29 @@ __device__ __forceinline__ bool pass1_tile(const InstDev& d, const double* __res
     const int sx = threadIdx.x + Box::OX, sy = threadIdx.y + Box::OY;
     const long long cc = (long long)j * G.pitch + i;
     const bool inF = i >= flo && i <= fxhi && j >= flo && j <= fyhi;
-    bool bad = false;
+    if (B.p1Init && i < G.nxt && j < G.nyt) {
+        d.scheme[B.st[c.k].schemeSel][cc] = (int8_t)R;
+        d.rrRec[cc] = (uint8_t)(R | (R << 2) | (R << 4) | (R << 6));
+        d.rec[cc] = 0;
+        d.recF[cc] = 0;
+        d.recB[cc] = 0;
+        d.recFB[cc] = 0;
+        d.dirty[cc] = 0;
+        d.innerCount[cc] = 0;
+    }
 #pragma unroll 1
     for (int dir = XDIR; dir <= YDIR; dir++) {  // the x-face, then the y-face of this cell
         const bool x = dir == XDIR;
         if (i >= clo && i <= cxhi + (x ? 1 : 0) && j >= clo && j <= cyhi + (x ? 0 : 1)) {
             const int a = x ? i : j, ahi = x ? cxhi : cyhi;
             const uint8_t bits = pass1_face<R, FH>(d, sU, sPv, sx, sy, dir, a - 1 >= clo, a <= ahi, inF, cc, acc);
-            (x ? d.failX : d.failY)[cc] = bits;
-            bad |= bits != 0;
+            if (bits) {
+                int* list = reinterpret_cast<int*>(B.L.face + 2 * (long long)B.instTiles[c.k].x * (TILE_X * TILE_Y));
+                if (bits & 1) pass1_fail(d.fail, list, &B.st[c.k].cFail, (int)(x ? cc - 1 : cc - G.pitch));
+                if (bits & 2) pass1_fail(d.fail, list, &B.st[c.k].cFail, (int)cc);
+            }
         }
     }
-    return bad;
 }
 
 // 16-byte asynchronous copy global -> shared (cp.async); src_bytes = 0
@@ -515,12 +540,12 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             }
             __syncthreads();  // tile t's box is in place for every thread
             const Cell c = tile_at(B, t);
-            InstState& S = B.st[c.k];
             const InstDev& d = B.dev[c.k];
-            if (first_tile_thread(c)) S.cascadeMode = CASCADE_FROM_FACES;
-            const bool bad = d.phys.force_hydro ? pass1_tile<R, 1>(d, smem, pvBuf, c, acc)
-                                                : pass1_tile<R, 0>(d, smem, pvBuf, c, acc);
-            warp_flag(&S.anyFail, bad);
+            // one instance per tile: the branch is uniform over the block
+            if (d.phys.force_hydro)
+                pass1_tile<R, 1>(B, d, smem, pvBuf, c, acc);
+            else
+                pass1_tile<R, 0>(B, d, smem, pvBuf, c, acc);
             __syncthreads();  // every read of this box is done before it is refilled
             t = next_tile(t + gridDim.x);
         }
@@ -559,12 +584,11 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
         const double* sU = smem + buf * Box::DOUBLES;
         const double* sPv = pvBuf + buf * Box::PVN;
         const Cell c = tile_at(B, t);
-        InstState& S = B.st[c.k];
         const InstDev& d = B.dev[c.k];
-        if (first_tile_thread(c)) S.cascadeMode = CASCADE_FROM_FACES;
-        // one instance per tile: the branch is uniform over the block
-        const bool bad = d.phys.force_hydro ? pass1_tile<R, 1>(d, sU, sPv, c, acc) : pass1_tile<R, 0>(d, sU, sPv, c, acc);
-        warp_flag(&S.anyFail, bad);
+        if (d.phys.force_hydro)
+            pass1_tile<R, 1>(B, d, sU, sPv, c, acc);
+        else
+            pass1_tile<R, 0>(B, d, sU, sPv, c, acc);
         __syncthreads();  // every read of this box is done before it is refilled
         buf ^= 1;
         t = tn;
@@ -638,6 +662,7 @@ __device__ __forceinline__ void d_cascade_cond(const Batch& B, int tid, cudaGrap
         if (in) {
             S.cascaded = 1;
             S.cascadeIters++;
+            S.chainIters++;
             any = 1;
         }
     }
@@ -688,10 +713,9 @@ __device__ __forceinline__ void lower_cell(const InstDev& d, const InstState& S,
     d.innerCount[cc] = (uint8_t)(d.innerCount[cc] + 1);
 }
 
-// For each cell of [g-2, g+n+1]^2 that failed (face verdicts of pass 1, or the
-// `fail` plane of a re-reconstruction, which is cleared as it is consumed):
-// lower it.
-__device__ __forceinline__ void t_cascade_lower(const Batch& B, const Cell c) {
+// For each cell of [g-2, g+n+1]^2 that failed (the `fail` plane of pass 1 or
+// of a re-reconstruction, cleared as it is consumed): lower it.
+__device__ __forceinline__ void t_cascade_lower(const Batch& B, int later, const Cell c) {
     InstState& S = B.st[c.k];
     if (!S.nextIter) return;
     const InstDev& d = B.dev[c.k];
@@ -701,24 +725,24 @@ __device__ __forceinline__ void t_cascade_lower(const Batch& B, const Cell c) {
     bool f = false;
     if (i >= g - 2 && j >= g - 2 && i <= g + G.nx + 1 && j <= g + G.ny + 1) {
         const long long cc = (long long)j * G.pitch + i;
-        if (S.cascadeMode == CASCADE_FROM_FACES) {
-            f = ((d.failX[cc] & 2) | (d.failX[cc + 1] & 1) | (d.failY[cc] & 2) | (d.failY[cc + G.pitch] & 1)) != 0;
-        } else {
-            f = d.fail[cc] != 0;
-            if (f) d.fail[cc] = 0;
+        f = d.fail[cc] != 0;
+        if (f) {
+            d.fail[cc] = 0;
+            lower_cell(d, S, i, j, cc);
         }
-        if (f) lower_cell(d, S, i, j, cc);
     }
     warp_count(&S.nInner, f);
-    // the first lowering of a cell in this pass puts it on the list whose
-    // translate classes the later-pass flag rebuild brings to one scheme
+    // the first lowering of a cell in a later pass puts it on the list whose
+    // translate classes that pass's flag rebuild brings to one scheme (pass 1
+    // rebuilds every cell; its list may hold a cluster instance's cells)
+    if (!later) return;
     const long long cc = (long long)j * G.pitch + i;
     const bool first = f && !(d.detMask[cc] & DM_CASC);
     if (first) d.detMask[cc] |= DM_CASC;
     warp_append(B.L, LIST_CASC, B.L.casc, B.L.cap, first, entry(c.k, cc));
 }
-__global__ void __launch_bounds__(NTHREADS) k_cascade_lower(Batch B) { PDL_ENTRY();
-    FOR_CASCADE_TILES(B, t) t_cascade_lower(B, tile_at(B, t));
+__global__ void __launch_bounds__(NTHREADS) k_cascade_lower(Batch B, int later) { PDL_ENTRY();
+    FOR_CASCADE_TILES(B, t) t_cascade_lower(B, later, tile_at(B, t));
 }
 
 
@@ -784,7 +808,6 @@ __device__ __forceinline__ void t_compact_next(const Batch& B, const Cell c) {
     const InstDev& d = B.dev[c.k];
     const Geo& G = d.geo;
     const int g = G.g;
-    if (first_tile_thread(c)) S.cascadeMode = CASCADE_FROM_CELLS;
     bool p = false;
     long long cc = 0;
     if (c.i >= g - 2 && c.j >= g - 2 && c.i <= g + G.nx + 1 && c.j <= g + G.ny + 1) {
@@ -1153,12 +1176,14 @@ __device__ __forceinline__ bool update_detect_at(const InstDev& d, const InstSta
 // neighbour needs is recomputed locally when the neighbour is flagged (it
 // writes the same value) and read from memory otherwise (nobody writes it).
 // A lowered cell sets `lowered` (cleared again after the flags are rebuilt)
-// and is appended to the lowered list.
+// and is appended to the lowered list.  ALL: pass 1, where recomputeFLICD
+// holds everywhere.
+template <bool ALL>
 __device__ __forceinline__ bool ct_cell_at(const InstDev& d, const InstState& S, int uout, int i, int j, long long cc,
                                            const CellSrc& src) {
     const Geo& G = d.geo;
     const int g = G.g;
-    if (!d.recF[cc]) return false;
+    if (!ALL && !d.recF[cc]) return false;
     const double* fxy = src.FX + MAGY * src.fplane;
     const double* fyx = src.FY + MAGX * src.fplane;
     const double ctx = flicd_x_at(fxy, fyx, src.fc, src.fp);
@@ -1167,18 +1192,32 @@ __device__ __forceinline__ bool ct_cell_at(const InstDev& d, const InstState& S,
     d.CTY[cc] = cty;
     if (i >= g + G.nx || j >= g + G.ny) return false;  // FLICD-only row and column
     const long long ce = cc + 1, cn = cc + G.pitch;
-    const double ctx_e = d.recF[ce] ? flicd_x_at(fxy, fyx, src.fc + 1, src.fp) : d.CTX[ce];
-    const double cty_n = d.recF[cn] ? flicd_y_at(fxy, fyx, src.fc + src.fp, src.fp) : d.CTY[cn];
+    const double ctx_e = ALL || d.recF[ce] ? flicd_x_at(fxy, fyx, src.fc + 1, src.fp) : d.CTX[ce];
+    const double cty_n = ALL || d.recF[cn] ? flicd_y_at(fxy, fyx, src.fc + src.fp, src.fp) : d.CTY[cn];
     return update_detect_at(d, S, uout, cc, src, ctx, cty, ctx_e, cty_n);
 }
+template <bool ALL>
 __device__ __forceinline__ bool ct_cell(const InstDev& d, const InstState& S, int uin, int uout, int i, int j,
                                         long long cc) {
-    return ct_cell_at(d, S, uout, i, j, cc, global_src(d, S, uin, cc));
+    return ct_cell_at<ALL>(d, S, uout, i, j, cc, global_src(d, S, uin, cc));
+}
+
+// the instance's list of the cells detect lowered in pass 1 (cell indices in
+// its segment of the batch's list), counted by nDetect: one atomic per warp
+__device__ __forceinline__ void low_append(const Batch& B, int k, bool low, long long cc) {
+    const unsigned m = __ballot_sync(0xffffffffu, low);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(&B.st[k].nDetect, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    int* list = reinterpret_cast<int*>(B.L.low + (long long)B.instTiles[k].x * (TILE_X * TILE_Y));
+    if (low) list[base + __popc(m & ((1u << lane) - 1))] = (int)cc;
 }
 
 __device__ __forceinline__ void t_ct_update_detect(const Batch& B, int uin, int uout, const Cell c, double* sV) {
     InstState& S = B.st[c.k];
-    if (!(S.stepping && S.stageActive)) return;  // uniform over the block
+    if (!S.stepping) return;  // uniform over the block
     detect_prep_tile(B, S, uin, c, sV);
     const InstDev& d = B.dev[c.k];
     const Geo& G = d.geo;
@@ -1187,10 +1226,9 @@ __device__ __forceinline__ void t_ct_update_detect(const Batch& B, int uin, int 
     long long cc = 0;
     if (c.i >= g && c.j >= g && c.i <= g + G.nx && c.j <= g + G.ny) {
         cc = (long long)c.j * G.pitch + c.i;
-        low = ct_cell(d, S, uin, uout, c.i, c.j, cc);
+        low = ct_cell<true>(d, S, uin, uout, c.i, c.j, cc);
     }
-    warp_count(&S.nDetect, low);
-    warp_append(B.L, LIST_LOW, B.L.low, B.L.cap, low, entry(c.k, cc));
+    low_append(B, c.k, low, cc);
 }
 // six resident blocks (a 40-register budget, a few hundred bytes of spills):
 // the tile's loads wait at two barriers, so more warps in flight keep HBM
@@ -1232,7 +1270,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_ct_update_detect_tma(Batch B, i
     FOR_TILES(B, t) {
         const Cell c = tile_at(B, t);
         InstState& S = B.st[c.k];
-        if (!(S.stepping && S.stageActive)) continue;  // uniform over the block
+        if (!S.stepping) continue;  // uniform over the block
         const InstDev& d = B.dev[c.k];
         const Geo& G = d.geo;
         const int x0 = c.i - (int)threadIdx.x, y0 = c.j - (int)threadIdx.y;  // the tile's origin
@@ -1262,10 +1300,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_ct_update_detect_tma(Batch B, i
             cc = (long long)c.j * G.pitch + c.i;
             const CellSrc src{sU,  (long long)(c.j - uy0) * CT_SX + (c.i - ux0), CT_UPL, CT_SX,
                               sFX, sFY, (long long)(c.j - fy0) * CT_SX + (c.i - ux0), CT_FPL, CT_SX};
-            low = ct_cell_at(d, S, uout, c.i, c.j, cc, src);
+            low = ct_cell_at<true>(d, S, uout, c.i, c.j, cc, src);
         }
-        warp_count(&S.nDetect, low);
-        warp_append(B.L, LIST_LOW, B.L.low, B.L.cap, low, entry(c.k, cc));
+        low_append(B, c.k, low, cc);
     }
 }
 
@@ -1281,7 +1318,7 @@ __device__ __forceinline__ void d_ct_list(const Batch& B, int uin, int uout, int
             const InstDev& d = B.dev[it.x];
             const long long cc = it.y;
             const int j = (int)(cc / d.geo.pitch), i = (int)(cc - (long long)j * d.geo.pitch);
-            low = ct_cell(d, S, uin, uout, i, j, cc);
+            low = ct_cell<false>(d, S, uin, uout, i, j, cc);
             if (low) atomicAdd(&S.nDetect, 1);
         }
         warp_append(B.L, LIST_LOW, B.L.low, B.L.cap, low, it);
@@ -1298,6 +1335,15 @@ __device__ __forceinline__ void d_clear_low(const Batch& B, int gt, int gs) {
     }
 }
 __global__ void __launch_bounds__(256) k_clear_low(Batch B) { PDL_ENTRY(); d_clear_low(B, GT1, GS1); }
+// the same after pass 1, whose lowered cells are listed per instance
+__global__ void __launch_bounds__(256) k_clear_low_pass1(Batch B) { PDL_ENTRY();
+    for (int k = 0; k < B.maxInst; k++) {
+        const InstState& S = B.st[k];
+        if (!(S.stepping && S.stageActive)) continue;
+        const int* list = reinterpret_cast<const int*>(B.L.low + (long long)B.instTiles[k].x * (TILE_X * TILE_Y));
+        for (int e = GT1; e < S.nDetect; e += GS1) B.dev[k].lowered[list[e]] = 0;
+    }
+}
 
 // ======================================================================
 // After detect: recompute = cross of lowered cells, recomputeFLICD = radius-2
@@ -1520,6 +1566,7 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
         if (flip && pass_lowered(S)) S.schemeSel = 1 - S.schemeSel;  // k_mood_flags wrote the other buffer
         S.passes++;
         S.passesTotal++;
+        S.chainPasses++;
         S.innerTotal += S.nInner;
         S.detectTotal += S.nDetect;
         S.lastInner = S.nInner;
@@ -1534,7 +1581,6 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
             S.error = HOSONO_EMOODCAP;
         } else {
             any = 1;
-            S.cascadeMode = CASCADE_FROM_CELLS;  // later passes' cascades start from re-reconstructions
         }
         S.nInner = 0;
         S.nDetect = 0;
@@ -1559,43 +1605,6 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
 __global__ void __launch_bounds__(PASS_END_THREADS) k_pass_end(Batch B, cudaGraphConditionalHandle h, int set_handle,
                                                                 int flip) { PDL_ENTRY();
     d_pass_end<PASS_END_THREADS>(B, threadIdx.x, h, set_handle, flip);
-}
-
-// timeStep_forwardEuler's reset (timeStep.f90:79-81) on every cell:
-// scheme = R, recompute = recomputeFLICD = .true.; plus the per-instance
-// stage scalars.
-__device__ __forceinline__ void t_stage_init(const Batch& B, const Cell c) {
-    InstState& S = B.st[c.k];
-    if (!S.stepping) return;
-    const InstDev& d = B.dev[c.k];
-    const Geo& G = d.geo;
-    if (first_tile_thread(c)) {
-        S.stageActive = 1;
-        S.passes = 0;
-        S.nInner = 0;
-        S.nDetect = 0;
-        S.anyFail = 0;
-        S.cascaded = 0;
-        S.stages++;
-    }
-    if (c.i >= G.nxt || c.j >= G.nyt) return;
-    const long long cc = (long long)c.j * G.pitch + c.i;
-    const int R = G.R;
-    d.scheme[S.schemeSel][cc] = (int8_t)R;
-    d.rec[cc] = 1;
-    d.recF[cc] = 1;
-    d.rrRec[cc] = (uint8_t)(R | (R << 2) | (R << 4) | (R << 6));
-    d.dirty[cc] = 0;
-    d.innerCount[cc] = 0;
-}
-__global__ void __launch_bounds__(NTHREADS) k_stage_init(Batch B) { PDL_ENTRY();
-    if (blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) {  // the recompute lists start empty
-        B.L.counts[LIST_REC] = 0;
-        B.L.counts[LIST_REC2] = 0;
-        for (int r = 0; r < 4; r++) B.flags->p1Next[r] = 0;  // pass 1's dynamic schedule starts over
-        B.gbar[0] = 0;  // the persistent later-pass launch's barrier count (after an aborted launch too)
-    }
-    FOR_TILES(B, t) t_stage_init(B, tile_at(B, t));
 }
 
 // ======================================================================
@@ -1879,7 +1888,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_mood_rest(Batch B, int uin, int
         if (blockIdx.x == 0) d_cascade_cond<NTHREADS>(B, tid, 0, 0);
         GSYNC_OR_LEAVE;
         while (ld_acquire_s32(&B.flags->anyFail)) {
-            FOR_CASCADE_TILES(B, t) t_cascade_lower(B, tile_at(B, t));
+            FOR_CASCADE_TILES(B, t) t_cascade_lower(B, 1, tile_at(B, t));
             GSYNC_OR_LEAVE;
             FOR_CASCADE_TILES(B, t) t_compact_next(B, tile_at(B, t));
             GSYNC_OR_LEAVE;
@@ -1907,15 +1916,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_mood_rest(Batch B, int uin, int
 }
 
 // The autotuner times pass 1 between steps: the instances that would step
-// are marked stepping, and put back at rest afterwards (the face-cascade
-// flag pass 1 raised is cleared too; every stage starts from stage_init).
+// are marked stepping, and put back at rest afterwards (the failing cells
+// pass 1 listed are cleared too).
 __global__ void k_tune_mark(Batch B, int on) { PDL_ENTRY();
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
         S.stepping = (on && S.live && !S.done && !B.hold[k]) ? 1 : 0;
-        S.anyFail = 0;
+        if (!S.live) continue;
+        const int* list = reinterpret_cast<const int*>(B.L.face + 2 * (long long)B.instTiles[k].x * (TILE_X * TILE_Y));
+        for (int e = 0; e < S.cFail; e++) B.dev[k].fail[list[e]] = 0;
+        S.cFail = 0;
     }
 }
+
+#include "mood_cluster.cuh"
 
 // ======================================================================
 const dim3 kTile(TILE_X, TILE_Y);
@@ -1975,7 +1989,6 @@ void l_step_begin(const Batch& B, int use_host_dt, cudaStream_t s) { lk(k_step_b
 void l_step_end(const Batch& B, cudaGraphConditionalHandle h, cudaStream_t s) {
     lk(k_step_end, dim3(1), dim3(128), 0, s, B, h, (int)(h != 0));
 }
-void l_stage_init(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_stage_init, B, s); }
 // dynamic shared memory of a pass-1 kernel variant
 template <int R, int NBUF>
 constexpr int pass1_smem() {
@@ -2036,10 +2049,58 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
     if (B.p1Radii & (1 << 1)) launch_pass1<1>(B, uin, s);
     if (B.p1Radii & (1 << 3)) launch_pass1<3>(B, uin, s);
 }
+// One cluster per instance slot: 16 blocks (a non-portable size, taken where
+// the GPU can place one) for up to nine slots, which fills the GPU, else 8.
+template <typename K>
+int cluster_blocks(K kernel, int maxInst) {
+    static const bool sixteen = [kernel] {  // once per process and kernel (thread-safe static initialisation)
+        if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(MC_THREADS);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 16;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return n >= 1;
+    }();
+    return sixteen && maxInst <= 9 ? 16 : 8;
+}
+template <typename... KArgs, typename... Args>
+void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t s, Args... args) {
+    pdl_take();  // a cluster launch is never programmatic itself
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(blocks * B.maxInst));
+    cfg.blockDim = dim3(MC_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, B, args...);
+}
+void l_mood_faces(const Batch& B, int uin, cudaGraphConditionalHandle h, cudaStream_t s) {
+    lk_cluster(k_mood_faces, cluster_blocks(k_mood_faces, B.maxInst), B, s, uin, h, (int)(h != 0));
+}
+void l_mood_passes(const Batch& B, int uin, int uout, cudaGraphConditionalHandle h, cudaStream_t s) {
+    lk_cluster(k_mood_passes, cluster_blocks(k_mood_passes, B.maxInst), B, s, uin, uout, h, (int)(h != 0));
+}
 void l_cascade_cond(const Batch& B, cudaGraphConditionalHandle h, cudaStream_t s) {
     lk(k_cascade_cond, dim3(1), dim3(PASS_END_THREADS), 0, s, B, h, (int)(h != 0));
 }
-void l_cascade_lower(const Batch& B, int /*later*/, cudaStream_t s) { TILE_LAUNCH(k_cascade_lower, B, s); }
+void l_cascade_lower(const Batch& B, int later, cudaStream_t s) { TILE_LAUNCH(k_cascade_lower, B, s, later); }
 void l_recon_check(const Batch& B, int uin, int /*later*/, cudaStream_t s) {
     TILE_LAUNCH(k_compact_next, B, s);
     LIST_LAUNCH(k_recon_group, B, s, uin, (int)LIST_NEXT);
@@ -2075,6 +2136,7 @@ void l_recon_list(const Batch& B, int uin, cudaStream_t s) { LIST_LAUNCH(k_recon
 void l_flux_list(const Batch& B, int uin, cudaStream_t s) { LIST_LAUNCH(k_flux_list, B, s, uin); }
 void l_ct_list(const Batch& B, int uin, int uout, cudaStream_t s) { LIST_LAUNCH(k_ct_list, B, s, uin, uout); }
 void l_clear_low(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low, B, s); }
+void l_clear_low_pass1(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low_pass1, B, s); }
 void l_bc_fill(const Batch& B, int role, cudaStream_t s) { TILE_LAUNCH(k_bc_fill, B, s, role); }
 void l_rk_combine2(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_rk_combine2, B, s); }
 void l_rk_final(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_rk_final, B, s); }
@@ -2100,8 +2162,8 @@ void l_launch_info(int R, int maxTiles, int* pass1, int* tile_grid_max) {
     *pass1 = R == 1   ? pass1_grid<1, false, false, 2, 2>(maxTiles)
              : R == 2 ? pass1_grid<2, false, false, 2, 2>(maxTiles)
                       : pass1_grid<3, false, false, 2, 2>(maxTiles);
-    const void* tile_kernels[] = {(const void*)k_cfl_reduce,     (const void*)k_stage_init,
-                                  (const void*)k_cascade_lower,  (const void*)k_compact_next, (const void*)k_compact_post,
+    const void* tile_kernels[] = {(const void*)k_cfl_reduce,     (const void*)k_cascade_lower,
+                                   (const void*)k_compact_next, (const void*)k_compact_post,
                                   (const void*)k_compact_dirty,  (const void*)k_ct_update_detect, (const void*)k_mood_flags,
                                   (const void*)k_bc_fill,        (const void*)k_rk_combine2,  (const void*)k_rk_final,
                                   (const void*)k_cons2prim_all};
@@ -2121,9 +2183,9 @@ const KernelSet kset = {
 #else
     "strict",
 #endif
-    l_cfl_reduce, l_step_prepare, l_step_begin, l_step_end, l_stage_init, l_face_pass1, l_cascade_cond, l_cascade_lower,
+    l_cfl_reduce, l_step_prepare, l_step_begin, l_step_end, l_face_pass1, l_mood_faces, l_mood_passes, l_cascade_cond, l_cascade_lower,
     l_recon_check, l_ct_update_detect, l_mood_flags, l_pass_end, l_recon_list,
-    l_compact_post, l_compact_dirty, l_flux_list, l_ct_list, l_clear_low, l_bc_fill, l_rk_combine2, l_rk_final,
+    l_compact_post, l_compact_dirty, l_flux_list, l_ct_list, l_clear_low, l_clear_low_pass1, l_bc_fill, l_rk_combine2, l_rk_final,
     l_cons2prim_all, l_tune_mark, l_mood_rest, l_launch_info, &mops};
 
 }  // namespace KNS
