@@ -20,7 +20,7 @@ INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-I", CSRC,
-               "--expt-relaxed-constexpr"] + ARCH
+               "--expt-relaxed-constexpr", "-split-compile", "0"] + ARCH
 
 
 def nvcc():

@@ -224,74 +224,176 @@ struct P1Box {
     static constexpr int PVN = NS * NQ * 4;
 };
 
-// GP prediction from the shared box: sum_k pv(k,q,f,RR) * U(:, stencil_k)
-// around shared coordinates (sx, sy), stencil order k=1..ns; pvq points at
-// the prediction vector in shared memory (one broadcast load per k)
-template <int RR, int R>
-__device__ __forceinline__ void gp_face_s(const double* __restrict__ sU, int sx, int sy,
-                                          const double* __restrict__ pvq, double out[NCONS]) {
-    constexpr int SX = P1Box<R>::SX, PL = P1Box<R>::PLANE;
-    const double* base = sU + sy * SX + sx;
+// GP predictions of both sides of a face at NQP quadrature points from the
+// shared box: u[q][side] = sum_k pv(k,q,f,RR) * U(:, stencil_k), stencil order
+// k=1..ns for each (reconstruct.f90:109-124), in face coordinates
+// (physics.cuh).  `base` is the right (upper) cell in plane 0; `swap` is 0 for
+// an x-face and one plane for a y-face, which exchanges the in-plane planes.
+// Variables the mode leaves out are not summed.  One sweep over the union of
+// the two stencils (18 points at R = 2 where the two have 26) in an order that
+// keeps each sum's own, and every value loaded serves both sides and both
+// points: a sweep per side and point read shared memory for 61 % of the
+// kernel's time.  pvL, pvR: the sides' prediction vectors of the first point
+// (broadcast loads).
+template <int R, int MODE, bool X, int NQP>
+__device__ __forceinline__ void gp_face_s(const double* __restrict__ base, int swap, const double* __restrict__ pvL,
+                                          const double* __restrict__ pvR, double (&u)[NQP][2][NCONS]) {
+    constexpr int SX = P1Box<R>::SX, PL = P1Box<R>::PLANE, NS = P1Box<R>::NS;
+    const double* up = base + swap;
+    const double* dn = base - swap;
+    // the first term onto zero in one operation: 0 + RN(p*x) and RN(p*x + 0)
+    // are one value
+    auto add = [](double s, double p, double x, bool first) { return first ? fma(p, x, 0.0) : s + p * x; };
+    int kL = 0, kR = 0;
 #pragma unroll
-    for (int v = 0; v < NCONS; v++) out[v] = 0.0;
-    int k = 0;
+    for (int a = X ? -R - 1 : -R; a <= R; a++) {
 #pragma unroll
-    for (int a = -RR; a <= RR; a++) {
+        for (int b = X ? -R : -R - 1; b <= R; b++) {
+            const bool inL = X ? iabs_c(a + 1) + iabs_c(b) <= R : iabs_c(a) + iabs_c(b + 1) <= R;
+            const bool inR = iabs_c(a) + iabs_c(b) <= R;
+            if (!inL && !inR) continue;
+            double pL[NQP], pR[NQP];
 #pragma unroll
-        for (int b = -RR; b <= RR; b++) {
-            if (iabs_c(a) + iabs_c(b) <= RR) {
-                const double p = pvq[k];
-#pragma unroll
-                for (int v = 0; v < NCONS; v++) out[v] = out[v] + p * base[v * PL + b * SX + a];
-                k++;
+            for (int q = 0; q < NQP; q++) {
+                if (inL) pL[q] = pvL[q * NS + kL];
+                if (inR) pR[q] = pvR[q * NS + kR];
             }
+#pragma unroll
+            for (int v = 0; v < NCONS; v++) {
+                if (!Solve<MODE>::var(v)) continue;
+                const double* w = v == MOMN || v == MAGN ? up : v == MOMT || v == MAGT ? dn : base;
+                const double x = w[v * PL + b * SX + a];
+#pragma unroll
+                for (int q = 0; q < NQP; q++) {
+                    if (inL) u[q][0][v] = add(u[q][0][v], pL[q], x, kL == 0);
+                    if (inR) u[q][1][v] = add(u[q][1][v], pR[q], x, kR == 0);
+                }
+            }
+            kL += inL;
+            kR += inR;
         }
     }
 }
 
-// one face (both sides, every quadrature point); returns the side verdict bits
-// (the Gauss sum of the fluxes accumulates in this thread's column of
-// shared memory, acc[v * NTHREADS], which keeps it out of the registers the
-// Riemann solver needs).  dir is a run-time value: the kernel holds one copy
-// of this code (and of the Riemann solver) for both face directions, which
-// halves its instruction footprint.
-template <int R, int FH>
+// What the thread that reads a box last needs to have it refilled (in shared
+// memory: nothing of it stays in registers through the solves).
+struct P1Ctl {
+    const InstDev* dev;
+    const InstState* st;
+    const int4* tiles;
+    uint64_t* bar;
+    double *box, *pv;
+    int n, uin;    // end of the launch's tiles, the stage input's role
+    int next[2];   // the block's tile of each turn, by the turn's parity
+    int turn;      // the turn whose box is in place
+    int released;  // threads done with that box
+};
+// One thread of the block releases the box.  The last one has the next
+// tile's box loaded into it, so that the copy runs beside the tile's last
+// solves instead of after them.  ctl is null where the block stages itself.
+template <int R>
+static __device__ __noinline__ void p1_refill(P1Ctl* ctl);
+template <int R>
+__device__ __forceinline__ void p1_release(P1Ctl* ctl) {
+    if (!ctl) return;
+    __threadfence_block();  // after this thread's reads of the box
+    if (atomicAdd(&ctl->released, 1) == NTHREADS - 1) p1_refill<R>(ctl);
+}
+
+// one face (both sides, every quadrature point); returns the side verdict bits.
+// Points go in pairs: one sweep of GP sums gives both, the second's states wait
+// in this thread's column of shared memory (park[k * NTHREADS]) while the first
+// is solved.  The Gauss sum of the fluxes accumulates in another column
+// (acc[v * NTHREADS]), which keeps it out of the registers the Riemann solver
+// needs.  dir is a run-time value: the kernel holds one copy of the Riemann
+// solver for both face directions, which halves its instruction footprint; the
+// solver works in face coordinates, so only plane offsets depend on it.
+template <int R, int MODE>
 __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __restrict__ sU,
                                               const double* __restrict__ sPv, int sx, int sy, int dir, bool needL,
-                                              bool needR, bool doFlux, long long c, double* acc) {
+                                              bool needR, bool doFlux, long long c, double* acc, double* park,
+                                              P1Ctl* ctl) {
+    typedef Solve<MODE> S;
     const Geo& G = d.geo;
     const Phys& P = d.phys;
-    constexpr int NQ = R + 1;
+    constexpr int NQ = R + 1, NS = P1Box<R>::NS;
     const bool x = dir == XDIR;
-    const int FL = x ? EAST : NORTH, FR = x ? WEST : SOUTH;
-    const int lx = x ? sx - 1 : sx, ly = x ? sy : sy - 1;
+    const double* pvL = sPv + NS * NQ * (x ? EAST : NORTH);
+    const double* pvR = sPv + NS * NQ * (x ? WEST : SOUTH);
+    const double* base = sU + sy * P1Box<R>::SX + sx;
+    const int swap = x ? 0 : P1Box<R>::PLANE;
     uint8_t bits = 0;
 #pragma unroll
-    for (int v = 0; v < NCONS; v++) acc[v * NTHREADS] = 0.0;
+    for (int v = 0; v < NCONS; v++)
+        if (S::var(v)) acc[v * NTHREADS] = 0.0;
 #pragma unroll 1
-    for (int q = 0; q < NQ; q++) {
+    for (int q0 = 0; q0 < NQ; q0 += 2) {
+        const bool pair = q0 + 1 < NQ;
         double uL[NCONS], uR[NCONS];
-        if (needL) {
-            gp_face_s<R, R>(sU, lx, ly, sPv + P1Box<R>::NS * (q + P1Box<R>::NQ * FL), uL);
-            if (!admissible(uL[DENS], cons2pres<FH>(P, uL))) bits |= 1;
-        }
-        if (needR) {
-            gp_face_s<R, R>(sU, sx, sy, sPv + P1Box<R>::NS * (q + P1Box<R>::NQ * FR), uR);
-            if (!admissible(uR[DENS], cons2pres<FH>(P, uR))) bits |= 2;
-        }
-        if (doFlux) {
-            double F[NCONS];
-            hllc<FH>(P, uL, uR, dir, F);
-            const double w = qw_at(d, R, q);
+        if ((NQ & 1) && !pair) {
+            double u[1][2][NCONS];
+            if (x)
+                gp_face_s<R, MODE, true, 1>(base, swap, pvL + NS * q0, pvR + NS * q0, u);
+            else
+                gp_face_s<R, MODE, false, 1>(base, swap, pvL + NS * q0, pvR + NS * q0, u);
 #pragma unroll
-            for (int v = 0; v < NCONS; v++) acc[v * NTHREADS] = acc[v * NTHREADS] + w * F[v];
+            for (int v = 0; v < NCONS; v++) {
+                uL[v] = u[0][0][v];
+                uR[v] = u[0][1][v];
+            }
+        } else {
+            double u[2][2][NCONS];
+            if (x)
+                gp_face_s<R, MODE, true, 2>(base, swap, pvL + NS * q0, pvR + NS * q0, u);
+            else
+                gp_face_s<R, MODE, false, 2>(base, swap, pvL + NS * q0, pvR + NS * q0, u);
+            int k = 0;
+#pragma unroll
+            for (int v = 0; v < NCONS; v++) {
+                uL[v] = u[0][0][v];
+                uR[v] = u[0][1][v];
+                if (!S::var(v)) continue;
+                park[k++ * NTHREADS] = u[1][0][v];
+                park[k++ * NTHREADS] = u[1][1][v];
+            }
+        }
+        if (!x && q0 + 2 >= NQ) p1_release<R>(ctl);  // this thread's last read of the box
+#pragma unroll 1
+        for (int q = q0;;) {
+            bool admL = true, admR = true;
+            if (doFlux) {  // in the flux range both sides are reconstructed
+                double F[NCONS];
+                face_flux<MODE>(P, uL, uR, F, admL, admR);
+                const double w = qw_at(d, R, q);
+#pragma unroll
+                for (int v = 0; v < NCONS; v++)
+                    if (S::var(v)) acc[v * NTHREADS] = acc[v * NTHREADS] + w * F[v];
+            } else {
+                if (needL) admL = state_adm<MODE>(P, uL);
+                if (needR) admR = state_adm<MODE>(P, uR);
+            }
+            if (!admL) bits |= 1;
+            if (!admR) bits |= 2;
+            if (q != q0 || !pair) break;
+            q++;
+            int k = 0;
+#pragma unroll
+            for (int v = 0; v < NCONS; v++) {
+                if (!S::var(v)) continue;
+                uL[v] = park[k++ * NTHREADS];
+                uR[v] = park[k++ * NTHREADS];
+            }
         }
     }
     if (doFlux) {
-        double* Fo = x ? d.FX : d.FY;
+        double* Fo = (x ? d.FX : d.FY) + c;
+        const long long sw = x ? 0 : G.plane;
 #pragma unroll
-        for (int v = 0; v < NCONS; v++) Fo[v * G.plane + c] = acc[v * NTHREADS];
-        (x ? d.CTX : d.CTY)[c] = acc[(x ? MAGY : MAGX) * NTHREADS];
+        for (int v = 0; v < NCONS; v++) {
+            const long long o = v * G.plane + (v == MOMN || v == MAGN ? sw : v == MOMT || v == MAGT ? -sw : 0);
+            Fo[o] = S::var(v) ? acc[v * NTHREADS] : 0.0;
+        }
+        (x ? d.CTX : d.CTY)[c] = S::var(MAGT) ? acc[MAGT * NTHREADS] : 0.0;
     }
     return bits;
 }
@@ -304,12 +406,24 @@ __device__ __noinline__ void pass1_fail(uint8_t* fail, int* list, int* count, in
     if (((old >> sh) & 0xffu) == 0) list[atomicAdd(count, 1)] = c;
 }
 
-// the x- and y-faces of one cell of the staged tile (sim_forceHydro fixed at
-// compile time)
-template <int R, int FH>
-__device__ __forceinline__ void pass1_tile(const Batch& B, const InstDev& d, const double* __restrict__ sU,
-                                           const double* __restrict__ sPv, const Cell& c, double* acc) {
+// the x- and y-faces of one cell (i, j) of the staged tile (the solver's mode
+// fixed at compile time).  Out of line, so that each mode has registers of
+// its own: inlined beside one another they spilled 112 loads a solve.  Shared
+// memory by offsets (doubles) of the box, the prediction vectors and this
+// thread's accumulators, which keeps the accesses shared-memory ones.
+struct P1Cell {
+    const InstDev* d;
+    InstState* S;
+    int* failList;
+    int init;
+    int i, j;
+    int box, pv, acc, ctl;  // offsets in doubles (ctl: 0 where the block stages itself)
+};
+template <int R, int MODE>
+static __device__ __noinline__ void pass1_tile(P1Cell c) {
+    extern __shared__ __align__(128) double smem[];
     using Box = P1Box<R>;
+    const InstDev& d = *c.d;
     const Geo& G = d.geo;
     const int i = c.i, j = c.j;
     const int g = G.g;
@@ -318,8 +432,8 @@ __device__ __forceinline__ void pass1_tile(const Batch& B, const InstDev& d, con
     const int sx = threadIdx.x + Box::OX, sy = threadIdx.y + Box::OY;
     const long long cc = (long long)j * G.pitch + i;
     const bool inF = i >= flo && i <= fxhi && j >= flo && j <= fyhi;
-    if (B.p1Init && i < G.nxt && j < G.nyt) {
-        d.scheme[B.st[c.k].schemeSel][cc] = (int8_t)R;
+    if (c.init && i < G.nxt && j < G.nyt) {
+        d.scheme[c.S->schemeSel][cc] = (int8_t)R;
         d.rrRec[cc] = (uint8_t)(R | (R << 2) | (R << 4) | (R << 6));
         d.rec[cc] = 0;
         d.recF[cc] = 0;
@@ -328,18 +442,66 @@ __device__ __forceinline__ void pass1_tile(const Batch& B, const InstDev& d, con
         d.dirty[cc] = 0;
         d.innerCount[cc] = 0;
     }
+    P1Ctl* ctl = c.ctl ? reinterpret_cast<P1Ctl*>(smem + c.ctl) : nullptr;
 #pragma unroll 1
     for (int dir = XDIR; dir <= YDIR; dir++) {  // the x-face, then the y-face of this cell
         const bool x = dir == XDIR;
         if (i >= clo && i <= cxhi + (x ? 1 : 0) && j >= clo && j <= cyhi + (x ? 0 : 1)) {
             const int a = x ? i : j, ahi = x ? cxhi : cyhi;
-            const uint8_t bits = pass1_face<R, FH>(d, sU, sPv, sx, sy, dir, a - 1 >= clo, a <= ahi, inF, cc, acc);
-            if (bits) {
-                int* list = reinterpret_cast<int*>(B.L.face + 2 * (long long)B.instTiles[c.k].x * (TILE_X * TILE_Y));
-                if (bits & 1) pass1_fail(d.fail, list, &B.st[c.k].cFail, (int)(x ? cc - 1 : cc - G.pitch));
-                if (bits & 2) pass1_fail(d.fail, list, &B.st[c.k].cFail, (int)cc);
-            }
+            const uint8_t bits = pass1_face<R, MODE>(d, smem + c.box, smem + c.pv, sx, sy, dir, a - 1 >= clo, a <= ahi,
+                                                     inF, cc, smem + c.acc, smem + c.acc + NCONS * NTHREADS, ctl);
+            if (bits & 1) pass1_fail(d.fail, c.failList, &c.S->cFail, (int)(x ? cc - 1 : cc - G.pitch));
+            if (bits & 2) pass1_fail(d.fail, c.failList, &c.S->cFail, (int)cc);
+        } else if (!x) {
+            p1_release<R>(ctl);
         }
+    }
+}
+
+// The faces of a staged tile in the solver's mode its data allow: a hydro run
+// has no field, and a planar flow has no out-of-plane momentum or field, so
+// those planes of the box are zeros, their face states and fluxes are zeros,
+// and their sums and products are left out (a quarter of an MHD cell's GP
+// sums, half of a hydro cell's).  Each warp looks at the rows its stencils
+// reach: fifteen loads of a plane pair, no block barrier.
+// SPEC: with the planar modes (the launch choice that large solves run).
+template <int R>
+__device__ __forceinline__ bool rows_nonzero(const double* sU, int plane) {
+    bool any = false;  // rows [y-1-R, y+R] of the warp's row y, 0-based row threadIdx.y of the box
+    const double* rows = sU + plane * P1Box<R>::PLANE + threadIdx.y * P1Box<R>::SX;
+    for (int e = threadIdx.x; e < (2 * R + 2) * P1Box<R>::SX; e += 32) any = any || !bits_zero(rows[e]);
+    return __any_sync(0xffffffffu, any);
+}
+template <int R, bool SPEC>
+__device__ __forceinline__ void pass1_tile_any(const Batch& B, int t, const double* sU, int pv, int acc, int ctl) {
+    extern __shared__ __align__(128) double smem[];
+    static_assert(TILE_X == 32, "a tile row is a warp");
+    const Cell cell = tile_at(B, t);
+    const InstDev& d = B.dev[cell.k];
+    P1Cell c;
+    c.d = &d;
+    c.S = B.st + cell.k;
+    c.failList = reinterpret_cast<int*>(B.L.face + 2 * (long long)B.instTiles[cell.k].x * (TILE_X * TILE_Y));
+    c.init = B.p1Init;
+    c.i = cell.i;
+    c.j = cell.j;
+    c.box = (int)(sU - smem);
+    c.pv = pv;
+    c.acc = acc;
+    c.ctl = ctl;
+    const bool z = !SPEC || rows_nonzero<R>(sU, MOMZ);
+    if (d.phys.force_hydro) {
+        if (rows_nonzero<R>(sU, MAGX) || rows_nonzero<R>(sU, MAGY) || rows_nonzero<R>(sU, MAGZ))
+            pass1_tile<R, SOLVE_HYDRO_FIELD>(c);
+        else if (z)
+            pass1_tile<R, SOLVE_HYDRO>(c);
+        else if (SPEC)
+            pass1_tile<R, SOLVE_HYDRO_PLANAR>(c);
+    } else {
+        if (z || rows_nonzero<R>(sU, MAGZ))
+            pass1_tile<R, SOLVE_MHD>(c);
+        else if (SPEC)
+            pass1_tile<R, SOLVE_MHD_PLANAR>(c);
     }
 }
 
@@ -374,6 +536,9 @@ __device__ __forceinline__ void mbar_fence_init() {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
 }
 // true once the barrier's phase `parity` has completed; false after kWaitCycles
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
@@ -459,16 +624,27 @@ __device__ __forceinline__ void pass1_stage(const Batch& B, int uin, int t, doub
 // the same staging by TMA: one (x, y, var) box of the stage input's tensor
 // map and one bulk copy of the prediction vectors, both completing on `bar`
 template <int R>
-__device__ __forceinline__ void pass1_stage_tma(const Batch& B, int uin, int t, double* dst, double* dstPv,
-                                                uint64_t* bar) {
+__device__ __forceinline__ void pass1_stage_tma(const InstDev& d, int par, int uin, const int4& tl, double* dst,
+                                                double* dstPv, uint64_t* bar) {
     using Box = P1Box<R>;
-    const int4 tl = B.tiles[t];
-    const InstDev& d = B.dev[tl.x];
-    const int par = B.st[tl.x].parity;
     const int u = uin == ROLE_STATE ? par : uin == ROLE_A ? 1 - par : 2;  // role_ptr's buffer index
     mbar_expect_tx(bar, (unsigned)((Box::DOUBLES + Box::PVN) * sizeof(double)));
     tma_box3(dst, &d.tmU[u], tl.y - Box::OX, tl.z - Box::OY, 0, bar);
     bulk_copy(dstPv, d.pv + (long long)Box::PVN * (R - 1), (unsigned)(Box::PVN * sizeof(double)), bar);
+}
+
+template <int R>
+static __device__ __noinline__ void p1_refill(P1Ctl* ctl) {
+    __threadfence_block();
+    ctl->released = 0;
+    const int t = ctl->next[++ctl->turn & 1];
+    if (t >= ctl->n) {  // nothing to copy: the waiting threads see the end
+        mbar_arrive(ctl->bar);
+        return;
+    }
+    const int4 tl = ctl->tiles[t];
+    const InstDev& d = ctl->dev[tl.x];
+    pass1_stage_tma<R>(d, ctl->st[tl.x].parity, ctl->uin, tl, ctl->box, ctl->pv, ctl->bar);
 }
 
 // One launch per radius: blocks skip tiles of instances with another GP
@@ -485,22 +661,27 @@ __device__ __forceinline__ void pass1_stage_tma(const Batch& B, int uin, int t, 
 // live: at two blocks per SM that wins over double-buffering on the 2048^2
 // workloads.  Three or four blocks per SM keep one box (their shared memory
 // would not fit two).
+constexpr int P1_THREAD = 3 * NCONS;  // doubles of shared memory per thread: accumulators, parked face states
 template <int R>
-struct P1Smem {  // dynamic shared memory layout (doubles): boxes, accumulators, prediction vectors, mbarriers
+struct P1Smem {  // dynamic shared memory layout (doubles): boxes, per-thread columns, prediction vectors, mbarriers
     static constexpr int box(int nbuf) { return nbuf * P1Box<R>::DOUBLES; }
     static constexpr int bytes(int nbuf) {
-        return (nbuf * P1Box<R>::DOUBLES + NCONS * NTHREADS + nbuf * P1Box<R>::PVN) * (int)sizeof(double) + 2 * 8;
+        return ctl(nbuf) * (int)sizeof(double) + (int)sizeof(P1Ctl);
+    }
+    static constexpr int ctl(int nbuf) {  // the control block, after the two mbarriers
+        return nbuf * P1Box<R>::DOUBLES + P1_THREAD * NTHREADS + nbuf * P1Box<R>::PVN + 2;
     }
 };
 template <int R, bool TMA, bool DYN, int MINB, int NBUF>
 __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin) { PDL_ENTRY();
     static_assert(NBUF == 1 || NBUF == 2, "one or two stencil boxes");
+    constexpr bool SPEC = TMA && MINB == 2 && NBUF == 1;
     extern __shared__ __align__(128) double smem[];
     __shared__ int sTile;  // the dynamic schedule's tile, as thread 0 took it
     using Box = P1Box<R>;
     const int tid = threadIdx.y * TILE_X + threadIdx.x;
-    double* acc = smem + P1Smem<R>::box(NBUF) + tid;
-    double* pvBuf = smem + P1Smem<R>::box(NBUF) + NCONS * NTHREADS;  // NBUF prediction-vector buffers
+    const int acc = P1Smem<R>::box(NBUF) + tid;
+    double* pvBuf = smem + P1Smem<R>::box(NBUF) + P1_THREAD * NTHREADS;  // NBUF prediction-vector buffers
     uint64_t* bars = reinterpret_cast<uint64_t*>(pvBuf + NBUF * Box::PVN);
     if (!(B.flags->radii & (1 << R))) return;  // no instance of this radius
     if (TMA) {
@@ -522,40 +703,53 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
         __syncthreads();
         return sTile;
     };
-    int t = next_tile(B.p1First + blockIdx.x);
-    int buf = 0;
-    if constexpr (NBUF == 1) {  // one box: load, compute, next
+    auto stage_tma = [&](int t, double* dst, double* dstPv, uint64_t* bar) {
+        const int4 tl = B.tiles[t];
+        pass1_stage_tma<R>(B.dev[tl.x], B.st[tl.x].parity, uin, tl, dst, dstPv, bar);
+    };
+    if constexpr (NBUF == 1 && !TMA) {  // one box: load, compute, next
+        int t = next_tile(B.p1First + blockIdx.x);
         while (t < n) {
-            if (!TMA) {
-                pass1_stage<R>(B, uin, t, smem, pvBuf, tid);
-                cp_async_wait<0>();
-            } else {
-                if (tid == 0) pass1_stage_tma<R>(B, uin, t, smem, pvBuf, bars);
-                const bool ok = mbar_wait(bars, phase & 1u);
-                phase ^= 1u;
-                if (!__syncthreads_and(ok)) {  // a copy that never lands: report it, leave without reading
-                    if (tid == 0) atomicExch(&B.flags->error, HOSONO_ETIMEOUT);
-                    return;
-                }
-            }
+            pass1_stage<R>(B, uin, t, smem, pvBuf, tid);
+            cp_async_wait<0>();
             __syncthreads();  // tile t's box is in place for every thread
-            const Cell c = tile_at(B, t);
-            const InstDev& d = B.dev[c.k];
-            // one instance per tile: the branch is uniform over the block
-            if (d.phys.force_hydro)
-                pass1_tile<R, 1>(B, d, smem, pvBuf, c, acc);
-            else
-                pass1_tile<R, 0>(B, d, smem, pvBuf, c, acc);
+            pass1_tile_any<R, SPEC>(B, t, smem, (int)(pvBuf - smem), acc, 0);
             __syncthreads();  // every read of this box is done before it is refilled
             t = next_tile(t + gridDim.x);
         }
         return;
     }
+    if constexpr (NBUF == 1 && TMA) {  // one box, refilled by the last thread that reads it
+        // A thread that finds the box of its turn in place knows that every
+        // thread has released the one before: the copy needs no block barrier.
+        constexpr int CTL = P1Smem<R>::ctl(1);
+        P1Ctl* ctl = reinterpret_cast<P1Ctl*>(smem + CTL);
+        if (tid == 0) {
+            *ctl = P1Ctl{B.dev, B.st, B.tiles, bars, smem, pvBuf, n, uin, {0, 0}, -1, 0};
+            ctl->next[0] = DYN ? pass1_take<R>(B, n) : pass1_next<R>(B, B.p1First + blockIdx.x, n);
+            p1_refill<R>(ctl);
+        }
+        __syncthreads();
+        for (int turn = 0;; turn++) {
+            if (!mbar_wait(bars, turn & 1)) {  // a copy that never lands: report it, leave without reading
+                atomicExch(&B.flags->error, HOSONO_ETIMEOUT);
+                return;
+            }
+            const int t = ctl->next[turn & 1];
+            if (t >= n) return;
+            __syncthreads();  // in step: warps apart evict one another's instructions (7 % slower)
+            // the next turn's tile, before this thread releases the box
+            if (tid == 0) ctl->next[(turn + 1) & 1] = DYN ? pass1_take<R>(B, n) : pass1_next<R>(B, t + gridDim.x, n);
+            pass1_tile_any<R, SPEC>(B, t, smem, (int)(pvBuf - smem), acc, CTL);
+        }
+    }
+    int t = next_tile(B.p1First + blockIdx.x);
+    int buf = 0;
     if (t < n) {
         if (!TMA)
             pass1_stage<R>(B, uin, t, smem, pvBuf, tid);
         else if (tid == 0)
-            pass1_stage_tma<R>(B, uin, t, smem, pvBuf, bars);
+            stage_tma(t, smem, pvBuf, bars);
     }
     while (t < n) {
         const int tn = next_tile(t + gridDim.x);
@@ -568,8 +762,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             }
         } else {
             if (tn < n && tid == 0)
-                pass1_stage_tma<R>(B, uin, tn, smem + (buf ^ 1) * Box::DOUBLES, pvBuf + (buf ^ 1) * Box::PVN,
-                                   bars + (buf ^ 1));
+                stage_tma(tn, smem + (buf ^ 1) * Box::DOUBLES, pvBuf + (buf ^ 1) * Box::PVN, bars + (buf ^ 1));
             const bool ok = mbar_wait(bars + buf, (phase >> buf) & 1u);
             phase ^= 1u << buf;
             if (!__syncthreads_and(ok)) {
@@ -581,14 +774,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             }
         }
         __syncthreads();  // tile t's box is in place for every thread
-        const double* sU = smem + buf * Box::DOUBLES;
-        const double* sPv = pvBuf + buf * Box::PVN;
-        const Cell c = tile_at(B, t);
-        const InstDev& d = B.dev[c.k];
-        if (d.phys.force_hydro)
-            pass1_tile<R, 1>(B, d, sU, sPv, c, acc);
-        else
-            pass1_tile<R, 0>(B, d, sU, sPv, c, acc);
+        pass1_tile_any<R, SPEC>(B, t, smem + buf * Box::DOUBLES, (int)(pvBuf - smem) + buf * Box::PVN, acc, 0);
         __syncthreads();  // every read of this box is done before it is refilled
         buf ^= 1;
         t = tn;

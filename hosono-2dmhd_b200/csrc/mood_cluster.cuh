@@ -226,8 +226,9 @@ __device__ __forceinline__ void mc_flux(const Mc& m, const int* list, int n, con
     const Geo& G = m.d.geo;
     const int f = m.lane >> 3, v = m.lane & 7;
     const bool x = f == EAST || f == WEST;
-    const int dir = x ? XDIR : YDIR;
     const int fL = x ? EAST : NORTH, fR = x ? WEST : SOUTH;
+    // variable v's place in face coordinates (physics.cuh)
+    const int vf = x ? v : v == MOMX || v == MAGX ? v + 1 : v == MOMY || v == MAGY ? v - 1 : v;
     for (int e = m.gw; e < n; e += m.nw) {
         const int c = list[e];
         const int cf = f == EAST ? c + 1 : f == NORTH ? c + G.pitch : c;  // the face's right / upper cell
@@ -242,10 +243,10 @@ __device__ __forceinline__ void mc_flux(const Mc& m, const int* list, int n, con
             double o[4] = {0.0, 0.0, 0.0, 0.0};
             mc_face_states(m, rrL, cl, fL, v, rr + 1, o);
 #pragma unroll
-            for (int q = 0; q < 4; q++) m.buf[f * MC_FS + (2 * q) * 8 + v] = o[q];
+            for (int q = 0; q < 4; q++) m.buf[f * MC_FS + (2 * q) * 8 + vf] = o[q];
             mc_face_states(m, rrR, cf, fR, v, rr + 1, o);
 #pragma unroll
-            for (int q = 0; q < 4; q++) m.buf[f * MC_FS + (2 * q + 1) * 8 + v] = o[q];
+            for (int q = 0; q < 4; q++) m.buf[f * MC_FS + (2 * q + 1) * 8 + vf] = o[q];
         }
         __syncwarp();
         double F[NCONS];
@@ -257,7 +258,7 @@ __device__ __forceinline__ void mc_flux(const Mc& m, const int* list, int n, con
                 uL[w] = m.buf[f * MC_FS + (2 * v) * 8 + w];
                 uR[w] = m.buf[f * MC_FS + (2 * v + 1) * 8 + w];
             }
-            hllc(m.P, uL, uR, dir, F);
+            hllc_face(m.P, uL, uR, F);
         }
         __syncwarp();
         if (solve) {
@@ -268,10 +269,10 @@ __device__ __forceinline__ void mc_flux(const Mc& m, const int* list, int n, con
         if (act) {
             double s;
             if (rr == 0) {
-                s = m.buf[f * MC_FS + v];
+                s = m.buf[f * MC_FS + vf];
             } else {
                 s = 0.0;
-                for (int q = 0; q <= rr; q++) s = s + m.sqw[q + G.nqMax * (rr - 1)] * m.buf[f * MC_FS + q * 8 + v];
+                for (int q = 0; q <= rr; q++) s = s + m.sqw[q + G.nqMax * (rr - 1)] * m.buf[f * MC_FS + q * 8 + vf];
             }
             (x ? m.d.FX : m.d.FY)[v * G.plane + cf] = s;
             if (v == (x ? MAGY : MAGX)) (x ? m.d.CTX : m.d.CTY)[cf] = s;

@@ -85,6 +85,17 @@ __device__ __forceinline__ double cons2pres(const Phys& s, const double* U) {
     return (s.gamma - 1.0) * (U[ENER] - Bp - 0.5 * msq / U[DENS]);
 }
 
+// src/detect.f90:250-265 (CAD) and :238-248 (PAD): both finite (not NaN,
+// not infinite) and both > 0, i.e. each bit pattern is a positive, nonzero,
+// finite double (tested on the integer pipes)
+__device__ __forceinline__ bool positive_finite(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return u - 1ull < 0x7fefffffffffffffull;  // u in [1, 0x7fefffffffffffff]
+}
+__device__ __forceinline__ bool admissible(double dens, double pres) {
+    return positive_finite(dens) && positive_finite(pres);
+}
+
 // src/eigen.f90:305-321 (Ryu & Jones 1995, eqs. 2.18-2.19)
 __device__ __forceinline__ double c_fs(double gam, double rho, double p, double BB, double B_N, double pm) {
     double c = (gam * p + BB) / rho;
@@ -96,248 +107,448 @@ __device__ __forceinline__ double dot3(double a0, double a1, double a2, double b
     return (0.0 + a0 * b0) + a1 * b1 + a2 * b2;
 }
 
-// Division policies for the Riemann solver.  Most of its quotients come in
-// groups with one denominator (the density of a side, sR - sL, the HLL
-// density, sK - sStar).
-//
-// IeeeDiv divides each one ('/': IEEE, correctly rounded).
-//
-// SharedRecipDiv takes y = RN(1/b) once per group (__drcp_rn, correctly
-// rounded) and each quotient by Markstein's theorem (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34(1), 1990): when y = RN(1/b) and q is within one ulp of a/b, the
-// remainder r = a - b*q is exact and RN(q + r*y) = RN(a/b).  q0 = RN(a*y) is
-// within two ulps of a/b; one correction q1 = RN(q0 + y*RN(a - b*q0)) brings
-// it within one ulp, and a second gives the correctly rounded quotient -- the
-// same bits as '/' (tests/div_check.cu compares the two on the GPU).  The
-// proof assumes no overflow, underflow or subnormal in a, b, a*y and the
-// remainders; every operand outside [2^-500, 2^501) (zero
-// numerators excepted) clears `ok`, and the caller then recomputes the whole
-// solve with IeeeDiv.  Cost per quotient: one multiply and four FMAs, no
-// branch.
-struct IeeeDiv {
-    struct R {
-        double b;
-    };
-    bool ok = true;
-    __device__ __forceinline__ R recip(double b) { return R{b}; }
-    __device__ __forceinline__ double div(double a, const R& r) { return a / r.b; }
+// ---- division by shared denominators.  Most quotients of the Riemann solver
+// come in groups with one denominator (the density of a side, sR - sL, the
+// HLL density, sK - sStar).  SharedRecip holds b, y = RN(1/b) (__drcp_rn,
+// correctly rounded) and z, the rest of 1/b rounded, so y + z is 1/b to twice
+// the precision; shared_quot then takes each quotient in four operations:
+// q0 = fma(a, y, a*z) is within one ulp of a/b, and by Markstein's theorem
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990; a reciprocal kept in
+// two parts: N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating correctly
+// rounded floating-point division when the divisor is known in advance", IEEE
+// Trans. Comput. 53(8), 2004) the remainder r = a - b*q0 is exact and
+// RN(q0 + r*y) = RN(a/b): the same bits as '/', whose sign a zero quotient
+// takes from the operands (tests/div_check.cu compares the two on the GPU).
+// Without a*z, q0 = RN(a*y) is up to two ulps off and takes a second
+// correction per quotient.  The proof assumes no overflow, underflow or
+// subnormal on the way, which the operand ranges of GroupDiv guarantee.  A zero
+// quotient is +0; with_sign gives it the operands' sign, which the solver does
+// not need: no expression of it tells the zeros apart.
+struct SharedRecip {
+    double b, y, z;
 };
+__device__ __forceinline__ SharedRecip shared_recip(double b) {
+    const double y = __drcp_rn(b);
+    return SharedRecip{b, y, fma(-b, y, 1.0) * y};
+}
+__device__ __forceinline__ double shared_quot(double a, const SharedRecip& r) {
+    const double q0 = fma(a, r.y, a * r.z);
+    return fma(fma(-r.b, q0, a), r.y, q0);
+}
+__device__ __forceinline__ double with_sign(double q, double a, double b) {
+    const int sign = (__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000;
+    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | sign, __double2loint(q));
+}
+// Quotients with their operand ranges watched: |b| in [2^DLO, 2^(DHI+1)), a
+// zero or |a| in [2^NLO, 2^(NHI+1)).  The smallest and largest exponents seen
+// are kept as integer keys (the magnitude's high word, one bit for the rest),
+// four integer instructions a numerator, and compared once.
+template <int NLO, int NHI, int DLO, int DHI>
+struct GroupDiv {
+    unsigned nmin = ~0u, nmax = 0u, dmin = ~0u, dmax = 0u;
+    __device__ __forceinline__ SharedRecip recip(double b) {
+        watch(b);
+        return shared_recip(b);
+    }
+    // a value that has to lie in the denominators' range
+    __device__ __forceinline__ void watch(double b) {
+        const unsigned k = (unsigned)__double2hiint(b) << 1;
+        dmin = min(dmin, k);
+        dmax = max(dmax, k);
+    }
+    __device__ __forceinline__ double div(double a, const SharedRecip& r) {
+        const unsigned k = ((unsigned)__double2hiint(a) << 1) + min((unsigned)__double2loint(a), 1u);
+        nmin = min(nmin, k - 1u);  // a zero wraps to the top
+        nmax = max(nmax, k);
+        return shared_quot(a, r);
+    }
+    __device__ __forceinline__ bool ok() const {
+        return nmin >= ((1023u + NLO) << 21) - 1u && nmax < ((1024u + NHI) << 21) && dmin >= ((1023u + DLO) << 21) &&
+               dmax < ((1024u + DHI) << 21);
+    }
+};
+// The solver's ranges: b in [2^-100, 2^101) and a down to 2^-860 keep every
+// intermediate normal (the quotient above 2^-962, the remainder a multiple of
+// 2^-965); momenta ahead of a front fall off by orders of magnitude a cell, so
+// the numerators' range is the wide one.
+typedef GroupDiv<-860, 900, -100, 100> SolverDiv;
+// one quotient at a time over a symmetric range, as tests/div_check.cu drives it
 struct SharedRecipDiv {
-    struct R {
-        double b, y;
-    };
+    GroupDiv<-500, 500, -500, 500> g;
     bool ok = true;
-    // |x| in [2^-500, 2^501), from the exponent bits (integer pipes)
-    __device__ __forceinline__ static bool in_range(unsigned long long mag) {
-        return (unsigned)((int)(mag >> 52) - (1023 - 500)) <= 1000u;
-    }
-    __device__ __forceinline__ R recip(double b) {
-        ok = ok && in_range((unsigned long long)__double_as_longlong(b) & 0x7fffffffffffffffull);
-        return R{b, __drcp_rn(b)};
-    }
-    __device__ __forceinline__ double div(double a, const R& r) {
-        const unsigned long long mag = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
-        ok = ok && (mag == 0 || in_range(mag));
-        const double q0 = a * r.y;
-        const double q1 = fma(fma(-r.b, q0, a), r.y, q0);
-        const double q2 = fma(fma(-r.b, q1, a), r.y, q1);
-        return mag == 0 ? q0 : q2;  // a = +-0: q0 carries the sign of the IEEE quotient
+    __device__ __forceinline__ SharedRecip recip(double b) { return g.recip(b); }
+    __device__ __forceinline__ double div(double a, const SharedRecip& r) {
+        const double q = g.div(a, r);
+        ok = g.ok();
+        return with_sign(q, a, r.b);
     }
 };
 
-// The primitive variables HLLC reads from one side: cons2prim
-// (convert.f90:198-234) without eint; b* are zero for a hydro run.
-template <class D>
-struct Side {
-    double rho, vx, vy, vz, p, bx, by, bz;
-    typename D::R rrho;  // the density as a shared denominator
+// ---- src/riemannSolver.f90:68-221 (HLLC for MHD, Li 2005) in face
+// coordinates: N the normal, T the other in-plane component, Z out of plane.
+// A y-face is the x-face of the state with x and y exchanged, bit for bit:
+// the solver's sums over components are of two commuted in-plane terms, then
+// the z term, so no expression's rounding changes.
+enum : int { MOMN = 1, MOMT = 2, MOMZ_ = 3, MAGN = 5, MAGT = 6, MAGZ_ = 7 };
+
+// The solver with IEEE division, statement by statement: for the operands the
+// shared-denominator form does not take, and hydro runs whose conserved
+// state carries a field.  What the chosen branch does not read is not
+// computed.
+template <int FH>
+struct IeeeSide {
+    double rho, v[3], p, b[3];
 };
-template <int FH, class D>
-__device__ __forceinline__ void side_prim(const Phys& s, const double* U, Side<D>& V, D& dv) {
+template <int FH>
+__device__ __forceinline__ void ieee_prim(const Phys& s, const double* U, IeeeSide<FH>& V) {
     double Bp;
     if (hydro<FH>(s))
         Bp = 0.0;
     else
-        Bp = 0.5 * (U[MAGX] * U[MAGX] + U[MAGY] * U[MAGY] + U[MAGZ] * U[MAGZ]);
-    const double density = U[DENS];
-    V.rho = density;
-    V.rrho = dv.recip(density);
-    V.vx = dv.div(U[MOMX], V.rrho);
-    V.vy = dv.div(U[MOMY], V.rrho);
-    V.vz = dv.div(U[MOMZ], V.rrho);
-    const double eint = dv.div(U[ENER] - Bp, V.rrho) - 0.5 * (V.vx * V.vx + V.vy * V.vy + V.vz * V.vz);
-    V.p = eos_pres(s, density, eint);
-    V.bx = hydro<FH>(s) ? 0.0 : U[MAGX];
-    V.by = hydro<FH>(s) ? 0.0 : U[MAGY];
-    V.bz = hydro<FH>(s) ? 0.0 : U[MAGZ];
+        Bp = 0.5 * (U[5] * U[5] + U[6] * U[6] + U[7] * U[7]);
+    V.rho = U[DENS];
+    for (int k = 0; k < 3; k++) {
+        V.v[k] = U[1 + k] / V.rho;
+        V.b[k] = hydro<FH>(s) ? 0.0 : U[5 + k];
+    }
+    const double eint = (U[ENER] - Bp) / V.rho - 0.5 * (V.v[0] * V.v[0] + V.v[1] * V.v[1] + V.v[2] * V.v[2]);
+    V.p = eos_pres(s, V.rho, eint);
 }
-template <class D>
-__device__ __forceinline__ double side_vel(const Side<D>& V, int c) {
-    return c == 0 ? V.vx : c == 1 ? V.vy : V.vz;
-}
-template <class D>
-__device__ __forceinline__ double side_mag(const Side<D>& V, int c) {
-    return c == 0 ? V.bx : c == 1 ? V.by : V.bz;
-}
-
 // fast magnetosonic speed of one side or of the average state (eigen.f90:257-303)
-__device__ __forceinline__ double side_cf(const Phys& s, double rho0, double p0, double bx, double by, double bz,
-                                          double bN) {
+__device__ __forceinline__ double side_cf(const Phys& s, double rho0, double p0, double bN, double bT, double bZ) {
     const double rho = fmax(rho0, s.small_density);
     const double p = fmax(p0, s.small_pressure);
-    const double BB = bx * bx + by * by + bz * bz;
+    const double BB = bN * bN + bT * bT + bZ * bZ;
     return c_fs(s.gamma, rho, p, BB, bN, +1.0);
 }
-
-// cons2flux (convert.f90:28-92) of one side
-template <int FH, class D>
-__device__ __forceinline__ void side_flux(const Phys& s, const double* U, const Side<D>& V, int dir, double* F,
-                                          D& dv) {
+// cons2flux (convert.f90:28-92)
+template <int FH>
+__device__ __forceinline__ void ieee_flux(const Phys& s, const double* U, const IeeeSide<FH>& V, double* F) {
     double Bp = 0.0;
-    if (!hydro<FH>(s)) Bp = 0.5 * (U[MAGX] * U[MAGX] + U[MAGY] * U[MAGY] + U[MAGZ] * U[MAGZ]);
-    const double E = U[ENER];
+    if (!hydro<FH>(s)) Bp = 0.5 * (U[5] * U[5] + U[6] * U[6] + U[7] * U[7]);
     const double Ptot = V.p + Bp;
-    // normal (N) and tangential (T1, T2 = z) components; the array slots are
-    // chosen by selects, so a run-time dir keeps F and U in registers
-    const bool x = dir == XDIR;
-    const double vN = side_vel(V, dir), vT1 = side_vel(V, 1 - dir), vT2 = V.vz;
-    const double BN = side_mag(V, dir), BT1 = side_mag(V, 1 - dir), BT2 = V.bz;
-    const double mN = x ? U[MOMX] : U[MOMY];
-    double fN = dv.div(mN * mN, V.rrho) + Ptot;
-    double fT1 = mN * vT1;
-    double fT2 = mN * vT2;
-    double fE = (E + Ptot) * vN;
-    double gT1 = 0.0, gT2 = 0.0;  // induction fluxes; the normal one is 0
+    F[DENS] = U[MOMN];
+    F[MOMN] = U[MOMN] * U[MOMN] / V.rho + Ptot;
+    F[MOMT] = U[MOMN] * V.v[1];
+    F[MOMZ_] = U[MOMN] * V.v[2];
+    F[ENER] = (U[ENER] + Ptot) * V.v[0];
+    F[MAGN] = F[MAGT] = F[MAGZ_] = 0.0;
     if (!hydro<FH>(s)) {
-        fN = fN - BN * BN;
-        fT1 = fT1 - BT1 * BN;
-        fT2 = fT2 - BT2 * BN;
-        gT1 = vN * BT1 - vT1 * BN;
-        gT2 = vN * BT2 - vT2 * BN;
-        fE = fE - BN * (V.vx * V.bx + V.vy * V.by + V.vz * V.bz);
+        F[MOMN] = F[MOMN] - V.b[0] * V.b[0];
+        F[MOMT] = F[MOMT] - V.b[1] * V.b[0];
+        F[MOMZ_] = F[MOMZ_] - V.b[2] * V.b[0];
+        F[MAGT] = V.v[0] * V.b[1] - V.v[1] * V.b[0];
+        F[MAGZ_] = V.v[0] * V.b[2] - V.v[2] * V.b[0];
+        F[ENER] = F[ENER] - V.b[0] * (V.v[0] * V.b[0] + V.v[1] * V.b[1] + V.v[2] * V.b[2]);
     }
-    F[DENS] = mN;
-    F[MOMX] = x ? fN : fT1;
-    F[MOMY] = x ? fT1 : fN;
-    F[MOMZ] = fT2;
-    F[ENER] = fE;
-    F[MAGX] = x ? 0.0 : gT1;
-    F[MAGY] = x ? gT1 : 0.0;
-    F[MAGZ] = gT2;
 }
-
-// src/riemannSolver.f90:68-221 (HLLC for MHD, Li 2005).  Every value keeps
-// the reference's expression; what the chosen branch does not read is not
-// computed: a supersonic face (flux = fL or fR) evaluates one physical flux
-// and no HLL or star state, and the star state is evaluated once, on the
-// operands of the chosen side.
-template <int FH, class D>
-__device__ __forceinline__ void hllc_t(const Phys& s, const double* uL, const double* uR, int dir, double* flux,
-                                       D& dv) {
-    Side<D> L, R;
-    side_prim<FH>(s, uL, L, dv);
-    side_prim<FH>(s, uR, R, dv);
-    // array slots of the normal / first tangential components are chosen by
-    // selects, so a run-time dir keeps every array in registers
-    const bool x = dir == XDIR;
-    const double velNL = side_vel(L, dir), velNR = side_vel(R, dir);
-    const double magNL = side_mag(L, dir), magNR = side_mag(R, dir);
+template <int FH>
+__device__ __forceinline__ void ieee_solve(const Phys& s, const double* uL, const double* uR, double* flux) {
+    IeeeSide<FH> L, R;
+    ieee_prim<FH>(s, uL, L);
+    ieee_prim<FH>(s, uR, R);
     // eigenvalues 1 and 7 of L, R and the arithmetic average (riemannSolver.f90:84-96)
-    const double eL1 = velNL - side_cf(s, L.rho, L.p, L.bx, L.by, L.bz, magNL);
-    const double eR7 = velNR + side_cf(s, R.rho, R.p, R.bx, R.by, R.bz, magNR);
-    double sL, sR;
-    {
-        const double vNA = (velNL + velNR) / 2.0;
-        const double cfA = side_cf(s, (L.rho + R.rho) / 2.0, (L.p + R.p) / 2.0, (L.bx + R.bx) / 2.0,
-                                   (L.by + R.by) / 2.0, (L.bz + R.bz) / 2.0, (magNL + magNR) / 2.0);
-        sL = fmin(eL1, vNA - cfA);
-        sR = fmax(vNA + cfA, eR7);
-    }
-    const double rhoL = L.rho, rhoR = R.rho;
-    const double pTotL = L.p + 0.5 * dot3(L.bx, L.by, L.bz, L.bx, L.by, L.bz);
-    const double pTotR = R.p + 0.5 * dot3(R.bx, R.by, R.bz, R.bx, R.by, R.bz);
-    const double dL = sL - velNL, dR = sR - velNR;
-    const double mNL = x ? uL[MOMX] : uL[MOMY], mNR = x ? uR[MOMX] : uR[MOMY];
-    const double sStr = (mNR * dR - mNL * dL + pTotL - pTotR - magNL * magNL + magNR * magNR) /
-                        (rhoR * dR - rhoL * dL);
+    const double vNA = (L.v[0] + R.v[0]) / 2.0;
+    const double cfA = side_cf(s, (L.rho + R.rho) / 2.0, (L.p + R.p) / 2.0, (L.b[0] + R.b[0]) / 2.0,
+                               (L.b[1] + R.b[1]) / 2.0, (L.b[2] + R.b[2]) / 2.0);
+    const double sL = fmin(L.v[0] - side_cf(s, L.rho, L.p, L.b[0], L.b[1], L.b[2]), vNA - cfA);
+    const double sR = fmax(vNA + cfA, R.v[0] + side_cf(s, R.rho, R.p, R.b[0], R.b[1], R.b[2]));
+    const double pTotL = L.p + 0.5 * dot3(L.b[0], L.b[1], L.b[2], L.b[0], L.b[1], L.b[2]);
+    const double pTotR = R.p + 0.5 * dot3(R.b[0], R.b[1], R.b[2], R.b[0], R.b[1], R.b[2]);
+    const double dL = sL - L.v[0], dR = sR - R.v[0];
+    const double sStr = (uR[MOMN] * dR - uL[MOMN] * dL + pTotL - pTotR - L.b[0] * L.b[0] + R.b[0] * R.b[0]) /
+                        (R.rho * dR - L.rho * dL);
     // final choice (riemannSolver.f90:189-219): fL if 0 < sL; left star state
     // if sL <= 0 < sStr; right star state if sStr <= 0 <= sR; fR otherwise.
-    int side;
-    if (0.0 < sL)
-        side = 0;
-    else if ((sL <= 0.0) && (0.0 < sStr))
-        side = 1;
-    else if ((sStr <= 0.0) && (0.0 <= sR))
-        side = 2;
-    else
-        side = 3;
+    const int side = 0.0 < sL ? 0 : (sL <= 0.0) && (0.0 < sStr) ? 1 : (sStr <= 0.0) && (0.0 <= sR) ? 2 : 3;
+    double fL[NCONS], fR[NCONS], uHLL[NCONS], uStr[NCONS];
+    ieee_flux<FH>(s, uL, L, fL);
+    ieee_flux<FH>(s, uR, R, fR);
     if (side == 0 || side == 3) {
-        if (side == 0)
-            side_flux<FH>(s, uL, L, dir, flux, dv);
-        else
-            side_flux<FH>(s, uR, R, dir, flux, dv);
+        for (int v = 0; v < NCONS; v++) flux[v] = side == 0 ? fL[v] : fR[v];
         return;
     }
+    for (int v = 0; v < NCONS; v++) uHLL[v] = (sR * uR[v] - sL * uL[v] + fL[v] - fR[v]) / (sR - sL);
+    const double magDotVelHLL = dot3(uHLL[5], uHLL[6], uHLL[7], uHLL[1] / uHLL[0], uHLL[2] / uHLL[0], uHLL[3] / uHLL[0]);
+    const double pStr = L.rho * dL * (sStr - L.v[0]) + pTotL - L.b[0] * L.b[0] + uHLL[MAGN] * uHLL[MAGN];
+    const bool left = side == 1;
+    const IeeeSide<FH>& K = left ? L : R;
+    const double* uK = left ? uL : uR;
+    const double sK = left ? sL : sR, dK = left ? dL : dR, pTotK = left ? pTotL : pTotR;
+    const double magDotVelK = dot3(K.b[0], K.b[1], K.b[2], K.v[0], K.v[1], K.v[2]);
+    uStr[DENS] = K.rho * dK / (sK - sStr);
+    uStr[MOMN] = uStr[DENS] * sStr;
+    uStr[MOMT] = uStr[DENS] * K.v[1] - (uHLL[MAGN] * uHLL[MAGT] - K.b[0] * K.b[1]) / (sK - sStr);
+    uStr[MOMZ_] = uStr[DENS] * K.v[2] - (uHLL[MAGN] * uHLL[MAGZ_] - K.b[0] * K.b[2]) / (sK - sStr);
+    uStr[MAGN] = uHLL[MAGN];
+    uStr[MAGT] = uHLL[MAGT];
+    uStr[MAGZ_] = uHLL[MAGZ_];
+    uStr[ENER] = uK[ENER] * dK + pStr * sStr - pTotK * K.v[0] - uHLL[MAGN] * magDotVelHLL + K.b[0] * magDotVelK;
+    uStr[ENER] = uStr[ENER] / (sK - sStr);
+    for (int v = 0; v < NCONS; v++) flux[v] = (left ? fL[v] : fR[v]) + sK * (uStr[v] - uK[v]);
+}
+// out of line and by value: a pointer to the caller's states would keep them
+// in local memory on the common path too
+struct Cons8 {
+    double v[NCONS];
+};
+template <int FH>
+static __device__ __noinline__ Cons8 hllc_ieee(Phys s, Cons8 uL, Cons8 uR) {
+    Cons8 F;
+    ieee_solve<FH>(s, uL.v, uR.v, F.v);
+    return F;
+}
+
+// What a solve may leave out, because its terms are zeros (bits: a sum with
+// them, and a product kept under another sum, has the same value without):
+// out-of-plane momentum and field of a planar flow, the field of a hydro run.
+// SOLVE_HYDRO_FIELD: a hydro run whose conserved state carries a field, which
+// the solver reads in its HLL state (IEEE form only).
+enum : int { SOLVE_MHD = 0, SOLVE_MHD_PLANAR = 1, SOLVE_HYDRO = 2, SOLVE_HYDRO_PLANAR = 3, SOLVE_HYDRO_FIELD = 4 };
+template <int MODE>
+struct Solve {
+    static constexpr bool H = MODE >= SOLVE_HYDRO;            // hydro: no field
+    static constexpr bool Z = (MODE & 1) == 0;                // out-of-plane momentum
+    static constexpr bool BZ = MODE == SOLVE_MHD;             // out-of-plane field
+    static constexpr __host__ __device__ bool var(int v) {   // state variables it reads
+        return MODE == SOLVE_HYDRO_FIELD || v < 3 || v == ENER || (v == MOMZ_ && Z) || (!H && (v == MAGN || v == MAGT)) || (BZ && v == MAGZ_);
+    }
+};
+template <int MODE>
+struct FaceSide {
+    double rho, vN, vT, vZ, p, bN, bT, bZ, Bp, cf;
+    SharedRecip r;
+};
+// the primitive variables of one side (cons2prim, convert.f90:198-234), its
+// fast speed; returns CAD and PAD on its density and cons2pres
+// (convert.f90:236-254, not floored).  A density below the floor that
+// eigen.f90 applies goes to the IEEE form.
+template <int MODE>
+__device__ __forceinline__ bool side_eval(const Phys& s, const double* U, FaceSide<MODE>& V, SolverDiv& g, bool& floored) {
+    typedef Solve<MODE> S;
+    V.rho = U[DENS];
+    V.r = g.recip(V.rho);
+    floored = floored || V.rho < s.small_density;
+    double BB = 0.0;
+    V.Bp = V.bN = V.bT = V.bZ = 0.0;
+    if (!S::H) {
+        V.bN = U[MAGN];
+        V.bT = U[MAGT];
+        BB = V.bN * V.bN + V.bT * V.bT;
+        if (S::BZ) {
+            V.bZ = U[MAGZ_];
+            BB = BB + V.bZ * V.bZ;
+        }
+        V.Bp = 0.5 * BB;
+    }
+    const double EB = S::H ? U[ENER] : U[ENER] - V.Bp;
+    double msq = U[MOMN] * U[MOMN] + U[MOMT] * U[MOMT];
+    if (S::Z) msq = msq + U[MOMZ_] * U[MOMZ_];
+    const bool adm = admissible(V.rho, (s.gamma - 1.0) * (EB - g.div(0.5 * msq, V.r)));
+    V.vN = g.div(U[MOMN], V.r);
+    V.vT = g.div(U[MOMT], V.r);
+    V.vZ = S::Z ? g.div(U[MOMZ_], V.r) : 0.0;
+    double vsq = V.vN * V.vN + V.vT * V.vT;
+    if (S::Z) vsq = vsq + V.vZ * V.vZ;
+    V.p = eos_pres(s, V.rho, g.div(EB, V.r) - 0.5 * vsq);
+    // c_fs (eigen.f90:305-321) of the floored state, whose floors hold here
+    if (S::H) {
+        // the discriminant is c*c, whose root is c (rounding to nearest, no
+        // overflow or underflow: c is watched), and 0.5*(c + c) = c
+        const double c = g.div(s.gamma * V.p, V.r);
+        g.watch(c);
+        V.cf = sqrt(fmax(1.0e-14, c));
+    } else {
+        const double c = g.div(s.gamma * V.p + BB, V.r);
+        V.cf = sqrt(fmax(1.0e-14,
+                         0.5 * (c + sqrt(c * c - 4.0 * s.gamma * V.p * (V.bN * V.bN) / (V.rho * V.rho)))));
+    }
+    return adm;
+}
+// the flux of one side (cons2flux, convert.f90:28-92) without the energy
+template <int MODE>
+__device__ __forceinline__ void side_flux(const double* U, const FaceSide<MODE>& V, double* F, SolverDiv& g) {
+    typedef Solve<MODE> S;
+    const double Ptot = V.p + V.Bp;
+    F[DENS] = U[MOMN];
+    F[MOMN] = g.div(U[MOMN] * U[MOMN], V.r) + Ptot;
+    F[MOMT] = U[MOMN] * V.vT;
+    if (S::Z) F[MOMZ_] = U[MOMN] * V.vZ;
+    if (!S::H) {
+        F[MOMN] = F[MOMN] - V.bN * V.bN;
+        F[MOMT] = F[MOMT] - V.bT * V.bN;
+        if (S::Z) F[MOMZ_] = F[MOMZ_] - V.bZ * V.bN;
+        F[MAGT] = V.vN * V.bT - V.vT * V.bN;
+        if (S::BZ) F[MAGZ_] = V.vN * V.bZ - V.vZ * V.bN;
+    }
+}
+// HLLC in face coordinates with shared denominators; false when an operand
+// left their range (flux is then not to be used).  The variables the mode
+// leaves out are not read and not written.  admL, admR: CAD and PAD of the
+// sides.
+template <int MODE>
+__device__ __forceinline__ bool face_solve(const Phys& s, const double* uL, const double* uR, double* flux,
+                                           bool& admL, bool& admR) {
+    typedef Solve<MODE> S;
+    SolverDiv g;
+    bool floored = false;
+    FaceSide<MODE> L, R;
+    admL = side_eval<MODE>(s, uL, L, g, floored);
+    admR = side_eval<MODE>(s, uR, R, g, floored);
+    // eigenvalues 1 and 7 of L, R and the arithmetic average (riemannSolver.f90:84-96)
+    double cfA;
+    {
+        const double rho = (L.rho + R.rho) / 2.0, p = (L.p + R.p) / 2.0;
+        if (S::H) {
+            const double c = s.gamma * p / rho;
+            g.watch(c);
+            cfA = sqrt(fmax(1.0e-14, c));
+        } else {
+            const double bN = (L.bN + R.bN) / 2.0, bT = (L.bT + R.bT) / 2.0;
+            double BB = bN * bN + bT * bT;
+            if (S::BZ) {
+                const double bZ = (L.bZ + R.bZ) / 2.0;
+                BB = BB + bZ * bZ;
+            }
+            cfA = c_fs(s.gamma, rho, p, BB, bN, +1.0);
+        }
+    }
+    const double vNA = (L.vN + R.vN) / 2.0;
+    const double sL = fmin(L.vN - L.cf, vNA - cfA);
+    const double sR = fmax(vNA + cfA, R.vN + R.cf);
+    const double pTotL = L.p + L.Bp, pTotR = R.p + R.Bp;
+    const double dL = sL - L.vN, dR = sR - R.vN;
+    double num = uR[MOMN] * dR - uL[MOMN] * dL + pTotL - pTotR;
+    if (!S::H) num = num - L.bN * L.bN + R.bN * R.bN;
+    const double sStr = num / (R.rho * dR - L.rho * dL);
+    // final choice (riemannSolver.f90:189-219): fL if 0 < sL; left star state
+    // if sL <= 0 < sStr; right star state if sStr <= 0 <= sR; fR otherwise.
+    const bool left = 0.0 < sL || ((sL <= 0.0) && (0.0 < sStr));
+    const bool star = !(0.0 < sL) && (left || ((sStr <= 0.0) && (0.0 <= sR)));
     double fL[NCONS], fR[NCONS];
-    side_flux<FH>(s, uL, L, dir, fL, dv);
-    side_flux<FH>(s, uR, R, dir, fR, dv);
-    double uHLL[NCONS];
-    const typename D::R rS = dv.recip(sR - sL);
+    side_flux<MODE>(uL, L, fL, g);
+    side_flux<MODE>(uR, R, fR, g);
+    // the chosen side
+    const double vNK = left ? L.vN : R.vN, pTotK = left ? pTotL : pTotR, bNK = left ? L.bN : R.bN;
+    const double eK = left ? uL[ENER] : uR[ENER];
+    double bDotV = 0.0;  // of the chosen side
+    double fE = (eK + pTotK) * vNK;
+    if (!S::H) {
+        const double vTK = left ? L.vT : R.vT, bTK = left ? L.bT : R.bT;
+        bDotV = vNK * bNK + vTK * bTK;
+        if (S::BZ) bDotV = bDotV + (left ? L.vZ : R.vZ) * (left ? L.bZ : R.bZ);
+        fE = fE - bNK * bDotV;
+    }
 #pragma unroll
     for (int v = 0; v < NCONS; v++)
-        if (v != ENER) uHLL[v] = dv.div(sR * uR[v] - sL * uL[v] + fL[v] - fR[v], rS);
-    const typename D::R rH = dv.recip(uHLL[DENS]);
-    const double velHx = dv.div(uHLL[MOMX], rH);
-    const double velHy = dv.div(uHLL[MOMY], rH);
-    const double velHz = dv.div(uHLL[MOMZ], rH);
-    const double magDotVelHLL = dot3(uHLL[MAGX], uHLL[MAGY], uHLL[MAGZ], velHx, velHy, velHz);
-    const double magNHLL = x ? uHLL[MAGX] : uHLL[MAGY];
-    const double magT1HLL = x ? uHLL[MAGY] : uHLL[MAGX];
-    const double pStr = rhoL * dL * (sStr - velNL) + pTotL - magNL * magNL + magNHLL * magNHLL;
-    const bool left = side == 1;
-    const Side<D>& K = left ? L : R;
-    const double sK = left ? sL : sR;
-    const double dK = left ? dL : dR;
-    const double velNK = left ? velNL : velNR;
-    const double pTotK = left ? pTotL : pTotR;
-    const double magNK = left ? magNL : magNR;
-    const double magDotVelK = dot3(K.bx, K.by, K.bz, K.vx, K.vy, K.vz);
-    const double vT1K = side_vel(K, 1 - dir), vT2K = K.vz;
-    const double bT1K = side_mag(K, 1 - dir), bT2K = K.bz;
-    const double eK = left ? uL[ENER] : uR[ENER];
-    const typename D::R rK = dv.recip(sK - sStr);
-    double uStr[NCONS];
-    uStr[DENS] = dv.div(K.rho * dK, rK);
-    const double sN = uStr[DENS] * sStr;
-    const double sT1 = uStr[DENS] * vT1K - dv.div(magNHLL * magT1HLL - magNK * bT1K, rK);
-    const double sT2 = uStr[DENS] * vT2K - dv.div(magNHLL * uHLL[MAGZ] - magNK * bT2K, rK);
-    uStr[MOMX] = x ? sN : sT1;
-    uStr[MOMY] = x ? sT1 : sN;
-    uStr[MOMZ] = sT2;
-    uStr[MAGX] = x ? magNHLL : magT1HLL;
-    uStr[MAGY] = x ? magT1HLL : magNHLL;
-    uStr[MAGZ] = uHLL[MAGZ];
-    uStr[ENER] = eK * dK + pStr * sStr - pTotK * velNK - magNHLL * magDotVelHLL + magNK * magDotVelK;
-    uStr[ENER] = dv.div(uStr[ENER], rK);
+        if (S::var(v)) flux[v] = v == ENER ? fE : v == MAGN ? 0.0 : left ? fL[v] : fR[v];
+    if (star) {
+        const double sK = left ? sL : sR, dK = left ? dL : dR;
+        const double rhoK = left ? L.rho : R.rho, vTK = left ? L.vT : R.vT;
+        const SharedRecip rK = g.recip(sK - sStr);
+        double uStr[NCONS];
+        uStr[DENS] = g.div(rhoK * dK, rK);
+        uStr[MOMN] = uStr[DENS] * sStr;
+        uStr[MOMT] = uStr[DENS] * vTK;
+        if (S::Z) uStr[MOMZ_] = uStr[DENS] * (left ? L.vZ : R.vZ);
+        double pStr = L.rho * dL * (sStr - L.vN) + pTotL;
+        if (S::H) {
+            // without a field the HLL state enters no other term
+            uStr[ENER] = g.div(eK * dK + pStr * sStr - pTotK * vNK, rK);
+        } else {
+            double uHLL[NCONS];
+            const SharedRecip rS = g.recip(sR - sL);
 #pragma unroll
-    for (int v = 0; v < NCONS; v++) flux[v] = (left ? fL[v] : fR[v]) + sK * (uStr[v] - (left ? uL[v] : uR[v]));
+            for (int v = 0; v < NCONS; v++)
+                if (S::var(v) && v != ENER)
+                    uHLL[v] = v == MAGN ? g.div(sR * uR[v] - sL * uL[v] + 0.0, rS)
+                                        : g.div(sR * uR[v] - sL * uL[v] + fL[v] - fR[v], rS);
+            const SharedRecip rH = g.recip(uHLL[DENS]);
+            double bvH = 0.0 + uHLL[MAGN] * g.div(uHLL[MOMN], rH);
+            bvH = bvH + uHLL[MAGT] * g.div(uHLL[MOMT], rH);
+            if (S::BZ) bvH = bvH + uHLL[MAGZ_] * g.div(uHLL[MOMZ_], rH);
+            const double bTK = left ? L.bT : R.bT;
+            pStr = pStr - L.bN * L.bN + uHLL[MAGN] * uHLL[MAGN];
+            uStr[MOMT] = uStr[MOMT] - g.div(uHLL[MAGN] * uHLL[MAGT] - bNK * bTK, rK);
+            if (S::BZ)
+                uStr[MOMZ_] = uStr[MOMZ_] - g.div(uHLL[MAGN] * uHLL[MAGZ_] - bNK * (left ? L.bZ : R.bZ), rK);
+            uStr[MAGN] = uHLL[MAGN];
+            uStr[MAGT] = uHLL[MAGT];
+            if (S::BZ) uStr[MAGZ_] = uHLL[MAGZ_];
+            uStr[ENER] = g.div(eK * dK + pStr * sStr - pTotK * vNK - uHLL[MAGN] * bvH + bNK * (0.0 + bDotV), rK);
+        }
+#pragma unroll
+        for (int v = 0; v < NCONS; v++)
+            if (S::var(v)) flux[v] = flux[v] + sK * (uStr[v] - (left ? uL[v] : uR[v]));
+    }
+    return g.ok() && !floored;
 }
-
-// the Riemann solver with IEEE division throughout (the rare fallback)
-template <int FH>
-static __device__ __noinline__ void hllc_ieee(const Phys& s, const double* uL, const double* uR, int dir, double* flux) {
-    IeeeDiv dv;
-    hllc_t<FH>(s, uL, uR, dir, flux, dv);
+// CAD and PAD of a state whose left-out variables are zeros
+template <int MODE>
+__device__ __forceinline__ bool state_adm(const Phys& s, const double* u) {
+    double U[NCONS];
+#pragma unroll
+    for (int v = 0; v < NCONS; v++) U[v] = Solve<MODE>::var(v) ? u[v] : 0.0;
+    return admissible(U[DENS], cons2pres<Solve<MODE>::H ? 1 : 0>(s, U));
 }
-
-// HLLC with shared reciprocals; any operand outside their proven range sends
-// the whole solve through IEEE division instead (same result bits either way)
-template <int FH = -1>
+// a mode's solve, the IEEE form where it has to be
+template <int MODE>
+__device__ __forceinline__ void face_flux(const Phys& s, const double* uL, const double* uR, double* F, bool& admL,
+                                          bool& admR) {
+    bool done = false;
+    if (MODE != SOLVE_HYDRO_FIELD) done = face_solve<MODE>(s, uL, uR, F, admL, admR);
+    if (!done) {
+        Cons8 a, b;
+#pragma unroll
+        for (int v = 0; v < NCONS; v++) {
+            a.v[v] = Solve<MODE>::var(v) ? uL[v] : 0.0;
+            b.v[v] = Solve<MODE>::var(v) ? uR[v] : 0.0;
+        }
+        const Cons8 f = hllc_ieee<Solve<MODE>::H ? 1 : 0>(s, a, b);
+#pragma unroll
+        for (int v = 0; v < NCONS; v++)
+            if (Solve<MODE>::var(v)) F[v] = f.v[v];
+        admL = state_adm<MODE>(s, uL);
+        admR = state_adm<MODE>(s, uR);
+    }
+}
+__device__ __forceinline__ bool bits_zero(double a) {
+    return (((unsigned)__double2hiint(a) << 1) | (unsigned)__double2loint(a)) == 0u;
+}
+// in face coordinates, hydro flag at run time
+__device__ __forceinline__ void hllc_face(const Phys& s, const double* uL, const double* uR, double* F) {
+    bool al, ar;
+    if (!s.force_hydro) {
+        face_flux<SOLVE_MHD>(s, uL, uR, F, al, ar);
+        return;
+    }
+    bool field = false;
+#pragma unroll
+    for (int v = MAGN; v <= MAGZ_; v++) field = field || !bits_zero(uL[v]) || !bits_zero(uR[v]);
+    if (field) {
+        face_flux<SOLVE_HYDRO_FIELD>(s, uL, uR, F, al, ar);
+        return;
+    }
+    face_flux<SOLVE_HYDRO>(s, uL, uR, F, al, ar);
+    F[MAGN] = F[MAGT] = F[MAGZ_] = 0.0;
+}
+// in grid coordinates: a y-face exchanges x and y on the way in and out
 __device__ __forceinline__ void hllc(const Phys& s, const double* uL, const double* uR, int dir, double* flux) {
-    SharedRecipDiv dv;
-    hllc_t<FH>(s, uL, uR, dir, flux, dv);
-    if (!dv.ok) hllc_ieee<FH>(s, uL, uR, dir, flux);
+    const bool x = dir == XDIR;
+    double a[NCONS], b[NCONS], F[NCONS];
+#pragma unroll
+    for (int v = 0; v < NCONS; v++) {
+        const int t = v == MOMX ? MOMY : v == MOMY ? MOMX : v == MAGX ? MAGY : v == MAGY ? MAGX : v;
+        a[v] = x ? uL[v] : uL[t];
+        b[v] = x ? uR[v] : uR[t];
+    }
+    hllc_face(s, a, b, F);
+#pragma unroll
+    for (int v = 0; v < NCONS; v++) {
+        const int t = v == MOMX ? MOMY : v == MOMY ? MOMX : v == MAGX ? MAGY : v == MAGY ? MAGX : v;
+        flux[v] = x ? F[v] : F[t];
+    }
 }
 
 
@@ -532,17 +743,6 @@ __device__ inline void eigen_vecs(const Phys& s, const double* V, int dir, bool 
         Rm[q] = Rc[q];
         Lm[q] = Lc[q];
     }
-}
-
-// src/detect.f90:250-265 (CAD) and :238-248 (PAD): both finite (not NaN,
-// not infinite) and both > 0, i.e. each bit pattern is a positive, nonzero,
-// finite double (tested on the integer pipes)
-__device__ __forceinline__ bool positive_finite(double x) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    return u - 1ull < 0x7fefffffffffffffull;  // u in [1, 0x7fefffffffffffff]
-}
-__device__ __forceinline__ bool admissible(double dens, double pres) {
-    return positive_finite(dens) && positive_finite(pres);
 }
 
 }  // namespace hosono
