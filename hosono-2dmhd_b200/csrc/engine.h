@@ -37,8 +37,9 @@ struct Geo {
     double dx, dy, mindxdy, maxdxdy;
 };
 
-// Per-instance descriptor (device memory; written by the host at admission).
-struct InstDev {
+// Per-instance descriptor (device memory; written by the host at admission):
+// the part kernels may copy to shared memory, then the TMA descriptors.
+struct InstHead {
     Geo geo;
     Phys phys;
     double cfl;
@@ -58,10 +59,12 @@ struct InstDev {
     uint8_t* rrRec;     // radius each face was last reconstructed at (2 bits x 4 faces)
     uint8_t* fail;      // cell failed face CAD/PAD (pass 1, inner cascade)
     uint8_t* nextPass;  // reconstructNextPass
-    uint8_t* dirty;     // re-reconstructed by the pass-1 cascade
+    uint8_t* dirty;     // re-reconstructed by the chain's pass-1 cascade; the cluster form's marks of listed faces
     uint8_t* lowered;   // lowered by detect in this pass
     uint8_t* innerCount;  // per-cell inner lowerings of this pass (trace)
     uint8_t* detMask;     // per-stage detect_ALL terms (shock, plateau, u2 smooth)
+};
+struct InstDev : InstHead {
     // TMA descriptors of U[0..2] as (x: pitch, y: nyt, var: 8) boxes of the
     // pass-1 stencil box shape (zero fill outside the array)
     CUtensorMap tmU[3];
@@ -91,7 +94,7 @@ struct InstState {
     int big;         // this stage's work lists are too long for one cluster: the kernel chain takes it
     int cFail;       // cells that failed CAD/PAD in pass 1 (its list of them)
     int nCasc;       // cells on the cluster form's cascade-lowered list
-    int mc[8];       // the cluster form's list counters (mood_cluster.cuh MC_*)
+    int mc[10];      // the cluster form's list counters (mood_cluster.cuh MC_*)
     int nInner, nDetect;  // lowerings in the current pass
     int lastInner, lastDetect;  // lowerings of the last finished pass
     int passes;      // MOOD passes in the current stage
@@ -121,7 +124,7 @@ struct BatchFlags {
 // U[1-parity]; B in U[2].  The final RK combine writes A and flips parity.
 enum : int { ROLE_STATE = 0, ROLE_A = 1, ROLE_B = 2 };
 
-__host__ __device__ inline double* role_ptr(const InstDev& d, int parity, int role) {
+__host__ __device__ inline double* role_ptr(const InstHead& d, int parity, int role) {
     return role == ROLE_STATE ? d.U[parity] : role == ROLE_A ? d.U[1 - parity] : d.U[2];
 }
 

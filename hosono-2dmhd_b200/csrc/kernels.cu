@@ -19,6 +19,7 @@
 //   update/detect [strt,   stop]   -> [g,   g+n-1]   (timeStep.f90:108-109, detect.f90:81-82)
 
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 
 #include "engine.h"
@@ -1176,21 +1177,33 @@ __device__ __forceinline__ double flicd_y(const InstDev& d, long long c) {
 // and the per-pass test keeps the reference's order of decisions.
 
 
-// the per-pass test on the new state un of a cell: its detect terms in
-// *mask, the stage input's density at rho[c] (rows p doubles apart)
-__device__ __forceinline__ bool detect_cell_at(const Phys& P, const uint8_t* mask, const double* __restrict__ rho,
-                                               long long c, long long p, const double un[NCONS]) {
+// the per-pass test on the new state un of a cell: its detect terms m, the
+// stage input's density in the cell and its cross
+__device__ __forceinline__ bool detect_decide(const Phys& P, int m, const double (&d)[5], const double un[NCONS]) {
     const double presNew = cons2pres(P, un);
     if (!admissible(un[DENS], presNew)) return true;  // CAD, PAD
-    const int m = *mask;
     if (!(m & DM_SHOCK)) return false;
     if (m & DM_PLATEAU) return false;
-    const double d1 = rho[c], d2 = rho[c + 1], d3 = rho[c - 1], d4 = rho[c + p], d5 = rho[c - p];
-    const double mn = fmin(fmin(fmin(fmin(d1, d2), d3), d4), d5);
-    const double mx = fmax(fmax(fmax(fmax(d1, d2), d3), d4), d5);
+    const double mn = fmin(fmin(fmin(fmin(d[0], d[1]), d[2]), d[3]), d[4]);
+    const double mx = fmax(fmax(fmax(fmax(d[0], d[1]), d[2]), d[3]), d[4]);
     const double dn = un[DENS];
     if ((mn <= dn) && (dn <= mx)) return false;  // DMP
     return !(m & DM_SMOOTH);
+}
+// from the planes: the detect terms in *mask, the density at rho[c] (rows p
+// doubles apart)
+__device__ __forceinline__ bool detect_cell_at(const Phys& P, const uint8_t* mask, const double* __restrict__ rho,
+                                               long long c, long long p, const double un[NCONS]) {
+    const int m = *mask;
+    double d[5] = {};
+    if ((m & DM_SHOCK) && !(m & DM_PLATEAU)) {  // few cells
+        d[0] = rho[c];
+        d[1] = rho[c + 1];
+        d[2] = rho[c - 1];
+        d[3] = rho[c + p];
+        d[4] = rho[c - p];
+    }
+    return detect_decide(P, m, d, un);
 }
 
 // Per-stage part of detect_ALL on the interior, evaluated once per stage by

@@ -516,21 +516,21 @@ __device__ __forceinline__ void face_flux(const Phys& s, const double* uL, const
 __device__ __forceinline__ bool bits_zero(double a) {
     return (((unsigned)__double2hiint(a) << 1) | (unsigned)__double2loint(a)) == 0u;
 }
-// in face coordinates, hydro flag at run time
-__device__ __forceinline__ void hllc_face(const Phys& s, const double* uL, const double* uR, double* F) {
-    bool al, ar;
+// in face coordinates, hydro flag at run time; admL, admR: CAD and PAD of the sides
+__device__ __forceinline__ void hllc_face(const Phys& s, const double* uL, const double* uR, double* F, bool& admL,
+                                          bool& admR) {
     if (!s.force_hydro) {
-        face_flux<SOLVE_MHD>(s, uL, uR, F, al, ar);
+        face_flux<SOLVE_MHD>(s, uL, uR, F, admL, admR);
         return;
     }
     bool field = false;
 #pragma unroll
     for (int v = MAGN; v <= MAGZ_; v++) field = field || !bits_zero(uL[v]) || !bits_zero(uR[v]);
     if (field) {
-        face_flux<SOLVE_HYDRO_FIELD>(s, uL, uR, F, al, ar);
+        face_flux<SOLVE_HYDRO_FIELD>(s, uL, uR, F, admL, admR);
         return;
     }
-    face_flux<SOLVE_HYDRO>(s, uL, uR, F, al, ar);
+    face_flux<SOLVE_HYDRO>(s, uL, uR, F, admL, admR);
     F[MAGN] = F[MAGT] = F[MAGZ_] = 0.0;
 }
 // in grid coordinates: a y-face exchanges x and y on the way in and out
@@ -543,7 +543,8 @@ __device__ __forceinline__ void hllc(const Phys& s, const double* uL, const doub
         a[v] = x ? uL[v] : uL[t];
         b[v] = x ? uR[v] : uR[t];
     }
-    hllc_face(s, a, b, F);
+    bool al, ar;
+    hllc_face(s, a, b, F, al, ar);
 #pragma unroll
     for (int v = 0; v < NCONS; v++) {
         const int t = v == MOMX ? MOMY : v == MOMY ? MOMX : v == MAGX ? MAGY : v == MAGY ? MAGX : v;
