@@ -304,8 +304,8 @@ __device__ __forceinline__ void mc_flux(Mc& m, const McT& t, int n, int cur) {
     const Geo& G = m.d.geo;
     const int g8 = t.lane >> 3, v = t.lane & 7;
     double* buf = m.bufs + t.warp * MC_BUF + g8 * MC_FS;
-    for (int e0 = 4 * t.gw; e0 < n; e0 += 4 * t.nw) {
-        const int e = e0 + g8;
+    for (int e0 = t.gw; e0 < n; e0 += 4 * t.nw) {
+        const int e = e0 + g8 * t.nw;  // over the warps first: up to four faces each
         const bool act = e < n;
         int rr = 0, cf = 0, cl = 0, vf = v;
         bool x = true, flux = act, recL = false, recR = false;
@@ -408,7 +408,8 @@ __device__ __forceinline__ void mc_flux(Mc& m, const McT& t, int n, int cur) {
 // thread per cell (a face next to a listed cell does not read its entry)
 __device__ __forceinline__ void mc_record(Mc& m, const McT& t, const int* list, int n) {
     const Geo& G = m.d.geo;
-    for (int e = t.gw * 32 + t.lane; e < n; e += t.nw * 32) {
+    // from the last warp down: the first ones have most faces to solve
+    for (int e = (t.nw - 1 - t.gw) * 32 + t.lane; e < n; e += t.nw * 32) {
         const int c = list[e];
         const int j = cell_j(G, c), i = c - j * G.pitch;
         if (!mc_in_recon(G, i, j)) continue;
@@ -477,8 +478,8 @@ __device__ __forceinline__ void mc_update(Mc& m, const McT& t, const int* list, 
     const int v = t.lane & 7, base = t.lane & ~7;
     const double* fxy = d.FX + MAGY * G.plane;
     const double* fyx = d.FY + MAGX * G.plane;
-    for (int e0 = t.gw * 4; e0 < n; e0 += t.nw * 4) {
-        const int e = e0 + (t.lane >> 3);
+    for (int e0 = t.gw; e0 < n; e0 += t.nw * 4) {
+        const int e = e0 + (t.lane >> 3) * t.nw;
         int c = 0, i = 0, j = 0;
         bool in = false, cell = false;
         if (e < n) {
@@ -644,7 +645,7 @@ __device__ __forceinline__ McT mc_place() {
     McT t;
     const int rank = blockIdx.x % cluster_nctaid();
     t.warp = threadIdx.x >> 5;
-    t.gw = rank * MC_WARPS + t.warp;
+    t.gw = t.warp * (int)cluster_nctaid() + rank;  // a short list spreads over every block
     t.nw = cluster_nctaid() * MC_WARPS;
     t.lane = threadIdx.x & 31;
     t.lead = rank == 0 && threadIdx.x == 0;
@@ -777,8 +778,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
                     }
                     cur ^= 1;
                     nRec = mc_ld(&S.mc[MC_REC + cur]);
-                    mc_flux<true>(m, t, mc_ld(&S.mc[MC_FACE + cur]), cur);
                     mc_record(m, t, m.rec[cur], nRec);
+                    mc_flux<true>(m, t, mc_ld(&S.mc[MC_FACE + cur]), cur);
                     cluster_sync();
                     const int nFail = mc_ld(&S.mc[MC_FAIL]);
                     if (lead) S.nDetect = 0;  // nLow was read before this barrier
