@@ -284,8 +284,9 @@ struct P1Ctl {
     const int4* tiles;
     uint64_t* bar;
     double *box, *pv;
-    int n, uin;    // end of the launch's tiles, the stage input's role
-    int next[2];   // the block's tile of each turn, by the turn's parity
+    int n, sh;     // end of the launch's units, 1 << sh of them a tile
+    int uin;       // the stage input's role
+    int next[2];   // the block's unit of each turn, by the turn's parity
     int turn;      // the turn whose box is in place
     int released;  // threads done with that box
 };
@@ -313,7 +314,7 @@ template <int R, int MODE>
 __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __restrict__ sU,
                                               const double* __restrict__ sPv, int sx, int sy, int dir, bool needL,
                                               bool needR, bool doFlux, long long c, double* acc, double* park,
-                                              P1Ctl* ctl) {
+                                              P1Ctl* ctl, bool last) {
     typedef Solve<MODE> S;
     const Geo& G = d.geo;
     const Phys& P = d.phys;
@@ -358,7 +359,7 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
                 park[k++ * NTHREADS] = u[1][1][v];
             }
         }
-        if (!x && q0 + 2 >= NQ) p1_release<R>(ctl);  // this thread's last read of the box
+        if (last && q0 + 2 >= NQ) p1_release<R>(ctl);  // this thread's last read of the box
 #pragma unroll 1
         for (int q = q0;;) {
             bool admL = true, admR = true;
@@ -417,7 +418,8 @@ struct P1Cell {
     InstState* S;
     int* failList;
     int init;
-    int i, j;
+    int i, j, row;   // the cell, its row in the tile
+    int dir0, dir1;  // its faces: the x-face, the y-face or both
     int box, pv, acc, ctl;  // offsets in doubles (ctl: 0 where the block stages itself)
 };
 template <int R, int MODE>
@@ -430,10 +432,10 @@ static __device__ __noinline__ void pass1_tile(P1Cell c) {
     const int g = G.g;
     const int clo = g - 2, cxhi = g + G.nx + 1, cyhi = g + G.ny + 1;  // reconstruct range
     const int flo = g - 1, fxhi = g + G.nx + 1, fyhi = g + G.ny + 1;  // flux range
-    const int sx = threadIdx.x + Box::OX, sy = threadIdx.y + Box::OY;
+    const int sx = threadIdx.x + Box::OX, sy = c.row + Box::OY;
     const long long cc = (long long)j * G.pitch + i;
     const bool inF = i >= flo && i <= fxhi && j >= flo && j <= fyhi;
-    if (c.init && i < G.nxt && j < G.nyt) {
+    if (c.init && c.dir0 == XDIR && i < G.nxt && j < G.nyt) {
         d.scheme[c.S->schemeSel][cc] = (int8_t)R;
         d.rrRec[cc] = (uint8_t)(R | (R << 2) | (R << 4) | (R << 6));
         d.rec[cc] = 0;
@@ -445,15 +447,16 @@ static __device__ __noinline__ void pass1_tile(P1Cell c) {
     }
     P1Ctl* ctl = c.ctl ? reinterpret_cast<P1Ctl*>(smem + c.ctl) : nullptr;
 #pragma unroll 1
-    for (int dir = XDIR; dir <= YDIR; dir++) {  // the x-face, then the y-face of this cell
+    for (int dir = c.dir0; dir <= c.dir1; dir++) {  // the x-face, then the y-face of this cell
         const bool x = dir == XDIR;
         if (i >= clo && i <= cxhi + (x ? 1 : 0) && j >= clo && j <= cyhi + (x ? 0 : 1)) {
             const int a = x ? i : j, ahi = x ? cxhi : cyhi;
             const uint8_t bits = pass1_face<R, MODE>(d, smem + c.box, smem + c.pv, sx, sy, dir, a - 1 >= clo, a <= ahi,
-                                                     inF, cc, smem + c.acc, smem + c.acc + NCONS * NTHREADS, ctl);
+                                                     inF, cc, smem + c.acc, smem + c.acc + NCONS * NTHREADS, ctl,
+                                                     dir == c.dir1);
             if (bits & 1) pass1_fail(d.fail, c.failList, &c.S->cFail, (int)(x ? cc - 1 : cc - G.pitch));
             if (bits & 2) pass1_fail(d.fail, c.failList, &c.S->cFail, (int)cc);
-        } else if (!x) {
+        } else if (dir == c.dir1) {
             p1_release<R>(ctl);
         }
     }
@@ -467,39 +470,51 @@ static __device__ __noinline__ void pass1_tile(P1Cell c) {
 // reach: fifteen loads of a plane pair, no block barrier.
 // SPEC: with the planar modes (the launch choice that large solves run).
 template <int R>
-__device__ __forceinline__ bool rows_nonzero(const double* sU, int plane) {
-    bool any = false;  // rows [y-1-R, y+R] of the warp's row y, 0-based row threadIdx.y of the box
-    const double* rows = sU + plane * P1Box<R>::PLANE + threadIdx.y * P1Box<R>::SX;
+__device__ __forceinline__ bool rows_nonzero(const double* sU, int plane, int row) {
+    bool any = false;  // rows [y-1-R, y+R] of the warp's row y: from the box's row `row`
+    const double* rows = sU + plane * P1Box<R>::PLANE + row * P1Box<R>::SX;
     for (int e = threadIdx.x; e < (2 * R + 2) * P1Box<R>::SX; e += 32) any = any || !bits_zero(rows[e]);
     return __any_sync(0xffffffffu, any);
 }
+// u: the unit, of which a tile has 1 << sh.  Whole tiles (sh = 0): a warp takes
+// a row, its x-faces, then its y-faces.  Smaller units: a warp takes one
+// direction of a row, so a unit has 8 >> sh rows on twice as many warps.
 template <int R, bool SPEC>
-__device__ __forceinline__ void pass1_tile_any(const Batch& B, int t, const double* sU, int pv, int acc, int ctl) {
+__device__ __forceinline__ void pass1_tile_any(const Batch& B, int u, int sh, const double* sU, int pv, int acc, int ctl) {
     extern __shared__ __align__(128) double smem[];
     static_assert(TILE_X == 32, "a tile row is a warp");
-    const Cell cell = tile_at(B, t);
-    const InstDev& d = B.dev[cell.k];
+    const int4 tl = B.tiles[u >> sh];
+    const InstDev& d = B.dev[tl.x];
+    const int rows = TILE_Y >> sh;
+    const int dir = (int)threadIdx.y / rows;  // of a smaller unit
     P1Cell c;
+    c.row = sh ? (u & ((1 << sh) - 1)) * rows + (int)threadIdx.y % rows : (int)threadIdx.y;
+    c.dir0 = sh ? dir : XDIR;
+    c.dir1 = sh ? dir : YDIR;
+    if (sh && dir > YDIR) {  // fewer rows than half the warps
+        p1_release<R>(reinterpret_cast<P1Ctl*>(smem + ctl));
+        return;
+    }
     c.d = &d;
-    c.S = B.st + cell.k;
-    c.failList = reinterpret_cast<int*>(B.L.face + 2 * (long long)B.instTiles[cell.k].x * (TILE_X * TILE_Y));
+    c.S = B.st + tl.x;
+    c.failList = reinterpret_cast<int*>(B.L.face + 2 * (long long)B.instTiles[tl.x].x * (TILE_X * TILE_Y));
     c.init = B.p1Init;
-    c.i = cell.i;
-    c.j = cell.j;
+    c.i = tl.y + (int)threadIdx.x;
+    c.j = tl.z + c.row;
     c.box = (int)(sU - smem);
     c.pv = pv;
     c.acc = acc;
     c.ctl = ctl;
-    const bool z = !SPEC || rows_nonzero<R>(sU, MOMZ);
+    const bool z = !SPEC || rows_nonzero<R>(sU, MOMZ, c.row);
     if (d.phys.force_hydro) {
-        if (rows_nonzero<R>(sU, MAGX) || rows_nonzero<R>(sU, MAGY) || rows_nonzero<R>(sU, MAGZ))
+        if (rows_nonzero<R>(sU, MAGX, c.row) || rows_nonzero<R>(sU, MAGY, c.row) || rows_nonzero<R>(sU, MAGZ, c.row))
             pass1_tile<R, SOLVE_HYDRO_FIELD>(c);
         else if (z)
             pass1_tile<R, SOLVE_HYDRO>(c);
         else if (SPEC)
             pass1_tile<R, SOLVE_HYDRO_PLANAR>(c);
     } else {
-        if (z || rows_nonzero<R>(sU, MAGZ))
+        if (z || rows_nonzero<R>(sU, MAGZ, c.row))
             pass1_tile<R, SOLVE_MHD>(c);
         else if (SPEC)
             pass1_tile<R, SOLVE_MHD_PLANAR>(c);
@@ -575,25 +590,26 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned b
         : "memory");
 }
 
-// next tile at or after t (stride gridDim.x) that this launch works on
+// next unit at or after t (stride gridDim.x) that this launch works on; n
+// units, 1 << sh of them a tile
 template <int R>
-__device__ __forceinline__ int pass1_next(const Batch& B, int t, int n) {
+__device__ __forceinline__ int pass1_next(const Batch& B, int t, int n, int sh = 0) {
     for (; t < n; t += gridDim.x) {
-        const int k = B.tiles[t].x;
+        const int k = B.tiles[t >> sh].x;
         if (B.st[k].stepping && B.dev[k].geo.R == R) return t;
     }
     return n;
 }
 
-// the dynamic schedule: the next tile of this radius from the launch-wide
-// counter, counted from the launch's first tile (one atomic per tile taken;
+// the dynamic schedule: the next unit of this radius from the launch-wide
+// counter, counted from the launch's first tile (one atomic per unit taken;
 // n when none is left)
 template <int R>
-__device__ __forceinline__ int pass1_take(const Batch& B, int n) {
+__device__ __forceinline__ int pass1_take(const Batch& B, int n, int sh = 0) {
     for (;;) {
-        const int t = B.p1First + atomicAdd(&B.flags->p1Next[R], 1);
+        const int t = (B.p1First << sh) + atomicAdd(&B.flags->p1Next[R], 1);
         if (t >= n) return n;
-        const int k = B.tiles[t].x;
+        const int k = B.tiles[t >> sh].x;
         if (B.st[k].stepping && B.dev[k].geo.R == R) return t;
     }
 }
@@ -643,7 +659,7 @@ static __device__ __noinline__ void p1_refill(P1Ctl* ctl) {
         mbar_arrive(ctl->bar);
         return;
     }
-    const int4 tl = ctl->tiles[t];
+    const int4 tl = ctl->tiles[t >> ctl->sh];
     const InstDev& d = ctl->dev[tl.x];
     pass1_stage_tma<R>(d, ctl->st[tl.x].parity, ctl->uin, tl, ctl->box, ctl->pv, ctl->bar);
 }
@@ -662,6 +678,7 @@ static __device__ __noinline__ void p1_refill(P1Ctl* ctl) {
 // live: at two blocks per SM that wins over double-buffering on the 2048^2
 // workloads.  Three or four blocks per SM keep one box (their shared memory
 // would not fit two).
+constexpr int P1_HALF = 2;             // half-tile units below this many whole tiles per block
 constexpr int P1_THREAD = 3 * NCONS;  // doubles of shared memory per thread: accumulators, parked face states
 template <int R>
 struct P1Smem {  // dynamic shared memory layout (doubles): boxes, per-thread columns, prediction vectors, mbarriers
@@ -714,7 +731,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             pass1_stage<R>(B, uin, t, smem, pvBuf, tid);
             cp_async_wait<0>();
             __syncthreads();  // tile t's box is in place for every thread
-            pass1_tile_any<R, SPEC>(B, t, smem, (int)(pvBuf - smem), acc, 0);
+            pass1_tile_any<R, SPEC>(B, t, 0, smem, (int)(pvBuf - smem), acc, 0);
             __syncthreads();  // every read of this box is done before it is refilled
             t = next_tile(t + gridDim.x);
         }
@@ -725,9 +742,16 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
         // thread has released the one before: the copy needs no block barrier.
         constexpr int CTL = P1Smem<R>::ctl(1);
         P1Ctl* ctl = reinterpret_cast<P1Ctl*>(smem + CTL);
+        // Fewer tiles than two rounds of the grid: smaller units, so that more
+        // SMs work and the last round is shorter (us per launch, whole tiles ->
+        // units: 64^2 R=2 34.8 -> 22.6, 128^2 R=1 29.4 -> 20.1, 256^2 R=3 81.6 ->
+        // 79.2, 512^2 alike; at 1024^2, 14 rounds, halves cost 7 %).
+        const int tiles = n - B.p1First;
+        const int sh = tiles * 4 <= (int)gridDim.x ? 2 : tiles < P1_HALF * (int)gridDim.x ? 1 : 0;
+        const int nu = n << sh;
         if (tid == 0) {
-            *ctl = P1Ctl{B.dev, B.st, B.tiles, bars, smem, pvBuf, n, uin, {0, 0}, -1, 0};
-            ctl->next[0] = DYN ? pass1_take<R>(B, n) : pass1_next<R>(B, B.p1First + blockIdx.x, n);
+            *ctl = P1Ctl{B.dev, B.st, B.tiles, bars, smem, pvBuf, nu, sh, uin, {0, 0}, -1, 0};
+            ctl->next[0] = DYN ? pass1_take<R>(B, nu, sh) : pass1_next<R>(B, (B.p1First << sh) + blockIdx.x, nu, sh);
             p1_refill<R>(ctl);
         }
         __syncthreads();
@@ -737,11 +761,12 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
                 return;
             }
             const int t = ctl->next[turn & 1];
-            if (t >= n) return;
+            if (t >= nu) return;
             __syncthreads();  // in step: warps apart evict one another's instructions (7 % slower)
-            // the next turn's tile, before this thread releases the box
-            if (tid == 0) ctl->next[(turn + 1) & 1] = DYN ? pass1_take<R>(B, n) : pass1_next<R>(B, t + gridDim.x, n);
-            pass1_tile_any<R, SPEC>(B, t, smem, (int)(pvBuf - smem), acc, CTL);
+            // the next turn's unit, before this thread releases the box
+            if (tid == 0)
+                ctl->next[(turn + 1) & 1] = DYN ? pass1_take<R>(B, nu, sh) : pass1_next<R>(B, t + gridDim.x, nu, sh);
+            pass1_tile_any<R, SPEC>(B, t, sh, smem, (int)(pvBuf - smem), acc, CTL);
         }
     }
     int t = next_tile(B.p1First + blockIdx.x);
@@ -775,7 +800,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             }
         }
         __syncthreads();  // tile t's box is in place for every thread
-        pass1_tile_any<R, SPEC>(B, t, smem + buf * Box::DOUBLES, (int)(pvBuf - smem) + buf * Box::PVN, acc, 0);
+        pass1_tile_any<R, SPEC>(B, t, 0, smem + buf * Box::DOUBLES, (int)(pvBuf - smem) + buf * Box::PVN, acc, 0);
         __syncthreads();  // every read of this box is done before it is refilled
         buf ^= 1;
         t = tn;
@@ -2200,7 +2225,8 @@ int pass1_grid(int maxTiles) {
                              cudaFuncAttributeMaxDynamicSharedMemorySize, pass1_smem<R, NBUF>()) == cudaSuccess;
     (void)attr;
     const int r = resident_blocks((const void*)k_face_pass1<R, TMA, DYN, MINB, NBUF>, pass1_smem<R, NBUF>());
-    return r < maxTiles ? r : maxTiles;
+    const int units = TMA && NBUF == 1 && maxTiles < r ? 4 * maxTiles : maxTiles;  // few tiles go in quarters
+    return r < units ? r : units;
 }
 template <int R, bool TMA, bool DYN, int MINB, int NBUF>
 void launch_pass1_v(const Batch& B, int uin, cudaStream_t s) {
