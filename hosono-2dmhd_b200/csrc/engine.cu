@@ -791,6 +791,8 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     InstState st;
     TRYE(state(slot, &st));
     st.dt = dt;
+    st.dtdx = dt / slots_[slot].dev.geo.dx;
+    st.dtdy = dt / slots_[slot].dev.geo.dy;
     st.stepping = 1;
     st.error = 0;
     CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
@@ -1149,6 +1151,8 @@ int Engine::advance(int slot, double dt) {
     InstState st;
     TRYE(state(slot, &st));
     st.dt = dt;
+    st.dtdx = dt / slots_[slot].dev.geo.dx;
+    st.dtdy = dt / slots_[slot].dev.geo.dy;
     st.stepping = 1;
     st.error = 0;
     CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));

@@ -80,6 +80,7 @@ constexpr int CT_SX = TILE_X + 8, CT_UY = TILE_Y + 4, CT_FY = TILE_Y + 3;
 // Per-instance mutable scalars (device memory).
 struct InstState {
     double dt, t, tmax;
+    double dtdx, dtdy;  // dt/dx and dt/dy of the current step
     int nstep, nstepmax;
     int live;        // slot holds an instance
     int done;        // time loop finished (t >= tmax or nstep >= nstepmax) or failed

@@ -1202,23 +1202,25 @@ __device__ __forceinline__ double flicd_y(const InstDev& d, long long c) {
 // and the per-pass test keeps the reference's order of decisions.
 
 
-// the per-pass test on the new state un of a cell: its detect terms m, the
-// stage input's density in the cell and its cross
-__device__ __forceinline__ bool detect_decide(const Phys& P, int m, const double (&d)[5], const double un[NCONS]) {
-    const double presNew = cons2pres(P, un);
-    if (!admissible(un[DENS], presNew)) return true;  // CAD, PAD
+// the per-pass test on the new state of a cell (its density, |m|^2 and |B|^2
+// summed x, y, z from zero, energy): its detect terms m, the stage input's
+// density in the cell and its cross
+struct NewState {
+    double rho, msq, bsq, E;
+};
+__device__ __forceinline__ bool detect_decide(const Phys& P, int m, const double (&d)[5], const NewState& n) {
+    if (!state_admissible(P, n.rho, n.msq, n.bsq, n.E)) return true;  // CAD, PAD
     if (!(m & DM_SHOCK)) return false;
     if (m & DM_PLATEAU) return false;
     const double mn = fmin(fmin(fmin(fmin(d[0], d[1]), d[2]), d[3]), d[4]);
     const double mx = fmax(fmax(fmax(fmax(d[0], d[1]), d[2]), d[3]), d[4]);
-    const double dn = un[DENS];
-    if ((mn <= dn) && (dn <= mx)) return false;  // DMP
+    if ((mn <= n.rho) && (n.rho <= mx)) return false;  // DMP
     return !(m & DM_SMOOTH);
 }
 // from the planes: the detect terms in *mask, the density at rho[c] (rows p
 // doubles apart)
 __device__ __forceinline__ bool detect_cell_at(const Phys& P, const uint8_t* mask, const double* __restrict__ rho,
-                                               long long c, long long p, const double un[NCONS]) {
+                                               long long c, long long p, const NewState& n) {
     const int m = *mask;
     double d[5] = {};
     if ((m & DM_SHOCK) && !(m & DM_PLATEAU)) {  // few cells
@@ -1228,7 +1230,7 @@ __device__ __forceinline__ bool detect_cell_at(const Phys& P, const uint8_t* mas
         d[3] = rho[c + p];
         d[4] = rho[c - p];
     }
-    return detect_decide(P, m, d, un);
+    return detect_decide(P, m, d, n);
 }
 
 // Per-stage part of detect_ALL on the interior, evaluated once per stage by
@@ -1252,14 +1254,11 @@ __device__ __forceinline__ void detect_prep_tile_t(const InstDev& d, const Cell 
         const int gx = x0 + ex, gy = y0 + ey;
         double vx = 0.0, vy = 0.0, pr = 1.0, rho = 1.0;
         if (gx >= 0 && gx < G.nxt && gy >= 0 && gy < G.nyt) {
-            double u[NCONS], V[NPRIM];
+            double u[NCONS];
 #pragma unroll
             for (int v = 0; v < NCONS; v++) u[v] = load(v, gx, gy);
-            cons2prim(P, u, V);
-            vx = V[VELX];
-            vy = V[VELY];
-            pr = V[PRES];
-            rho = V[DENS];
+            rho = u[DENS];
+            pr = prim_pres(P, u, vx, vy);
         }
         sV[0 * DP_SX * DP_SY + e] = vx;
         sV[1 * DP_SX * DP_SY + e] = vy;
@@ -1275,16 +1274,25 @@ __device__ __forceinline__ void detect_prep_tile_t(const InstDev& d, const Cell 
     const double* spr = sV + 2 * DP_SX * DP_SY;
     const double* srho = sV + 3 * DP_SX * DP_SY;
     const double dx = G.dx, dy = G.dy;
-    double div_vel = (svx[e + 1] - svx[e - 1]) / (2 * dx);
-    div_vel = div_vel + (svy[e + DP_SX] - svy[e - DP_SX]) / (2 * dy);
-    const bool shock1 = div_vel < -(1.0 * (G.maxdxdy * G.maxdxdy));
-    double mach = svx[e] * svx[e] + svy[e] * svy[e];
-    mach = srho[e] * mach / (P.gamma * spr[e]);
-    mach = sqrt(mach);
-    const bool shock2 = mach > 0.2;
-    double pg = fabs(spr[e + 1] - spr[e - 1]) / (fmin(spr[e + 1], spr[e - 1]));
-    pg = pg + fabs(spr[e + DP_SX] - spr[e - DP_SX]) / (fmin(spr[e + DP_SX], spr[e - DP_SX]));
-    const bool shock3 = pg > 10.0 * G.maxdxdy;
+    // the pressure sensor first: it is off in all but a few cells, and seen to
+    // be off without its two divisions when the sum of the two ratios is
+    // below its threshold by more than rounding (a margin of 2^-40)
+    const double pE = spr[e + 1], pW = spr[e - 1], pN = spr[e + DP_SX], pS = spr[e - DP_SX];
+    const double ax = fabs(pE - pW), ay = fabs(pN - pS), mx = fmin(pE, pW), my = fmin(pN, pS);
+    const double thr = 10.0 * G.maxdxdy;
+    bool shock1 = false, shock2 = false, shock3 = false;
+    if (!((ax * my + ay * mx) * (1.0 + 0x1p-40) < thr * (mx * my))) {
+        double div_vel = (svx[e + 1] - svx[e - 1]) / (2 * dx);
+        div_vel = div_vel + (svy[e + DP_SX] - svy[e - DP_SX]) / (2 * dy);
+        shock1 = div_vel < -(1.0 * (G.maxdxdy * G.maxdxdy));
+        double mach = svx[e] * svx[e] + svy[e] * svy[e];
+        mach = srho[e] * mach / (P.gamma * spr[e]);
+        mach = sqrt(mach);
+        shock2 = mach > 0.2;
+        double pg = ax / mx;
+        pg = pg + ay / my;
+        shock3 = pg > thr;
+    }
     const long long cc = (long long)c.j * G.pitch + c.i;
     int m = 0;
     if (shock1 && shock2 && shock3) {
@@ -1363,9 +1371,8 @@ __device__ __forceinline__ bool update_detect_at(const InstDev& d, const InstSta
                                                  double cty_n) {
     const Geo& G = d.geo;
     double* Uo = role_ptr(d, S.parity, uout);
-    const double dt = S.dt;
-    const double dtdx = dt / G.dx, dtdy = dt / G.dy;
-    double un[NCONS];
+    const double dtdx = S.dtdx, dtdy = S.dtdy;
+    NewState n = {0.0, 0.0, 0.0, 0.0};  // not the eight new values: they would not stay in registers
 #pragma unroll
     for (int v = 0; v < NCONS; v++) {
         double f0, f1, g0, g1;
@@ -1385,12 +1392,16 @@ __device__ __forceinline__ bool update_detect_at(const InstDev& d, const InstSta
             g0 = src.FY[v * src.fplane + src.fc];
             g1 = src.FY[v * src.fplane + src.fc + src.fp];
         }
-        un[v] = src.U[v * src.uplane + src.uc] - dtdx * (f1 - f0) - dtdy * (g1 - g0);
-        Uo[v * G.plane + cc] = un[v];
+        const double un = src.U[v * src.uplane + src.uc] - dtdx * (f1 - f0) - dtdy * (g1 - g0);
+        Uo[v * G.plane + cc] = un;
+        if (v == DENS) n.rho = un;
+        if (v == ENER) n.E = un;
+        if (v >= MOMX && v <= MOMZ) n.msq = n.msq + un * un;
+        if (v >= MAGX && v <= MAGZ) n.bsq = n.bsq + un * un;
     }
     bool low = false;
     if (d.scheme[S.schemeSel][cc] > 0)
-        low = detect_cell_at(d.phys, d.detMask + cc, src.U + DENS * src.uplane, src.uc, src.up, un);
+        low = detect_cell_at(d.phys, d.detMask + cc, src.U + DENS * src.uplane, src.uc, src.up, n);
     if (low) d.lowered[cc] = 1;
     return low;
 }
@@ -1454,6 +1465,7 @@ __device__ __forceinline__ void t_ct_update_detect(const Batch& B, int uin, int 
     }
     low_append(B, c.k, low, cc);
 }
+constexpr int MINB_CT = 5;
 // six resident blocks (a 40-register budget, a few hundred bytes of spills):
 // the tile's loads wait at two barriers, so more warps in flight keep HBM
 // busier.  Per step on Orszag-Tang 2048^2: 3 blocks (80 registers) 11.66 ms,
@@ -1461,7 +1473,7 @@ __device__ __forceinline__ void t_ct_update_detect(const Batch& B, int uin, int 
 // cell's corrected fluxes once into shared memory (instead of a cell also
 // evaluating its east and north neighbours' FLICD) made a launch about 5 %
 // slower: the extra barrier costs more than the loads it saves, which hit L1.
-__global__ void __launch_bounds__(NTHREADS, 6) k_ct_update_detect(Batch B, int uin, int uout) { PDL_ENTRY();
+__global__ void __launch_bounds__(NTHREADS, MINB_CT) k_ct_update_detect(Batch B, int uin, int uout) { PDL_ENTRY();
     __shared__ double sV[4 * DP_SX * DP_SY];
     FOR_TILES(B, t) t_ct_update_detect(B, uin, uout, tile_at(B, t), sV);
 }
@@ -1998,6 +2010,8 @@ __global__ void k_step_begin(Batch B, int use_host_dt) { PDL_ENTRY();
             S.stepping = 0;
         }
         S.dt = dt;
+        S.dtdx = dt / d.geo.dx;
+        S.dtdy = dt / d.geo.dy;
     }
 }
 

@@ -527,8 +527,11 @@ __device__ __forceinline__ void mc_update(Mc& m, const McT& t, const int* list, 
 #pragma unroll
         for (int w = 0; w < NCONS; w++) u[w] = __shfl_sync(0xffffffffu, un, base + w);
         bool low = false;
-        if (cell && v == 0 && sch > 0)
-            low = detect_decide(m.d.phys, mask, rho, u);
+        if (cell && v == 0 && sch > 0) {
+            const double msq = (0.0 + u[MOMX] * u[MOMX]) + u[MOMY] * u[MOMY] + u[MOMZ] * u[MOMZ];
+            const double bsq = (0.0 + u[MAGX] * u[MAGX]) + u[MAGY] * u[MAGY] + u[MAGZ] * u[MAGZ];
+            low = detect_decide(m.d.phys, mask, rho, NewState{u[DENS], msq, bsq, u[ENER]});
+        }
         if (flags) {
             unsigned lows = __ballot_sync(0xffffffffu, low);
             if (lows && t.lane == 0) atomicAdd(&m.S->nDetect, __popc(lows));
@@ -620,8 +623,8 @@ __device__ __forceinline__ void mc_setup(const Batch& B, int k, int uin, int uou
         m.S = B.st + k;
         m.U = role_ptr(d, S.parity, uin);
         m.Uo = role_ptr(d, S.parity, uout);
-        m.dtdx = S.dt / G.dx;
-        m.dtdy = S.dt / G.dy;
+        m.dtdx = S.dtdx;
+        m.dtdy = S.dtdy;
         m.sch = d.scheme[S.schemeSel];
         // the segment of the batch's face list holds 2 entries of 2 ints a cell
         int* face = reinterpret_cast<int*>(B.L.face + 2 * seg);

@@ -185,6 +185,39 @@ struct SharedRecipDiv {
     }
 };
 
+// CAD and PAD of a state by its density, |m|^2 and |B|^2 (each summed x, y, z
+// from zero) and energy: admissible(rho, cons2pres).  Nearly every state is
+// seen to pass without cons2pres's division: rho * (E - Bp) exceeds 0.5 |m|^2
+// by more than its rounding (a margin of 2^-40), with every term far from
+// overflow and underflow.
+__device__ __forceinline__ bool state_admissible(const Phys& s, double rho, double msq, double bsq, double E) {
+    const double Bp = s.force_hydro ? 0.0 : 0.5 * bsq;
+    const double e = E - Bp;
+    if (rho > 1e-100 && rho < 1e100 && e > 1e-100 && e < 1e100 && e * rho > 0.5 * msq * (1.0 + 0x1p-40) &&
+        s.gamma > 1.001 && s.gamma < 1000.0)
+        return true;
+    return admissible(rho, (s.gamma - 1.0) * (E - Bp - 0.5 * msq / rho));
+}
+// pressure (floored) and in-plane velocity of a state as cons2prim gives them
+// (convert.f90:198-234), its four quotients by the density on one reciprocal
+__device__ __forceinline__ double prim_pres(const Phys& s, const double* U, double& vx, double& vy) {
+    double Bp = 0.0;
+    if (!s.force_hydro) Bp = 0.5 * (U[MAGX] * U[MAGX] + U[MAGY] * U[MAGY] + U[MAGZ] * U[MAGZ]);
+    const double EB = s.force_hydro ? U[ENER] : U[ENER] - Bp;
+    SolverDiv g;
+    const SharedRecip r = g.recip(U[DENS]);
+    vx = g.div(U[MOMX], r);
+    vy = g.div(U[MOMY], r);
+    double vz = g.div(U[MOMZ], r), q = g.div(EB, r);
+    if (!g.ok()) {
+        vx = U[MOMX] / U[DENS];
+        vy = U[MOMY] / U[DENS];
+        vz = U[MOMZ] / U[DENS];
+        q = EB / U[DENS];
+    }
+    return eos_pres(s, U[DENS], q - 0.5 * (vx * vx + vy * vy + vz * vz));
+}
+
 // ---- src/riemannSolver.f90:68-221 (HLLC for MHD, Li 2005) in face
 // coordinates: N the normal, T the other in-plane component, Z out of plane.
 // A y-face is the x-face of the state with x and y exchanged, bit for bit:
