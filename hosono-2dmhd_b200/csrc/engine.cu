@@ -263,6 +263,7 @@ int Engine::init(int max_inst, int max_tiles, int fp_mode) {
     CUE(cudaMemsetAsync(d_ntiles_, 0, sizeof(int), s_));
     CUE(cudaMemsetAsync(d_flags_, 0, sizeof(BatchFlags), s_));
     std::memset(h_flags_, 0, sizeof(BatchFlags));
+    std::memset(h_st_, 0, sizeof(InstState) * maxInst_);
     slots_.assign(maxInst_, Slot{});
     traceStageBase.assign(maxInst_, 0);
     tracePassesSeen_.assign(maxInst_, 0);
@@ -543,16 +544,25 @@ int Engine::upload_tables() {
     return HOSONO_OK;
 }
 
+// The instances' scalars at rest are mirrored in pinned host memory (h_st_):
+// every host write goes to both, and a run copies the device's back at its end
+// (check_errors), so reading them costs no round trip.  Writes are small
+// pageable copies, staged by the call and ordered on the stream.
 int Engine::write_state_field(int slot, size_t offset, const void* src, size_t n) {
+    std::memcpy((char*)(h_st_ + slot) + offset, src, n);
     CUE(cudaMemcpyAsync((char*)(d_st_ + slot) + offset, src, n, cudaMemcpyHostToDevice, s_));
-    CUE(cudaStreamSynchronize(s_));
+    return HOSONO_OK;
+}
+
+int Engine::write_state(int slot, const InstState& st) {
+    h_st_[slot] = st;
+    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
     return HOSONO_OK;
 }
 
 int Engine::state(int slot, InstState* out) {
     if (slot < 0 || slot >= maxInst_) return fail(HOSONO_EINVAL, "bad slot %d", slot);
-    CUE(cudaMemcpyAsync(out, d_st_ + slot, sizeof(InstState), cudaMemcpyDeviceToHost, s_));
-    CUE(cudaStreamSynchronize(s_));
+    *out = h_st_[slot];
     return HOSONO_OK;
 }
 
@@ -678,7 +688,7 @@ int Engine::add(const hosono_params& p, const double* pv, const double* qw, int*
     st.tmax = HUGE_VAL;
     st.nstepmax = INT_MAX;
     st.passCap = HOSONO_MOOD_CAP_DEFAULT(R, p.nx, p.ny);
-    CUE(cudaMemcpyAsync(d_st_ + k, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
+    TRYE(write_state(k, st));
     CUE(cudaMemsetAsync(d_hold_ + k, 0, sizeof(int), s_));
     sl.live = true;
     sl.ntiles = tiles_of(p);
@@ -694,8 +704,7 @@ int Engine::add(const hosono_params& p, const double* pv, const double* qw, int*
 int Engine::remove(int slot, bool commit) {
     if (slot < 0 || slot >= maxInst_ || !slots_[slot].live) return fail(HOSONO_EINVAL, "bad slot %d", slot);
     CUE(cudaStreamSynchronize(s_));
-    InstState st{};
-    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
+    TRYE(write_state(slot, InstState{}));
     slots_[slot].live = false;
     if (commit) TRYE(upload_tables());
     CUE(cudaStreamSynchronize(s_));  // no kernel of this stream still reads the memory
@@ -727,6 +736,7 @@ int Engine::upload(int slot, const double* U, const double* V) {
         launches++;
         CUE(cudaGetLastError());
         TRYE(write_field(slot, &InstState::stepping, 0));
+        CUE(cudaStreamSynchronize(s_));  // U may be pinned: its copy has to be done
     }
     return HOSONO_OK;
 }
@@ -795,7 +805,7 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     st.dtdy = dt / slots_[slot].dev.geo.dy;
     st.stepping = 1;
     st.error = 0;
-    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
+    TRYE(write_state(slot, st));
     TRYE(build_graphs());
     // the copies start once everything before on the main stream is done with the staging buffer
     CUE(cudaEventRecord(bandEv_[HOSONO_UPLOAD_BANDS_MAX], s_));
@@ -947,9 +957,7 @@ int Engine::set_time(int slot, double t, double tmax, int nstep, int nstepmax) {
     st.done = (t < tmax && nstep < nstepmax) ? 0 : 1;
     st.error = 0;
     st.stepping = 0;
-    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
-    CUE(cudaStreamSynchronize(s_));
-    return HOSONO_OK;
+    return write_state(slot, st);
 }
 
 // ----------------------------------------------------------------------
@@ -1130,16 +1138,16 @@ int Engine::cfl(int slot, double* dt) {
     TRYE(state(slot, &st));
     st.stepping = 1;
     st.cflbits[0] = st.cflbits[1] = 0;
-    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
+    TRYE(write_state(slot, st));
     K_->cfl_reduce(batch(), s_);
     launches++;
     CUE(cudaGetLastError());
-    TRYE(state(slot, &st));
-    const unsigned long long bits[2] = {st.cflbits[0], st.cflbits[1]};
+    CUE(cudaMemcpyAsync(h_st_[slot].cflbits, d_st_[slot].cflbits, sizeof st.cflbits, cudaMemcpyDeviceToHost, s_));
     TRYE(write_field(slot, &InstState::stepping, 0));
+    CUE(cudaStreamSynchronize(s_));
     double xm, ym;
-    std::memcpy(&xm, &bits[0], sizeof xm);
-    std::memcpy(&ym, &bits[1], sizeof ym);
+    std::memcpy(&xm, &h_st_[slot].cflbits[0], sizeof xm);
+    std::memcpy(&ym, &h_st_[slot].cflbits[1], sizeof ym);
     const Slot& sl = slots_[slot];
     *dt = sl.p.cfl * std::fmin(sl.dev.geo.dx / xm, sl.dev.geo.dy / ym);  // cfl.f90:50
     return HOSONO_OK;
@@ -1155,10 +1163,10 @@ int Engine::advance(int slot, double dt) {
     st.dtdy = dt / slots_[slot].dev.geo.dy;
     st.stepping = 1;
     st.error = 0;
-    CUE(cudaMemcpyAsync(d_st_ + slot, &st, sizeof(InstState), cudaMemcpyHostToDevice, s_));
+    TRYE(write_state(slot, st));
     if (use_graphs && !trace) {
         TRYE(build_graphs());
-        TRYE(launch(gAdvance_));
+        CUE(cudaGraphLaunch(gAdvance_, s_));  // check_errors waits for it
     } else {
         Rec r(this, nullptr);
         TRYE(record_step(r, true, 0, false));
@@ -1175,7 +1183,7 @@ int Engine::run(int max_steps) {
     CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
     if (use_graphs && !trace) {
         TRYE(build_graphs());
-        TRYE(launch(gRun_));
+        CUE(cudaGraphLaunch(gRun_, s_));  // check_errors waits for it
     } else {
         Rec r(this, nullptr);
         CUE(cudaStreamSynchronize(s_));

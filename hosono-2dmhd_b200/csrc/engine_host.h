@@ -150,6 +150,7 @@ class Engine {
     Batch batch() const;
     int upload_tables();
     int write_state_field(int slot, size_t offset, const void* src, size_t n);
+    int write_state(int slot, const InstState& st);
     template <typename T>
     int write_field(int slot, T InstState::*field, T value) {
         const InstState* z = nullptr;
@@ -193,7 +194,7 @@ class Engine {
     BatchFlags* d_flags_ = nullptr;
     Lists lists_{};
     BatchFlags* h_flags_ = nullptr;  // pinned
-    InstState* h_st_ = nullptr;      // pinned
+    InstState* h_st_ = nullptr;      // pinned mirror of d_st_ at rest
     double* staging_ = nullptr;
     size_t stagingCells_ = 0;
     int* schemeInt_ = nullptr;
