@@ -59,6 +59,8 @@ struct Mc {
     double dtdx, dtdy;
     double bufs[MC_WARPS * MC_BUF];  // the warps' exchange buffers
     double pv[MC_PV], qw[MC_QW];     // prediction vectors and weights
+    int faceC[4 * MC_WARPS];         // the block's faces: 2 * right cell + direction, and
+    int faceI[4 * MC_WARPS];         // radius | flux << 2 | test left << 3 | test right << 4
 };
 struct McT {  // a thread's place
     int gw, nw, lane, warp;  // warp of the cluster, warps of the cluster
@@ -283,9 +285,10 @@ __device__ __forceinline__ void mc_faces(Mc& m, const McT& t, const int* list, i
 }
 
 // getFluxes_ (getFluxes.f90:16-90) on the n faces of the face list, 8 lanes
-// per face: lane v sums variable v of both face states, lane q solves the
-// Riemann problem of point q, lane v adds the Gauss sum of flux v in
-// quadrature order.  Face states are rebuilt at the radius each side was last
+// per face: lane v sums variable v of both face states; then a thread of the
+// block's first warps solves the Riemann problem of each face and point (a
+// warp's own faces would keep eight to sixteen lanes of every warp busy); lane
+// v adds the Gauss sum of flux v in quadrature order.  Face states are rebuilt at the radius each side was last
 // reconstructed with (rrRec), the quadrature uses the face's current radius
 // (riemannSolver.f90:23-47), as in flux_list.
 // FIRST: the start of a later pass, reconstruct_faceValsWithGP's first inner
@@ -304,21 +307,25 @@ __device__ __forceinline__ void mc_flux(Mc& m, const McT& t, int n, int cur) {
     const Geo& G = m.d.geo;
     const int g8 = t.lane >> 3, v = t.lane & 7;
     double* buf = m.bufs + t.warp * MC_BUF + g8 * MC_FS;
-    for (int e0 = t.gw; e0 < n; e0 += 4 * t.nw) {
-        const int e = e0 + g8 * t.nw;  // over the warps first: up to four faces each
+    const int nq = G.nqMax;
+    for (int b0 = 0; b0 < n; b0 += 4 * t.nw) {
+        // a warp's faces of the round: over the warps first, up to four each
+        const int e = b0 + t.gw + g8 * t.nw;
         const bool act = e < n;
-        int rr = 0, cf = 0, cl = 0, vf = v;
-        bool x = true, flux = act, recL = false, recR = false;
+        const int slot = g8 * MC_WARPS + t.warp;  // in the block: filled from 0 up
+        int rr = 0, cf = 0, vf = v;
+        bool x = true, flux = act;
         if (act) {
             const int it = m.face[e];
             cf = it >> 1;
             x = (it & 1) == XDIR;
             // variable v's place in face coordinates (physics.cuh)
             vf = x ? v : v == MOMX || v == MAGX ? v + 1 : v == MOMY || v == MAGY ? v - 1 : v;
-            cl = x ? cf - 1 : cf - G.pitch;
+            const int cl = x ? cf - 1 : cf - G.pitch;
             const int fL = x ? EAST : NORTH, fR = x ? WEST : SOUTH;
             rr = min((int)m.sch[cf], (int)m.sch[cl]);
             int rrL = (m.d.rrRec[cl] >> (2 * fL)) & 3, rrR = (m.d.rrRec[cf] >> (2 * fR)) & 3;
+            bool recL = false, recR = false;
             if (FIRST) {
                 const int j = cell_j(G, cf), i = cf - j * G.pitch;
                 flux = i >= G.g - 1 && j >= G.g - 1 && i <= G.g + G.nx + 1 && j <= G.g + G.ny + 1;
@@ -327,6 +334,10 @@ __device__ __forceinline__ void mc_flux(Mc& m, const McT& t, int n, int cur) {
                 rrL = recL ? rr : rrL;
                 rrR = recR ? rr : rrR;
                 if (v == 0) m.d.dirty[cf] = 0;  // the face's mark
+            }
+            if (v == 0) {
+                m.faceC[slot] = it;
+                m.faceI[slot] = rr | (flux ? 4 : 0) | (recL ? 8 : 0) | (recR ? 16 : 0);
             }
             const double* Uv = m.U + v * G.plane;
             if (flux && rrL == rrR && (rrL == 1 || rrL == 2)) {  // nearly every face
@@ -353,55 +364,55 @@ __device__ __forceinline__ void mc_flux(Mc& m, const McT& t, int n, int cur) {
                 }
             }
         }
-        __syncwarp();
-        double F[NCONS];
-        const bool solve = flux && v <= rr;
-        bool badL = false, badR = false;
-        if (solve) {
-            double uL[NCONS], uR[NCONS];
-            bool admL, admR;
+        __syncthreads();
+        // the block's Riemann problems on as few warps as hold them: the slots
+        // are filled in the list's order, block after block
+        const int nct = t.nw / MC_WARPS, left = n - b0 - t.gw % nct;
+        const int faces = min(left > 0 ? (left + nct - 1) / nct : 0, 4 * MC_WARPS);
+        if ((int)threadIdx.x < faces * nq) {
+            const int k = (int)threadIdx.x / nq, q = (int)threadIdx.x - k * nq;
+            const int info = m.faceI[k], rq = info & 3;
+            double* st = m.bufs + (k % MC_WARPS) * MC_BUF + (k / MC_WARPS) * MC_FS + 16 * q;
+            if (q <= rq) {
+                bool badL = false, badR = false;
+                double uL[NCONS], uR[NCONS];
 #pragma unroll
-            for (int w = 0; w < NCONS; w++) {
-                uL[w] = buf[2 * v * 8 + w];
-                uR[w] = buf[(2 * v + 1) * 8 + w];
+                for (int w = 0; w < NCONS; w++) {
+                    uL[w] = st[w];
+                    uR[w] = st[8 + w];
+                }
+                if (info & 4) {
+                    double F[NCONS];
+                    bool admL, admR;
+                    hllc_face(m.d.phys, uL, uR, F, admL, admR);
+                    badL = !admL;
+                    badR = !admR;
+#pragma unroll
+                    for (int w = 0; w < NCONS; w++) st[w] = F[w];
+                } else if (FIRST) {  // a side that is not tested holds no state
+                    if (info & 8) badL = !admissible(uL[DENS], cons2pres(m.d.phys, uL));
+                    if (info & 16) badR = !admissible(uR[DENS], cons2pres(m.d.phys, uR));
+                }
+                if (FIRST && rq > 0) {
+                    const int it = m.faceC[k], c = it >> 1;
+                    if ((info & 8) && badL) mc_fail(m, (it & 1) == XDIR ? c - 1 : c - G.pitch);
+                    if ((info & 16) && badR) mc_fail(m, c);
+                }
             }
-            hllc_face(m.d.phys, uL, uR, F, admL, admR);
-            badL = !admL;
-            badR = !admR;
-        } else if (FIRST && act && v <= rr) {
-#pragma unroll 1
-            for (int side = 0; side < 2; side++) {
-                if (!(side ? recR : recL)) continue;
-                double u[NCONS];
-#pragma unroll
-                for (int w = 0; w < NCONS; w++) u[w] = buf[(2 * v + side) * 8 + w];
-                const bool bad = !admissible(u[DENS], cons2pres(m.d.phys, u));
-                badL = badL || (bad && side == 0);
-                badR = badR || (bad && side == 1);
-            }
         }
-        if (FIRST && rr > 0) {
-            if (recL && badL) mc_fail(m, cl);
-            if (recR && badR) mc_fail(m, cf);
-        }
-        __syncwarp();
-        if (solve) {
-#pragma unroll
-            for (int w = 0; w < NCONS; w++) buf[v * 8 + w] = F[w];
-        }
-        __syncwarp();
-        if (flux) {
+        __syncthreads();
+        if (act && flux) {
             double s;
             if (rr == 0) {
                 s = buf[vf];
             } else {
                 s = 0.0;
-                for (int q = 0; q <= rr; q++) s = s + m.qw[q + G.nqMax * (rr - 1)] * buf[q * 8 + vf];
+                for (int q = 0; q <= rr; q++) s = s + m.qw[q + G.nqMax * (rr - 1)] * buf[16 * q + vf];
             }
             (x ? m.d.FX : m.d.FY)[v * G.plane + cf] = s;
             if (v == (x ? MAGY : MAGX)) (x ? m.d.CTX : m.d.CTY)[cf] = s;
         }
-        __syncwarp();
+        __syncthreads();  // the buffers are read before the next round fills them
     }
 }
 // the radii the cells of the recompute list were reconstructed with, one
