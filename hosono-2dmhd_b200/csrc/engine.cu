@@ -1051,17 +1051,22 @@ int Engine::record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cas
 }
 
 // One time step (timeStep_RK3 + advanceSolution; with the driver's cfl and
-// validTimeStep unless the host supplies dt).  With profile, CUDA events
-// bracket the pass-1 kernel of each stage.
-int Engine::record_step(Rec& r, bool host_dt, cudaGraphConditionalHandle run_cond, bool profile,
-                        bool first_head) {
+// validTimeStep unless the host supplies dt).  STEP_TURN: the body of the run
+// graph's time loop, whose step was begun by the loop's prologue or by the
+// step before (rk_final collects the next CFL maxima, step_end begins the next
+// step).  With profile, CUDA events bracket the pass-1 kernel of each stage.
+int Engine::record_begin(Rec& r) {
     const Batch B = batch();
     const KernelSet* K = K_;
-    if (!host_dt) {
-        TRYE(r.k([&](cudaStream_t s) { K->step_prepare(B, 0, s); }));
-        TRYE(r.k([&](cudaStream_t s) { K->cfl_reduce(B, s); }));
-        TRYE(r.k([&](cudaStream_t s) { K->step_begin(B, 0, s); }));
-    }
+    TRYE(r.k([&](cudaStream_t s) { K->step_prepare(B, 0, s); }));
+    TRYE(r.k([&](cudaStream_t s) { K->cfl_reduce(B, s); }));
+    return r.k([&](cudaStream_t s) { K->step_begin(B, 0, s); });
+}
+int Engine::record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_cond, bool profile, bool first_head) {
+    const Batch B = batch();
+    const KernelSet* K = K_;
+    const int turn = form == STEP_TURN ? 1 : 0;
+    if (form == STEP_WHOLE) TRYE(record_begin(r));
     // U1 = FE(U), BC; U2 = FE(U1); U2 = (3U+U2)/4, BC; U3 = FE(U2); Unew = (U+2U3)/3
     const int uin[3] = {ROLE_STATE, ROLE_A, ROLE_A};
     const int uout[3] = {ROLE_A, ROLE_B, ROLE_B};
@@ -1070,9 +1075,9 @@ int Engine::record_step(Rec& r, bool host_dt, cudaGraphConditionalHandle run_con
                           profile ? profEv_[2 * st + 1] : nullptr, st > 0 || first_head));
         if (st == 0) TRYE(r.k([&](cudaStream_t s) { K->bc_fill(B, ROLE_A, s); }));
         if (st == 1) TRYE(r.k([&](cudaStream_t s) { K->rk_combine2(B, s); }));
-        if (st == 2) TRYE(r.k([&](cudaStream_t s) { K->rk_final(B, s); }));
+        if (st == 2) TRYE(r.k([&](cudaStream_t s) { K->rk_final(B, turn, s); }));
     }
-    TRYE(r.k([&](cudaStream_t s) { K->step_end(B, run_cond, s); }));
+    TRYE(r.k([&](cudaStream_t s) { K->step_end(B, run_cond, turn, s); }));
     return HOSONO_OK;
 }
 
@@ -1085,19 +1090,20 @@ int Engine::build_graphs() {
         Rec r(this, g);
         int rc;
         if (which == 0) {
-            rc = record_step(r, true, 0, false);
+            rc = record_step(r, STEP_HOST_DT, 0, false);
         } else if (which == 3) {  // the banded upload ran the first stage's set-up and pass 1
-            rc = record_step(r, true, 0, false, false);
+            rc = record_step(r, STEP_HOST_DT, 0, false, false);
         } else if (which == 2) {
             // one step at the graph's top level: event records are not allowed
             // inside conditional bodies, and pass 1 sits outside the MOOD loops
-            rc = record_step(r, false, 0, true);
+            rc = record_step(r, STEP_WHOLE, 0, true);
         } else {
             cudaGraphConditionalHandle hr;
-            rc = r.cond(&hr, 1);
+            rc = record_begin(r);
+            if (!rc) rc = r.cond(&hr, 1);
             if (!rc)
                 rc = r.loop(hr, &BatchFlags::anyLive, INT_MAX,
-                            [&](Rec& b) -> int { return record_step(b, false, hr, which == 2); });
+                            [&](Rec& b) -> int { return record_step(b, STEP_TURN, hr, false); });
         }
         if (!rc) rc = r.end();
         if (rc) {
@@ -1169,7 +1175,7 @@ int Engine::advance(int slot, double dt) {
         CUE(cudaGraphLaunch(gAdvance_, s_));  // check_errors waits for it
     } else {
         Rec r(this, nullptr);
-        TRYE(record_step(r, true, 0, false));
+        TRYE(record_step(r, STEP_HOST_DT, 0, false));
         CUE(cudaStreamSynchronize(s_));
     }
     return check_errors();
@@ -1191,7 +1197,7 @@ int Engine::run(int max_steps) {
         long long it = 0;
         while (h_flags_->anyLive) {
             if (++it > (long long)INT_MAX) break;
-            TRYE(record_step(r, false, 0, false));
+            TRYE(record_step(r, STEP_WHOLE, 0, false));
             TRYE(sync());
         }
     }

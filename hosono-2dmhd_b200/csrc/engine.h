@@ -219,7 +219,8 @@ struct KernelSet {
     void (*cfl_reduce)(const Batch&, cudaStream_t);
     void (*step_prepare)(const Batch&, int steps, cudaStream_t);
     void (*step_begin)(const Batch&, int use_host_dt, cudaStream_t);
-    void (*step_end)(const Batch&, cudaGraphConditionalHandle run_cond, cudaStream_t);
+    // turn: the next step begins here too (its CFL maxima came with rk_final)
+    void (*step_end)(const Batch&, cudaGraphConditionalHandle run_cond, int turn, cudaStream_t);
     // forward-Euler stage
     void (*face_pass1)(const Batch&, int uin, cudaStream_t);
     // one cluster per instance: the stage scalars, and pass 1's face cascade
@@ -250,7 +251,7 @@ struct KernelSet {
     // RK3 combines and boundary conditions
     void (*bc_fill)(const Batch&, int role, cudaStream_t);
     void (*rk_combine2)(const Batch&, cudaStream_t);
-    void (*rk_final)(const Batch&, cudaStream_t);
+    void (*rk_final)(const Batch&, int cfl, cudaStream_t);  // cfl: the next step's CFL maxima too
     void (*cons2prim_all)(const Batch&, cudaStream_t);
     // autotuner: mark the live, unfinished, not held instances as stepping
     // (on) or at rest (off) so that pass 1 can be timed outside a step

@@ -160,8 +160,9 @@ class Engine {
     int record_stage(Rec& r, int uin, int uout, cudaEvent_t ev0, cudaEvent_t ev1, bool head = true);
     template <class Cascade>
     int record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cascade_body);
-    int record_step(Rec& r, bool host_dt, cudaGraphConditionalHandle run_cond, bool profile,
-                    bool first_head = true);
+    enum StepForm { STEP_HOST_DT, STEP_WHOLE, STEP_TURN };
+    int record_begin(Rec& r);
+    int record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_cond, bool profile, bool first_head = true);
     int build_graphs();
     int launch(cudaGraphExec_t g);
     int sync();

@@ -42,12 +42,12 @@ hosono_stats stats_delta(const InstState& a, const InstState& b) {
     return s;
 }
 
-// kernels one graph execution launched, from the work counters: per step 4
-// time-loop kernels (cfl path) or 1 (host dt), 3 RK kernels; per stage the
-// two cluster kernels, the update and one pass-1 kernel per GP radius held;
+// kernels one graph execution launched, from the work counters: per step the
+// step end and 3 RK kernels, per run 3 to begin its first step (a host dt
+// needs none); per stage the two cluster kernels, the update and one pass-1 kernel per GP radius held;
 // what the kernel chain ran: 4 per face-cascade iteration, 9 per pass.
 long long graph_launches(const InstState& a, const InstState& b, int steps, bool host_dt, int radii) {
-    return (long long)steps * ((host_dt ? 1 : 4) + 3) + (3LL + radii) * (b.stages - a.stages) +
+    return (long long)steps * 4 + (host_dt ? 0 : 3) + (3LL + radii) * (b.stages - a.stages) +
            4LL * (b.chainIters - a.chainIters) + 9LL * (b.chainPasses - a.chainPasses);
 }
 

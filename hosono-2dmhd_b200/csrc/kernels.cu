@@ -1887,32 +1887,73 @@ __global__ void __launch_bounds__(NTHREADS) k_rk_combine2(Batch B) { PDL_ENTRY()
     FOR_TILES(B, t) t_rk_combine2(B, tile_at(B, t));
 }
 
+// |u| + c and |v| + c of one cell (cfl.f90:26-47) from its primitive variables
+__device__ __forceinline__ void cfl_speeds(const Phys& P, double rho, double pr, double gam, double vx, double vy, double bx,
+                                           double by, double bz, double& xm, double& ym) {
+    double cs;
+    if (P.force_hydro) {
+        cs = sqrt(gam * pr / rho);
+    } else {
+        const double BB = bx * bx + by * by + bz * bz;
+        const double bmin = fmin(fmin(fabs(bx), fabs(by)), fabs(bz));
+        cs = c_fs(gam, rho, pr, BB, bmin, +1.0);
+    }
+    xm = fabs(vx) + cs;
+    ym = fabs(vy) + cs;
+}
+// the warp's largest of a non-negative (or NaN: dropped, as fmax drops it)
+// value, as its bit pattern: such doubles order like their bits, so two
+// integer reductions of 32 bits give it
+__device__ __forceinline__ unsigned long long warp_max_bits(double x) {
+    const unsigned long long u = isnan(x) ? 0ull : (unsigned long long)__double_as_longlong(x);
+    const unsigned hi = (unsigned)(u >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)u : 0u);
+    return ((unsigned long long)top << 32) | lo;
+}
+
 // timeStep.f90:169 and :32-41: A = (U + 2 B)/3, V = cons2prim(A), on every
-// cell (guards from their images).  step_end makes A the state.
+// cell (guards from their images).  step_end makes A the state.  CFL: also the
+// next step's CFL maxima over the interior (cfl.f90:14-52), which are in
+// registers here: a pass over V (49 of its 80 bytes a cell) less per step of a
+// run.  The maxima only grow, so a warp whose own is not above the value it
+// reads leaves the atomic out.
+template <bool CFL>
 __device__ __forceinline__ void t_rk_final(const Batch& B, const Cell c) {
-    const InstState& S = B.st[c.k];
-    if (!S.stepping) return;
+    InstState& S = B.st[c.k];
+    if (!S.stepping) return;  // uniform over the block
     const InstDev& d = B.dev[c.k];
     const Geo& G = d.geo;
-    if (c.i >= G.nxt || c.j >= G.nyt) return;
-    const int si = bc_src(c.i, G.nx, G.g, G.bc), sj = bc_src(c.j, G.ny, G.g, G.bc);
-    const long long cc = (long long)c.j * G.pitch + c.i, s = (long long)sj * G.pitch + si;
-    const double* Un = role_ptr(d, S.parity, ROLE_STATE);
-    const double* Bb = role_ptr(d, S.parity, ROLE_B);
-    double* out = role_ptr(d, S.parity, ROLE_A);
-    double u[NCONS], V[NPRIM];
+    double xm = 0.0, ym = 0.0;
+    if (c.i < G.nxt && c.j < G.nyt) {
+        const int si = bc_src(c.i, G.nx, G.g, G.bc), sj = bc_src(c.j, G.ny, G.g, G.bc);
+        const long long cc = (long long)c.j * G.pitch + c.i, s = (long long)sj * G.pitch + si;
+        const double* Un = role_ptr(d, S.parity, ROLE_STATE);
+        const double* Bb = role_ptr(d, S.parity, ROLE_B);
+        double* out = role_ptr(d, S.parity, ROLE_A);
+        double u[NCONS], V[NPRIM];
 #pragma unroll
-    for (int v = 0; v < NCONS; v++) {
-        u[v] = (Un[v * G.plane + s] + 2 * Bb[v * G.plane + s]) / 3.0;
-        out[v * G.plane + cc] = u[v];
+        for (int v = 0; v < NCONS; v++) {
+            u[v] = (Un[v * G.plane + s] + 2 * Bb[v * G.plane + s]) / 3.0;
+            out[v * G.plane + cc] = u[v];
+        }
+        cons2prim(d.phys, u, V);
+#pragma unroll
+        for (int v = 0; v < NPRIM; v++) d.V[v * G.plane + cc] = V[v];
+        if (CFL && si == c.i && sj == c.j)
+            cfl_speeds(d.phys, V[DENS], V[PRES], V[GAMM], V[VELX], V[VELY], V[MAGX], V[MAGY], V[MAGZ], xm, ym);
     }
-    cons2prim(d.phys, u, V);
-#pragma unroll
-    for (int v = 0; v < NPRIM; v++) d.V[v * G.plane + cc] = V[v];
+    if (!CFL) return;
+    const unsigned long long bx = warp_max_bits(xm), by = warp_max_bits(ym);
+    if (threadIdx.x < 2) {
+        unsigned long long* m = &S.cflbits[threadIdx.x];
+        const unsigned long long mine = threadIdx.x ? by : bx;
+        if (mine > *reinterpret_cast<volatile unsigned long long*>(m)) atomicMax(m, mine);
+    }
 }
 // six resident blocks (40 registers) for more loads in flight
-__global__ void __launch_bounds__(NTHREADS, 6) k_rk_final(Batch B) { PDL_ENTRY();
-    FOR_TILES(B, t) t_rk_final(B, tile_at(B, t));
+template <bool CFL>
+__global__ void __launch_bounds__(NTHREADS, CFL ? 5 : 6) k_rk_final(Batch B) { PDL_ENTRY();
+    FOR_TILES(B, t) t_rk_final<CFL>(B, tile_at(B, t));
 }
 
 // V = cons2prim(state) on every cell (upload without V)
@@ -1948,18 +1989,8 @@ __device__ __forceinline__ void t_cfl_reduce(const Batch& B, const Cell c) {
     if (c.i >= G.g && c.j >= G.g && c.i < G.g + G.nx && c.j < G.g + G.ny) {
         const long long cc = (long long)c.j * G.pitch + c.i;
         const double* V = d.V;
-        const double rho = V[DENS * G.plane + cc], pr = V[PRES * G.plane + cc], gam = V[GAMM * G.plane + cc];
-        double cs;
-        if (d.phys.force_hydro) {
-            cs = sqrt(gam * pr / rho);
-        } else {
-            const double bx = V[MAGX * G.plane + cc], by = V[MAGY * G.plane + cc], bz = V[MAGZ * G.plane + cc];
-            const double BB = bx * bx + by * by + bz * bz;
-            const double bmin = fmin(fmin(fabs(bx), fabs(by)), fabs(bz));
-            cs = c_fs(gam, rho, pr, BB, bmin, +1.0);
-        }
-        xm = fabs(V[VELX * G.plane + cc]) + cs;
-        ym = fabs(V[VELY * G.plane + cc]) + cs;
+        cfl_speeds(d.phys, V[DENS * G.plane + cc], V[PRES * G.plane + cc], V[GAMM * G.plane + cc], V[VELX * G.plane + cc],
+                   V[VELY * G.plane + cc], V[MAGX * G.plane + cc], V[MAGY * G.plane + cc], V[MAGZ * G.plane + cc], xm, ym);
     }
     for (int o = 16; o > 0; o >>= 1) {
         xm = fmax(xm, __shfl_xor_sync(0xffffffffu, xm, o));
@@ -1992,26 +2023,30 @@ __global__ void __launch_bounds__(NTHREADS) k_cfl_reduce(Batch B) { PDL_ENTRY();
 
 // Step begin: dt = cfl * min(dx/xmax, dy/ymax) (cfl.f90:50) and validTimeStep
 // (mhd_driver.f90:117-144: clamp to tmax first, then reject negative, NaN or
-// infinite dt).  With use_host_dt the host already stored dt.
+// infinite dt).
+__device__ __forceinline__ void step_begin(const InstDev& d, InstState& S) {
+    const double xm = __longlong_as_double((long long)S.cflbits[0]);
+    const double ym = __longlong_as_double((long long)S.cflbits[1]);
+    double dt = d.cfl * fmin(d.geo.dx / xm, d.geo.dy / ym);
+    if (S.t + dt > S.tmax) {
+        dt = S.tmax - S.t;
+    } else if (dt < 0.0 || isnan(dt) || !isfinite(dt)) {
+        S.error = HOSONO_ENANDT;
+        S.done = 1;
+        S.stepping = 0;
+    }
+    S.dt = dt;
+    S.dtdx = dt / d.geo.dx;
+    S.dtdy = dt / d.geo.dy;
+}
 __global__ void k_step_begin(Batch B, int use_host_dt) { PDL_ENTRY();
+    if (use_host_dt) return;  // the host already stored dt
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
         if (!S.stepping) continue;
-        if (use_host_dt) continue;
-        const InstDev& d = B.dev[k];
-        const double xm = __longlong_as_double((long long)S.cflbits[0]);
-        const double ym = __longlong_as_double((long long)S.cflbits[1]);
-        double dt = d.cfl * fmin(d.geo.dx / xm, d.geo.dy / ym);
-        if (S.t + dt > S.tmax) {
-            dt = S.tmax - S.t;
-        } else if (dt < 0.0 || isnan(dt) || !isfinite(dt)) {
-            S.error = HOSONO_ENANDT;
-            S.done = 1;
-            S.stepping = 0;
-        }
-        S.dt = dt;
-        S.dtdx = dt / d.geo.dx;
-        S.dtdy = dt / d.geo.dy;
+        step_begin(B.dev[k], S);
+        S.cflbits[0] = 0;  // rk_final collects the next step's
+        S.cflbits[1] = 0;
     }
 }
 
@@ -2028,8 +2063,9 @@ __global__ void k_step_prepare(Batch B, int /*unused*/) { PDL_ENTRY();
 
 // Step end: the new state is buffer A (parity flips), t += dt, nstep += 1,
 // and the time-loop test of mhd_driver.f90:76; next step's participants and
-// the batch condition.
-__global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle) { PDL_ENTRY();
+// the batch condition.  turn: the run goes on in the same launch, so the next
+// step begins here (its CFL maxima came with rk_final).
+__global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle, int turn) { PDL_ENTRY();
     __shared__ int any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
@@ -2042,15 +2078,25 @@ __global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle
             if (!((S.t < S.tmax) && (S.nstep < S.nstepmax))) S.done = 1;
         }
         S.stepping = 0;  // at rest between launches; step_prepare picks the next participants
-        S.cflbits[0] = 0;
-        S.cflbits[1] = 0;
         if (S.live && !S.done && !B.hold[k]) any = 1;
     }
     __syncthreads();
+    __shared__ int go;
     if (threadIdx.x == 0) {
         const int left = --B.flags->stepsLeft;
-        B.flags->anyLive = any && left > 0;
-        if (set_handle) cudaGraphSetConditional(h, (any && left > 0) ? 1u : 0u);
+        go = any && left > 0;
+        B.flags->anyLive = go;
+        if (set_handle) cudaGraphSetConditional(h, go ? 1u : 0u);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
+        InstState& S = B.st[k];
+        if (turn && go && S.live && !S.done && !B.hold[k]) {
+            S.stepping = 1;
+            step_begin(B.dev[k], S);
+        }
+        S.cflbits[0] = 0;
+        S.cflbits[1] = 0;
     }
 }
 
@@ -2224,8 +2270,8 @@ void lk(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t
 void l_cfl_reduce(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_cfl_reduce, B, s); }
 void l_step_prepare(const Batch& B, int steps, cudaStream_t s) { lk(k_step_prepare, dim3(1), dim3(128), 0, s, B, steps); }
 void l_step_begin(const Batch& B, int use_host_dt, cudaStream_t s) { lk(k_step_begin, dim3(1), dim3(128), 0, s, B, use_host_dt); }
-void l_step_end(const Batch& B, cudaGraphConditionalHandle h, cudaStream_t s) {
-    lk(k_step_end, dim3(1), dim3(128), 0, s, B, h, (int)(h != 0));
+void l_step_end(const Batch& B, cudaGraphConditionalHandle h, int turn, cudaStream_t s) {
+    lk(k_step_end, dim3(1), dim3(128), 0, s, B, h, (int)(h != 0), turn);
 }
 // dynamic shared memory of a pass-1 kernel variant
 template <int R, int NBUF>
@@ -2378,7 +2424,12 @@ void l_clear_low(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low, B, s
 void l_clear_low_pass1(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low_pass1, B, s); }
 void l_bc_fill(const Batch& B, int role, cudaStream_t s) { TILE_LAUNCH(k_bc_fill, B, s, role); }
 void l_rk_combine2(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_rk_combine2, B, s); }
-void l_rk_final(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_rk_final, B, s); }
+void l_rk_final(const Batch& B, int cfl, cudaStream_t s) {
+    if (cfl)
+        TILE_LAUNCH(k_rk_final<true>, B, s);
+    else
+        TILE_LAUNCH(k_rk_final<false>, B, s);
+}
 void l_cons2prim_all(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_cons2prim_all, B, s); }
 void l_tune_mark(const Batch& B, int on, cudaStream_t s) { lk(k_tune_mark, dim3(1), dim3(128), 0, s, B, on); }
 // every block resident at once: a cooperative launch of as many blocks as
@@ -2404,7 +2455,7 @@ void l_launch_info(int R, int maxTiles, int* pass1, int* tile_grid_max) {
     const void* tile_kernels[] = {(const void*)k_cfl_reduce,     (const void*)k_cascade_lower,
                                    (const void*)k_compact_next, (const void*)k_compact_post,
                                   (const void*)k_compact_dirty,  (const void*)k_ct_update_detect, (const void*)k_mood_flags,
-                                  (const void*)k_bc_fill,        (const void*)k_rk_combine2,  (const void*)k_rk_final,
+                                  (const void*)k_bc_fill,        (const void*)k_rk_combine2,  (const void*)k_rk_final<false>,
                                   (const void*)k_cons2prim_all};
     int mx = 0;
     for (const void* k : tile_kernels) {
