@@ -23,8 +23,15 @@ struct DeviceAllocator {
 };
 
 // Most listed cells (pass 1's failing cells, then the cells detect lowered in
-// it) an instance may have for one cluster to take its stage.
-constexpr int kClusterCells = 2000;
+// it) an instance may have for one cluster to take its stage; above it the
+// kernel chain, which has the whole GPU for a pass but nine launches.  ms per
+// step with 200 / 400 / 800 / 2000 / all in the cluster / none: blast 256^2 R=3
+// from t=0.01 2.30 / 1.70 / 1.59 / 1.58 / - / 2.3, blast 512^2 R=3 from 0.015
+// 3.31 / 3.31 / 3.31 / 5.02 / 5.16 / 3.47, blast 1024^2 R=2 from 0.01 4.00 / 4.00
+// / 4.00 / 4.02 / 6.61 / 4.17, Orszag-Tang 256^2 R=2 from 0.3 3.08 / 3.08 / 3.00;
+// a batch of 16 blasts, whose instances then share a stage's launches, 132 / 101
+// / 92 / 92 ms.
+constexpr int kClusterCells = 800;
 
 class Engine {
   public:
