@@ -171,8 +171,10 @@ struct GroupDiv {
 // The solver's ranges: b in [2^-100, 2^101) and a down to 2^-860 keep every
 // intermediate normal (the quotient above 2^-962, the remainder a multiple of
 // 2^-965); momenta ahead of a front fall off by orders of magnitude a cell, so
-// the numerators' range is the wide one.
-typedef GroupDiv<-860, 900, -100, 100> SolverDiv;
+// the numerators' range is the wide one.  Below 2^301 they keep every product
+// of the solver finite, which the terms it leaves out need: zero times a
+// finite value.
+typedef GroupDiv<-860, 300, -100, 100> SolverDiv;
 // one quotient at a time over a symmetric range, as tests/div_check.cu drives it
 struct SharedRecipDiv {
     GroupDiv<-500, 500, -500, 500> g;
@@ -487,7 +489,11 @@ __device__ __forceinline__ bool face_solve(const Phys& s, const double* uL, cons
         if (S::Z) uStr[MOMZ_] = uStr[DENS] * (left ? L.vZ : R.vZ);
         double pStr = L.rho * dL * (sStr - L.vN) + pTotL;
         if (S::H) {
-            // without a field the HLL state enters no other term
+            // without a field the HLL state enters no other term, and its
+            // products with it are zeros where its velocity is finite: where
+            // its density is not lost to rounding (a side beyond Mach 2^53)
+            g.watch(sR - sL);
+            floored = floored || !(sR * uR[DENS] - sL * uL[DENS] + fL[DENS] - fR[DENS] > 0x1p-300);
             uStr[ENER] = g.div(eK * dK + pStr * sStr - pTotK * vNK, rK);
         } else {
             double uHLL[NCONS];
