@@ -1035,6 +1035,8 @@ int Engine::record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cas
         TRYE(b.k([&](cudaStream_t s) { K->compact_post(B, s); }));
         TRYE(b.k([&](cudaStream_t s) { K->flux_list(B, uin, s); }));
         TRYE(b.k([&](cudaStream_t s) { K->ct_list(B, uin, uout, s); }));
+        const bool rest = B.mcMax >= 0;  // short passes go to the clusters
+        if (rest) TRYE(b.k([&](cudaStream_t s) { K->handover(B, s); }));
         if (trace) {  // the trace reads `lowered` before it is cleared
             TRYE(b.k([&](cudaStream_t s) { K->mood_flags(B, MOOD_FLAGS_LISTS, s); }));
             TRYE(b.host([&] { return trace_snapshot(); }));
@@ -1044,6 +1046,7 @@ int Engine::record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cas
         }
         if (!b.graph()) launches += 2;  // three kernels
         TRYE(b.k([&](cudaStream_t s) { K->pass_end(B, hm, 0, s); }));
+        if (rest) TRYE(b.k([&](cudaStream_t s) { K->mood_passes_rest(B, uin, uout, s); }));
         if (trace) TRYE(b.host([&] { return trace_after_pass(); }));
         return HOSONO_OK;
     }));

@@ -93,7 +93,9 @@ struct InstState {
     int nextIter;    // face cascade: this instance runs the next inner iteration
     int cascaded;    // face cascade ran in the current pass (kernel-chain form)
     int big;         // this stage's work lists are too long for one cluster: the kernel chain takes it
+    int hand;        // the chain leaves the rest of the stage's passes to the cluster form
     int cFail;       // cells that failed CAD/PAD in pass 1 (its list of them)
+    int cLow;        // lowered cells of the pass at which it did
     int nCasc;       // cells on the cluster form's cascade-lowered list
     int mc[10];      // the cluster form's list counters (mood_cluster.cuh MC_*)
     int nInner, nDetect;  // lowerings in the current pass
@@ -229,6 +231,10 @@ struct KernelSet {
     // one cluster per instance: the end of pass 1 and every later pass of the
     // stage; h: some instance is left to the chain
     void (*mood_passes)(const Batch&, int uin, int uout, cudaGraphConditionalHandle h, cudaStream_t);
+    // in the chain's loop: list the instances whose pass lowered few cells for
+    // the clusters (after detect, before the flag rebuild), and run them
+    void (*handover)(const Batch&, cudaStream_t);
+    void (*mood_passes_rest)(const Batch&, int uin, int uout, cudaStream_t);
     void (*cascade_cond)(const Batch&, cudaGraphConditionalHandle h, cudaStream_t);
     // face cascade: the kernels walk the tiles of the instances in the
     // current iteration (Batch::casRange); `later` marks a later MOOD pass

@@ -45,10 +45,10 @@ hosono_stats stats_delta(const InstState& a, const InstState& b) {
 // kernels one graph execution launched, from the work counters: per step the
 // step end and 3 RK kernels, per run 3 to begin its first step (a host dt
 // needs none); per stage the two cluster kernels, the update and one pass-1 kernel per GP radius held;
-// what the kernel chain ran: 4 per face-cascade iteration, 9 per pass.
+// what the kernel chain ran: 4 per face-cascade iteration, 11 per pass.
 long long graph_launches(const InstState& a, const InstState& b, int steps, bool host_dt, int radii) {
     return (long long)steps * 4 + (host_dt ? 0 : 3) + (3LL + radii) * (b.stages - a.stages) +
-           4LL * (b.chainIters - a.chainIters) + 9LL * (b.chainPasses - a.chainPasses);
+           4LL * (b.chainIters - a.chainIters) + 11LL * (b.chainPasses - a.chainPasses);
 }
 
 }  // namespace

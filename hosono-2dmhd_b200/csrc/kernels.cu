@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <map>
 #include <mutex>
 
 #include "engine.h"
@@ -996,7 +997,7 @@ __device__ __forceinline__ bool recon_cell_group(const InstDev& d, const InstSta
         if (sub == 0) {
             const int rN = min(s, (int)sch[cc + G.pitch]), rS = min(s, (int)sch[cc - G.pitch]);
             const int rE = min(s, (int)sch[cc + 1]), rW = min(s, (int)sch[cc - 1]);
-            d.dirty[cc] = 1;
+            if (S.passes == 0) d.dirty[cc] = 1;  // read after pass 1's cascade only
             d.rrRec[cc] = (uint8_t)(rN | (rS << 2) | (rE << 4) | (rW << 6));
         }
         if (rr > 0 && q <= rr) {
@@ -1623,6 +1624,7 @@ __device__ __forceinline__ bool mood_flags_cell(const InstDev& d, const InstStat
     const long long cc = (long long)j * G.pitch + i;
     d.rec[cc] = rec;
     d.recF[cc] = recF;
+    d.dirty[cc] = 0;
     schN[cc] = (int8_t)s;
     d.detMask[cc] &= (uint8_t)~DM_CASC;
     return rec;
@@ -1678,6 +1680,31 @@ __device__ __forceinline__ void set_rec(const Batch& B, const InstDev& d, long l
             B.L.counts[LIST_OVERFLOW] = 1;
     }
 }
+// The chain hands an instance to the clusters when a pass of it lowered few
+// cells: the passes left are short.  Decided by values that stand from detect
+// to pass_end; the flag rebuild then leaves the instance's scheme, `lowered`
+// and cascade marks to the cluster form, which starts with them.
+__device__ __forceinline__ bool hand_over(const Batch& B, const InstState& S) {
+    return S.big && S.stageActive && S.nDetect > 0 && S.nDetect <= B.mcMax && S.passes + 1 < S.passCap;
+}
+// its lowered cells, and the cells its cascade lowered, into the instance's
+// segment of the cascade list `next`, free between the passes
+__global__ void __launch_bounds__(256) k_handover(Batch B) { PDL_ENTRY();
+    const int nL = min(B.L.counts[LIST_LOW], (int)B.L.cap), nC = min(B.L.counts[LIST_CASC], (int)B.L.cap);
+    for (int e = GT1; e < nL + nC; e += GS1) {
+        const bool low = e < nL;
+        const int2 it = low ? B.L.low[e] : B.L.casc[e - nL];
+        InstState& S = B.st[it.x];
+        if (!hand_over(B, S)) continue;
+        const int2 tl = B.instTiles[it.x];
+        int* seg = reinterpret_cast<int*>(B.L.next + (long long)tl.x * (TILE_X * TILE_Y));
+        if (low)
+            seg[atomicAdd(&S.cLow, 1)] = it.y;
+        else
+            seg[(long long)tl.y * (TILE_X * TILE_Y) + atomicAdd(&S.nCasc, 1)] = it.y;
+    }
+}
+
 __device__ __forceinline__ void sync_cell(const Batch& B, int e, int nLow, int2* it_out, bool* from_low) {
     *from_low = e < nLow;
     *it_out = *from_low ? B.L.low[e] : B.L.casc[e - nLow];
@@ -1723,6 +1750,7 @@ __device__ __forceinline__ void d_flags_scatter(const Batch& B, int gt, int gs) 
         sync_cell(B, e, nL, &it, &fromLow);
         const InstDev& d = B.dev[it.x];
         const InstState& S = B.st[it.x];
+        if (hand_over(B, S)) continue;
         const Geo& G = d.geo;
         const int8_t* sch = d.scheme[S.schemeSel];
         const long long c0 = it.y;
@@ -1764,6 +1792,7 @@ __device__ __forceinline__ void d_scheme_sync(const Batch& B, int clear_low, int
         int2 it;
         bool fromLow;
         sync_cell(B, e, nL, &it, &fromLow);
+        if (hand_over(B, B.st[it.x])) continue;
         const InstDev& d = B.dev[it.x];
         const Geo& G = d.geo;
         int8_t* sch = d.scheme[B.st[it.x].schemeSel];
@@ -1799,6 +1828,7 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
     for (int k = tid; k < B.maxInst; k += NT) {
         InstState& S = B.st[k];
         if (!(S.stepping && S.stageActive)) continue;
+        const bool hand = !flip && hand_over(B, S);
         if (flip && pass_lowered(S)) S.schemeSel = 1 - S.schemeSel;  // k_mood_flags wrote the other buffer
         S.passes++;
         S.passesTotal++;
@@ -1807,7 +1837,10 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
         S.detectTotal += S.nDetect;
         S.lastInner = S.nInner;
         S.lastDetect = S.nDetect;
-        if (S.nDetect == 0) {
+        if (hand) {
+            S.hand = 1;
+            S.stageActive = 0;
+        } else if (S.nDetect == 0) {
             S.stageActive = 0;
             if (S.passes > S.maxPasses) S.maxPasses = S.passes;
         } else if (S.passes >= S.passCap) {
@@ -2336,29 +2369,38 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
 }
 // One cluster per instance slot: 16 blocks (a non-portable size, taken where
 // the GPU can place one) for up to nine slots, which fills the GPU, else 8.
+// The shared memory a cluster kernel needs is static; 16 blocks take leave.
+template <typename K>
+bool cluster_sixteen(K kernel) {
+    if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(MC_THREADS);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n >= 1;
+}
 template <typename K>
 int cluster_blocks(K kernel, int maxInst) {
-    static const bool sixteen = [kernel] {  // once per process and kernel (thread-safe static initialisation)
-        if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(MC_THREADS);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 16;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return n >= 1;
-    }();
+    // asked once per kernel and process, under a lock (engines on several host threads)
+    static std::mutex mu;
+    static std::map<const void*, bool> known;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find((const void*)kernel);
+    if (it == known.end()) it = known.emplace((const void*)kernel, cluster_sixteen(kernel)).first;
+    const bool sixteen = it->second;
     return sixteen && maxInst <= 9 ? 16 : 8;
 }
 template <typename... KArgs, typename... Args>
@@ -2380,8 +2422,13 @@ void l_mood_faces(const Batch& B, int uin, cudaGraphConditionalHandle h, cudaStr
     lk_cluster(k_mood_faces, cluster_blocks(k_mood_faces, B.maxInst), B, s, uin, h, (int)(h != 0));
 }
 void l_mood_passes(const Batch& B, int uin, int uout, cudaGraphConditionalHandle h, cudaStream_t s) {
-    lk_cluster(k_mood_passes, cluster_blocks(k_mood_passes, B.maxInst), B, s, uin, uout, h, (int)(h != 0));
+    lk_cluster(k_mood_passes<false>, cluster_blocks(k_mood_passes<false>, B.maxInst), B, s, uin, uout, h, (int)(h != 0));
 }
+void l_mood_passes_rest(const Batch& B, int uin, int uout, cudaStream_t s) {
+    lk_cluster(k_mood_passes<true>, cluster_blocks(k_mood_passes<true>, B.maxInst), B, s, uin, uout,
+               (cudaGraphConditionalHandle)0, 0);
+}
+void l_handover(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_handover, B, s); }
 void l_cascade_cond(const Batch& B, cudaGraphConditionalHandle h, cudaStream_t s) {
     lk(k_cascade_cond, dim3(1), dim3(PASS_END_THREADS), 0, s, B, h, (int)(h != 0));
 }
@@ -2473,7 +2520,7 @@ const KernelSet kset = {
 #else
     "strict",
 #endif
-    l_cfl_reduce, l_step_prepare, l_step_begin, l_step_end, l_face_pass1, l_mood_faces, l_mood_passes, l_cascade_cond, l_cascade_lower,
+    l_cfl_reduce, l_step_prepare, l_step_begin, l_step_end, l_face_pass1, l_mood_faces, l_mood_passes, l_handover, l_mood_passes_rest, l_cascade_cond, l_cascade_lower,
     l_recon_check, l_ct_update_detect, l_mood_flags, l_pass_end, l_recon_list,
     l_compact_post, l_compact_dirty, l_flux_list, l_ct_list, l_clear_low, l_clear_low_pass1, l_bc_fill, l_rk_combine2, l_rk_final,
     l_cons2prim_all, l_tune_mark, l_mood_rest, l_launch_info, &mops};

@@ -737,7 +737,10 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_faces(Batch B, int uin, 
 }
 
 // After the pass-1 update: the end of pass 1 and every later MOOD pass of the
-// instances whose lowered cells are few.
+// instances whose lowered cells are few.  REST: in the chain's loop, the passes
+// left of the instances it hands over (hand_over), from the lists k_handover
+// made.
+template <bool REST>
 __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin, int uout,
                                                              cudaGraphConditionalHandle h, int set_handle) {
     PDL_ENTRY();
@@ -745,25 +748,31 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
     const McT t = mc_place();
     const int k = blockIdx.x / cluster_nctaid();
     InstState& S = B.st[k];
-    const bool on = S.stepping != 0;
+    const bool on = S.stepping != 0 && (!REST || S.hand);
     const bool lead = t.lead;
     bool left = false;
     if (on) {
-        int nLow = mc_ld(&S.nDetect), nCasc = mc_ld(&S.nCasc);
-        left = S.big || nLow > B.mcMax;
+        int nLow = mc_ld(REST ? &S.cLow : &S.nDetect), nCasc = mc_ld(&S.nCasc);
+        left = !REST && (S.big || nLow > B.mcMax);
         if (left) {
             if (lead) {
                 S.big = 1;
                 S.nCasc = 0;  // the dense flag rebuild clears the cascade's marks
             }
         } else {
-            int inner = S.nInner, passes = 1, lastInner = inner, lastDetect = nLow;
-            long long innerSum = inner, detectSum = nLow;
+            const int before = REST ? S.passes : 0;  // passes the chain has counted
+            int inner = S.nInner, passes = REST ? before : 1, lastInner = inner, lastDetect = nLow;
+            long long innerSum = inner, detectSum = REST ? 0 : nLow;
             int iters = 0;
             bool capped = false;
             if (nLow > 0 || nCasc > 0) {
                 mc_setup(B, k, uin, uout, m);
                 const int cap = S.passCap;
+                if (REST) {
+                    const int* cascRest = m.next + (long long)B.instTiles[k].y * (TILE_X * TILE_Y);
+                    for (int e = t.gw * 32 + t.lane; e < nLow; e += t.nw * 32) m.low[e] = m.next[e];
+                    for (int e = t.gw * 32 + t.lane; e < nCasc; e += t.nw * 32) m.casc[e] = cascRest[e];
+                }
                 cluster_sync();  // every block has read the scalars
                 int cur = 0, nRec = 0, nRecF = 0;
                 bool listed = true;  // the last pass's lowerings are on the low and cascade lists
@@ -822,8 +831,10 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
                 S.nDetect = 0;
                 S.nCasc = 0;
                 S.nInner = 0;
+                S.cLow = 0;
+                S.hand = 0;
                 S.passes = passes;
-                S.passesTotal += passes;
+                S.passesTotal += passes - before;
                 S.innerTotal += innerSum;
                 S.detectTotal += detectSum;
                 S.lastInner = lastInner;
