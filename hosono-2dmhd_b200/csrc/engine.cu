@@ -3,14 +3,20 @@
 // loop of mhd_driver.f90:76-95) recorded either as eager launches driven by
 // host loops, or as one CUDA graph whose loops are conditional WHILE nodes:
 //
-//   run:   WHILE(any instance stepping) {
-//            step_prepare, cfl_reduce, step_begin (dt, validTimeStep)
-//            stage(U->A), bc(A), stage(A->B), A=(3U+B)/4, stage(A->B), A=(U+2B)/3 + V
-//            step_end (t += dt, state = A) }
-//   stage: init, pass-1 kernel, WHILE(cascade) {lower, re-reconstruct}, fluxes,
-//          FLICD+update+detect, flags, pass_end,
-//          WHILE(MOOD) { re-reconstruct flagged, WHILE(cascade) {...}, fluxes,
-//                        FLICD+update+detect, flags, pass_end }
+//   run:   step_prepare, cfl_reduce, step_begin (dt, validTimeStep)
+//          WHILE(any instance stepping) {
+//            stage(U->A), bc(A), stage(A->B), A=(3U+B)/4, stage(A->B),
+//            A=(U+2B)/3 + V + the next step's CFL maxima
+//            step_end (t += dt, state = A, the next dt) }
+//   stage: pass-1 kernel, mood_faces (one cluster per instance: face cascade, fluxes),
+//          IF(an instance was too big for it) {
+//            WHILE(cascade) {lower, re-reconstruct}, fluxes }
+//          FLICD+update+detect,
+//          mood_passes (one cluster per instance: flags and every later pass),
+//          IF(an instance was too big for it) { flags, pass_end,
+//            WHILE(MOOD) { re-reconstruct flagged, WHILE(cascade) {...}, fluxes,
+//                          FLICD+update+detect, flags, pass_end,
+//                          mood_passes for instances whose passes got short } }
 //
 // Each loop condition is set on the device by the kernel that ends the loop
 // body (cudaGraphSetConditional), so a whole run is one graph launch.
@@ -806,7 +812,7 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     st.stepping = 1;
     st.error = 0;
     TRYE(write_state(slot, st));
-    TRYE(build_graphs());
+    TRYE(build_graph(&Engine::gAdvRest_));
     // the copies start once everything before on the main stream is done with the staging buffer
     CUE(cudaEventRecord(bandEv_[HOSONO_UPLOAD_BANDS_MAX], s_));
     CUE(cudaStreamWaitEvent(sCopy_, bandEv_[HOSONO_UPLOAD_BANDS_MAX], 0));
@@ -1084,40 +1090,43 @@ int Engine::record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_co
     return HOSONO_OK;
 }
 
-int Engine::build_graphs() {
-    if (gAdvance_) return HOSONO_OK;
-    graphRadii_ = radii_;
-    for (int which = 0; which < 4; which++) {
-        cudaGraph_t g;
-        CUE(cudaGraphCreate(&g, 0));
-        Rec r(this, g);
-        int rc;
-        if (which == 0) {
-            rc = record_step(r, STEP_HOST_DT, 0, false);
-        } else if (which == 3) {  // the banded upload ran the first stage's set-up and pass 1
-            rc = record_step(r, STEP_HOST_DT, 0, false, false);
-        } else if (which == 2) {
-            // one step at the graph's top level: event records are not allowed
-            // inside conditional bodies, and pass 1 sits outside the MOOD loops
-            rc = record_step(r, STEP_WHOLE, 0, true);
-        } else {
-            cudaGraphConditionalHandle hr;
-            rc = record_begin(r);
-            if (!rc) rc = r.cond(&hr, 1);
-            if (!rc)
-                rc = r.loop(hr, &BatchFlags::anyLive, INT_MAX,
-                            [&](Rec& b) -> int { return record_step(b, STEP_TURN, hr, false); });
-        }
-        if (!rc) rc = r.end();
-        if (rc) {
-            cudaGraphDestroy(g);
-            return rc;
-        }
-        cudaGraphExec_t ex;
-        cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+// A graph is recorded when a call first needs it.  Recording and instantiating
+// one takes 1.1-1.6 ms of a new handle's first step (all four took 3-4.6 ms:
+// blast 64^2, two driver steps of a new handle 11.1 -> 4.6 ms; Orszag-Tang
+// 1024^2 through host buffers 8.4 -> 5.6 ms; 2048^2, two steps 32.7 -> 21.4).
+int Engine::build_graph(cudaGraphExec_t Engine::*which) {
+    if (this->*which) return HOSONO_OK;
+    graphRadii_ = radii_;  // a subset of the radii of the graphs there are
+    cudaGraph_t g;
+    CUE(cudaGraphCreate(&g, 0));
+    Rec r(this, g);
+    int rc;
+    if (which == &Engine::gAdvance_) {
+        rc = record_step(r, STEP_HOST_DT, 0, false);
+    } else if (which == &Engine::gAdvRest_) {  // the banded upload ran the first stage's pass 1
+        rc = record_step(r, STEP_HOST_DT, 0, false, false);
+    } else if (which == &Engine::gProf_) {
+        // one step at the graph's top level: event records are not allowed
+        // inside conditional bodies, and pass 1 sits outside the MOOD loops
+        rc = record_step(r, STEP_WHOLE, 0, true);
+    } else {
+        cudaGraphConditionalHandle hr;
+        rc = record_begin(r);
+        if (!rc) rc = r.cond(&hr, 1);
+        if (!rc)
+            rc = r.loop(hr, &BatchFlags::anyLive, INT_MAX,
+                        [&](Rec& b) -> int { return record_step(b, STEP_TURN, hr, false); });
+    }
+    if (!rc) rc = r.end();
+    if (rc) {
         cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(HOSONO_ECUDA, "graph instantiate: %s", cudaGetErrorString(e));
-        (which == 0 ? gAdvance_ : which == 1 ? gRun_ : which == 2 ? gProf_ : gAdvRest_) = ex;
+        return rc;
+    }
+    cudaError_t e = cudaGraphInstantiate(&(this->*which), g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        this->*which = nullptr;
+        return fail(HOSONO_ECUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
     return HOSONO_OK;
 }
@@ -1174,7 +1183,7 @@ int Engine::advance(int slot, double dt) {
     st.error = 0;
     TRYE(write_state(slot, st));
     if (use_graphs && !trace) {
-        TRYE(build_graphs());
+        TRYE(build_graph(&Engine::gAdvance_));
         CUE(cudaGraphLaunch(gAdvance_, s_));  // check_errors waits for it
     } else {
         Rec r(this, nullptr);
@@ -1191,7 +1200,7 @@ int Engine::run(int max_steps) {
     f.stepsLeft = max_steps > 0 ? max_steps : INT_MAX;
     CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
     if (use_graphs && !trace) {
-        TRYE(build_graphs());
+        TRYE(build_graph(&Engine::gRun_));
         CUE(cudaGraphLaunch(gRun_, s_));  // check_errors waits for it
     } else {
         Rec r(this, nullptr);
@@ -1213,7 +1222,7 @@ int Engine::run_profiled_step(double* pass1_ms, int* pass1_launches) {
     f.radii = radii_;
     f.stepsLeft = 1;
     CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
-    TRYE(build_graphs());
+    TRYE(build_graph(&Engine::gProf_));
     TRYE(launch(gProf_));
     double ms = 0;
     for (int st = 0; st < 3; st++) {

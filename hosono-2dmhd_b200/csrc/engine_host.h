@@ -170,7 +170,7 @@ class Engine {
     enum StepForm { STEP_HOST_DT, STEP_WHOLE, STEP_TURN };
     int record_begin(Rec& r);
     int record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_cond, bool profile, bool first_head = true);
-    int build_graphs();
+    int build_graph(cudaGraphExec_t Engine::*which);
     int launch(cudaGraphExec_t g);
     int sync();
     int check_errors();
