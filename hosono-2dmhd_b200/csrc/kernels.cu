@@ -22,6 +22,7 @@
 #include <cstddef>
 #include <map>
 #include <mutex>
+#include <utility>
 
 #include "engine.h"
 #include "hosono_gpu.h"
@@ -143,10 +144,6 @@ __device__ __forceinline__ void face_value(const InstDev& d, const double* __res
         gp_face<3>(U, G.plane, G.pitch, i, j, pvq, out);
 }
 
-__device__ __forceinline__ void warp_flag(int* flag, bool v) {
-    const unsigned m = __ballot_sync(0xffffffffu, v);
-    if (m && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
-}
 __device__ __forceinline__ void warp_count(int* counter, bool v) {
     const unsigned m = __ballot_sync(0xffffffffu, v);
     if (m && (threadIdx.x & 31) == 0) atomicAdd(counter, __popc(m));
@@ -672,13 +669,19 @@ static __device__ __noinline__ void p1_refill(P1Ctl* ctl) {
 //
 // MINB is the number of resident blocks per SM the register budget aims at
 // (launch bounds: 128 registers at 2, 80 at 3, 64 at 4).  With two boxes the
-// next tile's box loads while the current one is computed; with one box a
-// block loads, computes, then loads the next, and relies on the other
-// resident blocks to hide the load.  One box takes 36 KB less shared memory
-// per block, which the SM gives to L1, where the kernel's register spills
-// live: at two blocks per SM that wins over double-buffering on the 2048^2
-// workloads.  Three or four blocks per SM keep one box (their shared memory
-// would not fit two).
+// next tile's box loads while the current one is computed; with one box (TMA)
+// the last thread that reads it has it refilled, beside the tile's last
+// solves.  One box takes 36 KB less shared memory per block, which the SM gives
+// to L1, where the kernel's register spills live: at two blocks per SM that
+// wins over double-buffering on the 2048^2 workloads.  Three or four blocks per
+// SM keep one box.
+//
+// What bounds the kernel: FP64 latency.  Orszag-Tang 1024^2 R=2: 0.467 ms, the
+// FP64 pipe 57 % active at 4 warps a scheduler (0.27 ms were it full); 730 of a
+// warp's 1,480 instructions a solve are FP64; stalls per instruction 1.8 on fixed
+// latencies, 0.8 on the pipe, 0.95 on L1 and shared memory (spills, descriptors),
+// 0.3 on the tile's barrier, 0.3 on instruction fetch.  Before the shared sweeps,
+// face coordinates and zero planes: 0.720 ms, 1,058 of 2,183 instructions.
 constexpr int P1_HALF = 2;             // half-tile units below this many whole tiles per block
 constexpr int P1_THREAD = 3 * NCONS;  // doubles of shared memory per thread: accumulators, parked face states
 template <int R>
@@ -1466,15 +1469,17 @@ __device__ __forceinline__ void t_ct_update_detect(const Batch& B, int uin, int 
     }
     low_append(B, c.k, low, cc);
 }
-constexpr int MINB_CT = 5;
-// six resident blocks (a 40-register budget, a few hundred bytes of spills):
-// the tile's loads wait at two barriers, so more warps in flight keep HBM
-// busier.  Per step on Orszag-Tang 2048^2: 3 blocks (80 registers) 11.66 ms,
-// 4 blocks 11.23 ms, 5 blocks 11.14 ms, 6 blocks 11.08 ms.  Computing each
-// cell's corrected fluxes once into shared memory (instead of a cell also
-// evaluating its east and north neighbours' FLICD) made a launch about 5 %
-// slower: the extra barrier costs more than the loads it saves, which hit L1.
-__global__ void __launch_bounds__(NTHREADS, MINB_CT) k_ct_update_detect(Batch B, int uin, int uout) { PDL_ENTRY();
+// Five resident blocks (48 registers): the tile's loads wait at two barriers,
+// so warps in flight keep HBM busy, but spills are half of what the load/store
+// unit does at six (40 registers).  ms per step at 4 / 5 / 6: Orszag-Tang
+// 2048^2 6.73 / 6.61 / 6.77, 1024^2 1.89 / 1.87 / 1.90, Sedov 1024^2 1.70 / 1.69 /
+// 1.70.  A launch at 2048^2 takes 292 us for 1.1 GB (0.59 of the copy
+// bandwidth; 324 us before the sensors' divisions went).  Computing each cell's
+// corrected fluxes once into shared memory (instead of a cell also evaluating
+// its east and north neighbours' FLICD) made a launch about 5 % slower: the
+// extra barrier costs more than the loads it saves, which hit L1; prefetching
+// the next tile to L2 made it 30 % slower.
+__global__ void __launch_bounds__(NTHREADS, 5) k_ct_update_detect(Batch B, int uin, int uout) { PDL_ENTRY();
     __shared__ double sV[4 * DP_SX * DP_SY];
     FOR_TILES(B, t) t_ct_update_detect(B, uin, uout, tile_at(B, t), sV);
 }
@@ -2394,14 +2399,17 @@ bool cluster_sixteen(K kernel) {
 }
 template <typename K>
 int cluster_blocks(K kernel, int maxInst) {
-    // asked once per kernel and process, under a lock (engines on several host threads)
+    // asked once per device and kernel (the leave is the device's), under a lock
+    // (engines on several host threads)
     static std::mutex mu;
-    static std::map<const void*, bool> known;
+    static std::map<std::pair<int, const void*>, bool> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
-    auto it = known.find((const void*)kernel);
-    if (it == known.end()) it = known.emplace((const void*)kernel, cluster_sixteen(kernel)).first;
-    const bool sixteen = it->second;
-    return sixteen && maxInst <= 9 ? 16 : 8;
+    const auto key = std::make_pair(dev, (const void*)kernel);
+    auto it = known.find(key);
+    if (it == known.end()) it = known.emplace(key, cluster_sixteen(kernel)).first;
+    return it->second && maxInst <= 9 ? 16 : 8;
 }
 template <typename... KArgs, typename... Args>
 void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t s, Args... args) {

@@ -1,25 +1,29 @@
 // mood_cluster.cuh -- the short parts of a forward-Euler stage, one thread-
 // block cluster per instance (included by kernels.cu): pass 1's face cascade
-// (k_mood_faces) and, after the dense pass-1 update, every later MOOD pass
+// (k_mood_faces) and, after the dense pass-1 update, the later MOOD passes
 // (k_mood_passes; timeStep.f90:86-128).
 //
-// What bounds them: nothing but latency.  A later pass of a small solve
-// touches a few hundred cells; as a chain of grid-wide kernels it cost nine
-// launches (and four per cascade iteration) of 3-20 us each.  Here a pass is four
-// phases between hardware cluster barriers, and each item is split over
-// lanes so that a lane's chain is short: a cell's face states over 32 lanes
-// (4 faces x 8 variables: 13 loads at R = 2 instead of 104), a face's fluxes
-// over 8 lanes, an updated cell over 8 (its variables), a lowered cell's
-// flags over 13 (its diamond).  The lists are per instance (segments of the
-// batch's lists that start at the instance's first tile), and hold cell
+// What bounds them: latency.  A later pass of a small solve touches a few
+// hundred cells; as a chain of grid-wide kernels it cost nine launches (and
+// four per cascade iteration) of 3-20 us each, 75 us in all.  Here a pass is
+// two phases between hardware cluster barriers (0.6 us each) -- reconstruct,
+// test and solve the listed faces; update, detect and flag the listed cells --
+// of three or four dependent L2 accesses (0.45 us each), one or two atomics
+// and one Riemann solve (2.5 us alone on its scheduler): 13 us for a 64^2
+// blast's 200 faces and 150 cells, 19 us for a 128^2 Orszag-Tang's 900 and 640.
+// Each item is split over lanes so that a lane's chain is short: a cell's face
+// states over 32 lanes (4 faces x 8 variables: 13 loads at R = 2 instead of
+// 104), a face's over 8, an updated cell over 8 (its variables), a lowered
+// cell's flags over 13 (its diamond).  The lists are per instance (segments of
+// the batch's lists that start at the instance's first tile), and hold cell
 // indices; a flag's first setter appends its cell, so nothing scans the grid.
 // Orders differ from the chain's, values do not: every list is a set, and
 // each item's arithmetic is the chain's, statement by statement.
 //
 // Flags: a pass reads recompute / recomputeFLICD in one pair of planes (rec,
 // recF or recB, recFB) and its flag rebuild sets the other, so the old flags
-// are cleared in the same phase.  Between stages all of them, nextPass, fail,
-// lowered and DM_CASC are zero, and so are the counters.
+// are cleared beside the next pass's first phase.  Between stages all of them,
+// nextPass, fail, lowered and DM_CASC are zero, and so are the counters.
 //
 // Every branch around a barrier is taken on values all blocks of the cluster
 // read alike: a counter is changed only in phases a barrier away from its
