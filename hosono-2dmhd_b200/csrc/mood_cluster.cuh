@@ -647,8 +647,10 @@ __device__ __forceinline__ void mc_setup(const Batch& B, int k, int uin, int uou
         m.recF[1] = face + cells;
         m.face = face + 2 * cells;
         m.next = reinterpret_cast<int*>(B.L.next + seg);
-        m.rec[0] = reinterpret_cast<int*>(B.L.rec + seg);
-        m.rec[1] = reinterpret_cast<int*>(B.L.rec2 + seg);
+        // both recompute lists in the batch's free one: the other holds the chain's
+        // cells for its next pass when instances are handed over
+        m.rec[0] = reinterpret_cast<int*>(rec_list(B, true) + seg);
+        m.rec[1] = m.rec[0] + cells;
         m.recF[0] = reinterpret_cast<int*>(B.L.recF + seg);
         m.low = reinterpret_cast<int*>(B.L.low + seg);
         m.casc = reinterpret_cast<int*>(B.L.casc + seg);

@@ -82,6 +82,34 @@ def test_cluster_and_chain_share_a_batch(tmp_par_dir):
     b.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", [0, 1, 2])
+def test_handed_over_instances_beside_the_chain(first, tmp_par_dir):
+    """Blasts whose long passes end at different passes of a stage: the clusters
+    take one over, at the front, in the middle and at the back of the batch's
+    lists, while the chain still holds the others' recompute list."""
+    m = pkg.load()
+    kvs = [parfiles.blast(200, 2, p_ratio=1000.0, theta=0.7), parfiles.blast(400, 3, p_ratio=1000.0, theta=0.4),
+           parfiles.blast(300, 1, p_ratio=300.0, theta=1.1)]
+    kvs = kvs[first:] + kvs[:first] + [parfiles.orszag_tang(40, 1)]
+    pars = [parfiles.make(tmp_par_dir, f"hand{i}", kv) for i, kv in enumerate(kvs)]
+    b = m.Batch(len(pars), sum(m.Batch.tiles_for(m.par_load(p)[0]) for p in pars), fp_mode=m.FP_STRICT)
+    slots = [b.add_par(p) for p in pars]
+    for k in slots:
+        b.set_time(k, 0.0, 1e30)
+    b.run(max_steps=6)
+    for k, p in zip(slots, pars):
+        o = oracle.Oracle(p)
+        for _ in range(6):
+            o.advance(o.cfl())
+        U, V, S = b.download(k)
+        np.testing.assert_array_equal(U, o.U())
+        np.testing.assert_array_equal(V, o.V())
+        np.testing.assert_array_equal(S, o.scheme())
+        o.close()
+    b.close()
+
+
 def _wrap(U, g, periodic):
     """Guard cells from the interior (boundaryConditions_applyBlk)."""
     inner = U[g:-g, g:-g]
