@@ -441,6 +441,7 @@ int Engine::autotune(int trials, bool force, hosono_tune_report* rep) {
         }
     }
     K_->tune_mark(batch(), 0, s_);
+    cudaMemsetAsync(d_flags_->p1Next, 0, sizeof d_flags_->p1Next, s_);  // as a stage leaves them
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     tune_ = saved;

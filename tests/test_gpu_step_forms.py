@@ -110,6 +110,27 @@ def test_handed_over_instances_beside_the_chain(first, tmp_par_dir):
     b.close()
 
 
+@pytest.mark.gpu
+def test_step_after_autotune(tmp_par_dir):
+    """The timing launches leave pass 1's tile counters at their start for a
+    step with the caller's dt."""
+    m = pkg.load()
+    par = parfiles.make(tmp_par_dir, "tuned", parfiles.orszag_tang(96, 2))
+    s = m.Solver.from_par(par)
+    o = oracle.Oracle(par)
+    default = s.tuning()
+    s.autotune(trials=1, force=True)
+    s.set_tuning(**default)
+    dt = o.cfl()
+    s.timeStep_advanceSolution(dt)
+    o.advance(dt)
+    U, V, S = s.download()
+    np.testing.assert_array_equal(U, o.U())
+    np.testing.assert_array_equal(S, o.scheme())
+    s.close()
+    o.close()
+
+
 def _wrap(U, g, periodic):
     """Guard cells from the interior (boundaryConditions_applyBlk)."""
     inner = U[g:-g, g:-g]
