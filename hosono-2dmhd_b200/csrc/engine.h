@@ -97,7 +97,7 @@ struct InstState {
     int cFail;       // cells that failed CAD/PAD in pass 1 (its list of them)
     int cLow;        // lowered cells of the pass at which it did
     int nCasc;       // cells on the cluster form's cascade-lowered list
-    int mc[10];      // the cluster form's list counters (mood_cluster.cuh MC_*)
+    int mc[12];      // the cluster form's list counters (mood_cluster.cuh MC_*)
     int nInner, nDetect;  // lowerings in the current pass
     int lastInner, lastDetect;  // lowerings of the last finished pass
     int passes;      // MOOD passes in the current stage

@@ -27,12 +27,24 @@
 //
 // Every branch around a barrier is taken on values all blocks of the cluster
 // read alike: a counter is changed only in phases a barrier away from its
-// last read.
+// last read, and started over only in phases a barrier away from its next
+// addition, so counters come in pairs that the passes (cascade iterations)
+// take in turn.  With cur a pass's half, and its phases flux (reconstruct, test,
+// solve), then, if cells failed, the cascade's, then update, a barrier after
+// each:
+//   counter          added to in               read in               back to 0 in
+//   LOW[cur]         update                    next flux             next update
+//   REC, RECF[cur]   update before, cascade    flux, update          next flux
+//   FACE[cur]        update before, cascade    flux, cascade         next flux; cascade, a barrier before its own
+//   nCasc            cascade                   update                next flux
+//   FAIL, NEXT[it]   flux or iteration it - 1  iteration it          iteration it, a barrier after its read
+// (where the lowered cells are listed, their flags are set in a phase of their
+// own after update, with a barrier to flux).
 #pragma once
 
 constexpr int MC_THREADS = 512, MC_WARPS = MC_THREADS / 32;
-enum : int { MC_FAIL = 0, MC_NEXT = 2, MC_REC = 4, MC_RECF = 6, MC_FACE = 8 };  // InstState::mc, two of each
-constexpr int MC_N = 10;                  // counters
+enum : int { MC_FAIL = 0, MC_NEXT = 2, MC_REC = 4, MC_RECF = 6, MC_FACE = 8, MC_LOW = 10 };  // InstState::mc, two of each
+constexpr int MC_N = 12;                  // counters
 constexpr int MC_FS = 72;                 // doubles per face of a warp's exchange buffer (64 + 8 against bank conflicts)
 constexpr int MC_BUF = 4 * MC_FS;         // a warp's exchange buffer
 constexpr int MC_PV = 25 * 4 * 4 * 3;     // prediction vectors of the largest radius
@@ -549,7 +561,7 @@ __device__ __forceinline__ void mc_update(Mc& m, const McT& t, const int* list, 
         }
         if (flags) {
             unsigned lows = __ballot_sync(0xffffffffu, low);
-            if (lows && t.lane == 0) atomicAdd(&m.S->nDetect, __popc(lows));
+            if (lows && t.lane == 0) atomicAdd(&m.S->mc[MC_LOW + cur], __popc(lows));
             while (lows) {  // the warp takes its lowered cells in turn
                 const int src = __ffs(lows) - 1;
                 lows &= lows - 1;
@@ -562,7 +574,7 @@ __device__ __forceinline__ void mc_update(Mc& m, const McT& t, const int* list, 
             }
         } else {
             if (low) d.lowered[c] = 1;
-            mc_append(m.low, &m.S->nDetect, low, c, t.lane);
+            mc_append(m.low, &m.S->mc[MC_LOW + cur], low, c, t.lane);
         }
     }
 }
@@ -790,10 +802,9 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
                         break;
                     }
                     capped = passes >= cap;
-                    if (listed) {
-                        cluster_sync();
+                    if (listed || capped) cluster_sync();  // capped: every block has read nLow
+                    if (listed)
                         for (int e = t.gw * 32 + t.lane; e < nLow; e += t.nw * 32) m.d.lowered[m.low[e]] = 0;
-                    }
                     if (capped) break;  // (the next stage's pass 1 clears the flag planes)
                     // the old flags, and the counters every block has read a
                     // barrier ago, start over
@@ -811,7 +822,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
                     mc_flux<true>(m, t, mc_ld(&S.mc[MC_FACE + cur]), cur);
                     cluster_sync();
                     const int nFail = mc_ld(&S.mc[MC_FAIL]);
-                    if (lead) S.nDetect = 0;  // nLow was read before this barrier
+                    if (lead) S.mc[MC_LOW + (cur ^ 1)] = 0;  // nLow was read before this barrier
                     inner = 0;
                     if (nFail > 0) {
                         const int2 r = mc_cascade_later(&m, t, nFail, cur);
@@ -824,7 +835,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
                     listed = nCasc > 0;
                     mc_update(m, t, m.recF[cur], nRecF, cur, !listed);
                     cluster_sync();
-                    nLow = mc_ld(&S.nDetect);
+                    nLow = mc_ld(&S.mc[MC_LOW + cur]);
                     passes++;
                     lastInner = inner;
                     lastDetect = nLow;
