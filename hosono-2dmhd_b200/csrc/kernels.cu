@@ -300,7 +300,9 @@ __device__ __forceinline__ void p1_release(P1Ctl* ctl) {
     if (atomicAdd(&ctl->released, 1) == NTHREADS - 1) p1_refill<R>(ctl);
 }
 
-// one face (both sides, every quadrature point); returns the side verdict bits.
+// one face (both sides, every quadrature point); returns the side verdict bits
+// (1 left, 2 right; P1_REST: the columns of the variables the mode leaves out
+// hold fluxes too, as an IEEE solve of a point gave them).
 // Points go in pairs: one sweep of GP sums gives both, the second's states wait
 // in this thread's column of shared memory (park[k * NTHREADS]) while the first
 // is solved.  The Gauss sum of the fluxes accumulates in another column
@@ -308,6 +310,14 @@ __device__ __forceinline__ void p1_release(P1Ctl* ctl) {
 // needs.  dir is a run-time value: the kernel holds one copy of the Riemann
 // solver for both face directions, which halves its instruction footprint; the
 // solver works in face coordinates, so only plane offsets depend on it.
+constexpr uint8_t P1_REST = 4;
+template <int MODE>  // their fluxes to the planes (rare: kept out of line)
+static __device__ __noinline__ void pass1_rest(double* Fo, long long sw, long long plane, double* ct, const double* acc) {
+    for (int v = 0; v < NCONS; v++)
+        if (!Solve<MODE>::var(v))
+            Fo[v * plane + (v == MOMN || v == MAGN ? sw : v == MOMT || v == MAGT ? -sw : 0)] = acc[v * NTHREADS];
+    if (!Solve<MODE>::var(MAGT)) *ct = acc[MAGT * NTHREADS];
+}
 template <int R, int MODE>
 __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __restrict__ sU,
                                               const double* __restrict__ sPv, int sx, int sy, int dir, bool needL,
@@ -363,7 +373,14 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
             bool admL = true, admR = true;
             if (doFlux) {  // in the flux range both sides are reconstructed
                 double F[NCONS];
-                face_flux<MODE>(P, uL, uR, F, admL, admR);
+                face_flux<MODE>(P, uL, uR, F, admL, admR, [&](const Cons8& f) {
+                    const double w = qw_at(d, R, q);
+                    for (int v = 0; v < NCONS; v++) {
+                        if (S::var(v)) continue;
+                        acc[v * NTHREADS] = (bits & P1_REST ? acc[v * NTHREADS] : 0.0) + w * f.v[v];
+                    }
+                    if (S::LEFT) bits |= P1_REST;
+                });
                 const double w = qw_at(d, R, q);
 #pragma unroll
                 for (int v = 0; v < NCONS; v++)
@@ -394,6 +411,7 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
             Fo[o] = S::var(v) ? acc[v * NTHREADS] : 0.0;
         }
         (x ? d.CTX : d.CTY)[c] = S::var(MAGT) ? acc[MAGT * NTHREADS] : 0.0;
+        if (S::LEFT && (bits & P1_REST)) pass1_rest<MODE>(Fo, sw, G.plane, (x ? d.CTX : d.CTY) + c, acc);
     }
     return bits;
 }

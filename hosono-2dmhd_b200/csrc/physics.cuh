@@ -346,6 +346,7 @@ struct Solve {
     static constexpr bool H = MODE >= SOLVE_HYDRO;            // hydro: no field
     static constexpr bool Z = (MODE & 1) == 0;                // out-of-plane momentum
     static constexpr bool BZ = MODE == SOLVE_MHD;             // out-of-plane field
+    static constexpr bool LEFT = MODE != SOLVE_MHD && MODE != SOLVE_HYDRO_FIELD;  // it leaves some out
     static constexpr __host__ __device__ bool var(int v) {   // state variables it reads
         return MODE == SOLVE_HYDRO_FIELD || v < 3 || v == ENER || (v == MOMZ_ && Z) || (!H && (v == MAGN || v == MAGT)) || (BZ && v == MAGZ_);
     }
@@ -531,10 +532,12 @@ __device__ __forceinline__ bool state_adm(const Phys& s, const double* u) {
     for (int v = 0; v < NCONS; v++) U[v] = Solve<MODE>::var(v) ? u[v] : 0.0;
     return admissible(U[DENS], cons2pres<Solve<MODE>::H ? 1 : 0>(s, U));
 }
-// a mode's solve, the IEEE form where it has to be
-template <int MODE>
+// a mode's solve, the IEEE form where it has to be; that form's eight fluxes go
+// to `all`, for a left-out variable's flux is NaN where a speed or a product of
+// the solve is infinite (zero times infinity, zero by zero)
+template <int MODE, class All>
 __device__ __forceinline__ void face_flux(const Phys& s, const double* uL, const double* uR, double* F, bool& admL,
-                                          bool& admR) {
+                                          bool& admR, All&& all) {
     bool done = false;
     if (MODE != SOLVE_HYDRO_FIELD) done = face_solve<MODE>(s, uL, uR, F, admL, admR);
     if (!done) {
@@ -548,6 +551,7 @@ __device__ __forceinline__ void face_flux(const Phys& s, const double* uL, const
 #pragma unroll
         for (int v = 0; v < NCONS; v++)
             if (Solve<MODE>::var(v)) F[v] = f.v[v];
+        all(f);
         admL = state_adm<MODE>(s, uL);
         admR = state_adm<MODE>(s, uR);
     }
@@ -558,19 +562,24 @@ __device__ __forceinline__ bool bits_zero(double a) {
 // in face coordinates, hydro flag at run time; admL, admR: CAD and PAD of the sides
 __device__ __forceinline__ void hllc_face(const Phys& s, const double* uL, const double* uR, double* F, bool& admL,
                                           bool& admR) {
+    auto whole = [](const Cons8&) {};  // the mode's own variables are all there are
     if (!s.force_hydro) {
-        face_flux<SOLVE_MHD>(s, uL, uR, F, admL, admR);
+        face_flux<SOLVE_MHD>(s, uL, uR, F, admL, admR, whole);
         return;
     }
     bool field = false;
 #pragma unroll
     for (int v = MAGN; v <= MAGZ_; v++) field = field || !bits_zero(uL[v]) || !bits_zero(uR[v]);
     if (field) {
-        face_flux<SOLVE_HYDRO_FIELD>(s, uL, uR, F, admL, admR);
+        face_flux<SOLVE_HYDRO_FIELD>(s, uL, uR, F, admL, admR, whole);
         return;
     }
-    face_flux<SOLVE_HYDRO>(s, uL, uR, F, admL, admR);
     F[MAGN] = F[MAGT] = F[MAGZ_] = 0.0;
+    face_flux<SOLVE_HYDRO>(s, uL, uR, F, admL, admR, [&](const Cons8& f) {
+        F[MAGN] = f.v[MAGN];
+        F[MAGT] = f.v[MAGT];
+        F[MAGZ_] = f.v[MAGZ_];
+    });
 }
 // in grid coordinates: a y-face exchanges x and y on the way in and out
 __device__ __forceinline__ void hllc(const Phys& s, const double* uL, const double* uR, int dir, double* flux) {
