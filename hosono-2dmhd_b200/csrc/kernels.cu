@@ -1255,6 +1255,11 @@ __device__ __forceinline__ bool detect_cell_at(const Phys& P, const uint8_t* mas
     return detect_decide(P, m, d, n);
 }
 
+// x in [2^-900, 2^900), from the exponent (integer pipes)
+__device__ __forceinline__ bool mid_range(double x) {
+    return (unsigned)__double2hiint(x) - ((1023u - 900u) << 20) < (1800u << 20);
+}
+
 // Per-stage part of detect_ALL on the interior, evaluated once per stage by
 // the pass-1 update kernel (it reads only the stage input U).  The primitive
 // variables of the tile and a one-cell halo are computed once into shared
@@ -1298,12 +1303,14 @@ __device__ __forceinline__ void detect_prep_tile_t(const InstDev& d, const Cell 
     const double dx = G.dx, dy = G.dy;
     // the pressure sensor first: it is off in all but a few cells, and seen to
     // be off without its two divisions when the sum of the two ratios is
-    // below its threshold by more than rounding (a margin of 2^-40)
+    // below its threshold by more than rounding (a margin of 2^-40), with the
+    // products far from overflow and underflow
     const double pE = spr[e + 1], pW = spr[e - 1], pN = spr[e + DP_SX], pS = spr[e - DP_SX];
     const double ax = fabs(pE - pW), ay = fabs(pN - pS), mx = fmin(pE, pW), my = fmin(pN, pS);
     const double thr = 10.0 * G.maxdxdy;
+    const double tp = thr * (mx * my);  // in the middle, and with it mx * my where dx is below 2^60
     bool shock1 = false, shock2 = false, shock3 = false;
-    if (!((ax * my + ay * mx) * (1.0 + 0x1p-40) < thr * (mx * my))) {
+    if (!((ax * my + ay * mx) * (1.0 + 0x1p-40) < tp) | !mid_range(tp) | !(G.maxdxdy < 0x1p60)) {
         double div_vel = (svx[e + 1] - svx[e - 1]) / (2 * dx);
         div_vel = div_vel + (svy[e + DP_SX] - svy[e - DP_SX]) / (2 * dy);
         shock1 = div_vel < -(1.0 * (G.maxdxdy * G.maxdxdy));

@@ -91,3 +91,26 @@ def test_riemann_non_finite(hydro, tmp_par_dir):
         np.testing.assert_array_equal(F.cpu().numpy(), ref)
     s.close()
     o.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1.0, 1e140, 1e153])
+def test_pressure_sensor_range(scale, tmp_par_dir):
+    """detect's pressure sensor where the products of two pressures leave the
+    range of 64 bits (1e153) and where they do not: a noisy converging flow,
+    every value of it scaled alike."""
+    def edit(U):
+        rng = np.random.default_rng(3)
+        n = U.shape[0]
+        rho, p = rng.uniform(0.8, 1.2, (n, n)), 14.0 * rng.uniform(0.7, 1.3, (n, n))
+        x = (np.arange(n) + 0.5) / n - 0.5
+        vx, vy = -2.5 * np.sign(x)[None, :] * rng.uniform(0.5, 1.0, (n, n)), -2.5 * np.sin(6 * x)[:, None] + 0 * rho
+        U[...] = 0.0
+        U[..., 0], U[..., 1], U[..., 2] = rho, rho * vx, rho * vy
+        U[..., 4] = p / 0.4 + 0.5 * rho * (vx * vx + vy * vy)
+        U *= scale
+    o, s = _pair(tmp_par_dir, f"sensor{scale}", parfiles.sedov(40, 2), edit)
+    _step_alike(o, s, 1e-3, steps=2)
+    assert (o.scheme() < 2).sum() > 100
+    s.close()
+    o.close()
