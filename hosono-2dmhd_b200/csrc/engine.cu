@@ -232,6 +232,9 @@ int Engine::init(int max_inst, int max_tiles, int fp_mode) {
     maxInst_ = max_inst;
     maxTiles_ = max_tiles;
     K_ = fp_mode == HOSONO_FP_FAST ? kernelset_fast() : kernelset_strict();
+    int device = 0;
+    CUE(cudaGetDevice(&device));
+    CUE(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
     CUE(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
     CUE(cudaMalloc(&d_dev_, sizeof(InstDev) * maxInst_));
     CUE(cudaMalloc(&d_st_, sizeof(InstState) * maxInst_));
@@ -474,6 +477,7 @@ Batch Engine::batch() const {
     B.p1End = INT_MAX;
     B.p1Init = 1;
     B.mcMax = trace || tune_.later_passes == HOSONO_LATER_PERSISTENT ? -1 : kClusterCells;
+    B.mcBlocks = mcBlocks_;
     B.ctStaged = tune_.update_staging == HOSONO_STAGE_TMA ? 1 : 0;
     B.dev = d_dev_;
     B.st = d_st_;
@@ -548,6 +552,14 @@ int Engine::upload_tables() {
     // the graphs launch pass 1 for the radii held when they were recorded:
     // a new radius needs new graphs
     if (radii_ & ~graphRadii_) drop_graphs();
+    // ... and so does another cluster size; a larger one waits until it would
+    // hold at twice the instances, so that a server's few admissions and
+    // retirements do not record graphs again and again
+    const int live = live_count(), want = cluster_blocks_for(live, sms_);
+    if (want < mcBlocks_ || cluster_blocks_for(2 * live, sms_) > mcBlocks_) {
+        mcBlocks_ = want;
+        drop_graphs();
+    }
     return HOSONO_OK;
 }
 

@@ -165,6 +165,7 @@ struct Batch {
     int ctStaged;        // the pass-1 update reads TMA-staged boxes (1) or the planes (0)
     int p1Init;          // pass 1 also resets the stage's MOOD planes (0: the autotuner's timing launches)
     int mcMax;           // most listed cells the cluster kernels take per instance (-1: everything to the chain)
+    int mcBlocks;        // blocks of an instance's cluster where 16 are not taken
     int maxTiles;        // capacity of the tile list
     int maxInst;         // capacity (slots)
     const int2* instTiles;  // per slot: first tile in the tile list, tile count (0: not live)

@@ -1602,13 +1602,15 @@ __device__ __forceinline__ void d_clear_low(const Batch& B, int gt, int gs) {
     }
 }
 __global__ void __launch_bounds__(256) k_clear_low(Batch B) { PDL_ENTRY(); d_clear_low(B, GT1, GS1); }
-// the same after pass 1, whose lowered cells are listed per instance
-__global__ void __launch_bounds__(256) k_clear_low_pass1(Batch B) { PDL_ENTRY();
-    for (int k = 0; k < B.maxInst; k++) {
+// the same after pass 1, whose lowered cells are listed per instance: a tile
+// takes as many entries of its instance's list as it has cells
+__global__ void __launch_bounds__(NTHREADS) k_clear_low_pass1(Batch B) { PDL_ENTRY();
+    FOR_TILES(B, t) {
+        const int k = B.tiles[t].x;
         const InstState& S = B.st[k];
         if (!(S.stepping && S.stageActive)) continue;
-        const int* list = reinterpret_cast<const int*>(B.L.low + (long long)B.instTiles[k].x * (TILE_X * TILE_Y));
-        for (int e = GT1; e < S.nDetect; e += GS1) B.dev[k].lowered[list[e]] = 0;
+        const int first = B.instTiles[k].x, e = (t - first) * NTHREADS + (int)(threadIdx.y * TILE_X + threadIdx.x);
+        if (e < S.nDetect) B.dev[k].lowered[reinterpret_cast<const int*>(B.L.low + (long long)first * NTHREADS)[e]] = 0;
     }
 }
 
@@ -2398,7 +2400,8 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
     if (B.p1Radii & (1 << 3)) launch_pass1<3>(B, uin, s);
 }
 // One cluster per instance slot: 16 blocks (a non-portable size, taken where
-// the GPU can place one) for up to nine slots, which fills the GPU, else 8.
+// the GPU can place one) for up to nine slots, which fills the GPU, else what
+// the engine chose for its live instances (kClusterCells in engine_host.h).
 // The shared memory a cluster kernel needs is static; 16 blocks take leave.
 template <typename K>
 bool cluster_sixteen(K kernel) {
@@ -2423,7 +2426,7 @@ bool cluster_sixteen(K kernel) {
     return n >= 1;
 }
 template <typename K>
-int cluster_blocks(K kernel, int maxInst) {
+int cluster_blocks(K kernel, const Batch& B) {
     // asked once per device and kernel (the leave is the device's), under a lock
     // (engines on several host threads)
     static std::mutex mu;
@@ -2434,7 +2437,7 @@ int cluster_blocks(K kernel, int maxInst) {
     const auto key = std::make_pair(dev, (const void*)kernel);
     auto it = known.find(key);
     if (it == known.end()) it = known.emplace(key, cluster_sixteen(kernel)).first;
-    return it->second && maxInst <= 9 ? 16 : 8;
+    return it->second && B.maxInst <= 9 ? 16 : B.mcBlocks;
 }
 template <typename... KArgs, typename... Args>
 void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t s, Args... args) {
@@ -2452,13 +2455,13 @@ void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t
     cudaLaunchKernelEx(&cfg, kern, B, args...);
 }
 void l_mood_faces(const Batch& B, int uin, cudaGraphConditionalHandle h, cudaStream_t s) {
-    lk_cluster(k_mood_faces, cluster_blocks(k_mood_faces, B.maxInst), B, s, uin, h, (int)(h != 0));
+    lk_cluster(k_mood_faces, cluster_blocks(k_mood_faces, B), B, s, uin, h, (int)(h != 0));
 }
 void l_mood_passes(const Batch& B, int uin, int uout, cudaGraphConditionalHandle h, cudaStream_t s) {
-    lk_cluster(k_mood_passes<false>, cluster_blocks(k_mood_passes<false>, B.maxInst), B, s, uin, uout, h, (int)(h != 0));
+    lk_cluster(k_mood_passes<false>, cluster_blocks(k_mood_passes<false>, B), B, s, uin, uout, h, (int)(h != 0));
 }
 void l_mood_passes_rest(const Batch& B, int uin, int uout, cudaStream_t s) {
-    lk_cluster(k_mood_passes<true>, cluster_blocks(k_mood_passes<true>, B.maxInst), B, s, uin, uout,
+    lk_cluster(k_mood_passes<true>, cluster_blocks(k_mood_passes<true>, B), B, s, uin, uout,
                (cudaGraphConditionalHandle)0, 0);
 }
 void l_handover(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_handover, B, s); }
@@ -2501,7 +2504,7 @@ void l_recon_list(const Batch& B, int uin, cudaStream_t s) { LIST_LAUNCH(k_recon
 void l_flux_list(const Batch& B, int uin, cudaStream_t s) { LIST_LAUNCH(k_flux_list, B, s, uin); }
 void l_ct_list(const Batch& B, int uin, int uout, cudaStream_t s) { LIST_LAUNCH(k_ct_list, B, s, uin, uout); }
 void l_clear_low(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low, B, s); }
-void l_clear_low_pass1(const Batch& B, cudaStream_t s) { LIST_LAUNCH(k_clear_low_pass1, B, s); }
+void l_clear_low_pass1(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_clear_low_pass1, B, s); }
 void l_bc_fill(const Batch& B, int role, cudaStream_t s) { TILE_LAUNCH(k_bc_fill, B, s, role); }
 void l_rk_combine2(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_rk_combine2, B, s); }
 void l_rk_final(const Batch& B, int cfl, cudaStream_t s) {

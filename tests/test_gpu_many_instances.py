@@ -1,0 +1,80 @@
+"""Batches of more instances than clusters fit the GPU at once: the cluster
+size follows the live instances, each instance bit for bit its own solve."""
+import statistics
+import time
+
+import numpy as np
+import pytest
+
+import oracle
+import parfiles
+import pkg
+
+
+def _problem(k):
+    n, radius = 24 + 6 * (k % 4), 1 + k % 3
+    return [parfiles.blast(n, radius, p_ratio=50.0 + 90 * (k % 7), theta=0.1 * (k % 11)), parfiles.orszag_tang(n, radius),
+            parfiles.sedov(n, radius)][(k // 3) % 3]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [17, 20, 40, 90])
+def test_cluster_size_follows_the_instances(count, tmp_par_dir):
+    """A step of `count` instances, a step of the eighth that stays, then one
+    beside as many new ones: each kind of graph is recorded anew in between."""
+    m = pkg.load()
+    pars = [parfiles.make(tmp_par_dir, f"many{k}", _problem(k)) for k in range(count)]
+    tiles = sum(m.Batch.tiles_for(m.par_load(p)[0]) for p in pars)
+    b = m.Batch(count, tiles, fp_mode=m.FP_STRICT)
+    held = {}
+
+    def add(p):
+        k = b.add_par(p)
+        b.set_time(k, 0.0, 1e30)
+        held[k] = oracle.Oracle(p)
+
+    def step():
+        b.run(max_steps=1)
+        for k, o in held.items():
+            o.advance(o.cfl())
+            U, V, S = b.download(k)
+            np.testing.assert_array_equal(U, o.U())
+            np.testing.assert_array_equal(V, o.V())
+            np.testing.assert_array_equal(S, o.scheme())
+    for p in pars:
+        add(p)
+    step()
+    for k in list(held)[count // 8:]:
+        b.remove(k)
+        held.pop(k).close()
+    step()
+    for p in pars[count // 8:]:
+        add(p)
+    step()
+    for o in held.values():
+        o.close()
+    b.close()
+
+
+@pytest.mark.gpu
+def test_many_small_instances_share_the_gpu(tmp_par_dir):
+    """256 small blasts take well under 256 / 36 times as long as 36: with a
+    cluster of eight blocks for each of them it was 5.9 times, with the sizes
+    the instances ask for 4.3."""
+    m = pkg.load()
+    pars = [parfiles.make(tmp_par_dir, f"small{k}", parfiles.blast(40 + 4 * (k % 5), 2, p_ratio=50.0 + 100 * (k % 7),
+                                                                   theta=0.02 * k)) for k in range(35)]
+
+    def per_step(count):
+        b = m.Batch(count, sum(m.Batch.tiles_for(m.par_load(pars[k % 35])[0]) for k in range(count)))
+        slots = [b.add_par(pars[k % 35]) for k in range(count)]
+        times = []
+        for _ in range(5):
+            for s in slots:
+                b.set_time(s, 0.0, 1e30)
+            t = time.perf_counter()
+            b.run(max_steps=8)
+            times.append(time.perf_counter() - t)
+        b.close()
+        return statistics.median(times[1:])
+    assert per_step(256) < 5.0 * per_step(36)
