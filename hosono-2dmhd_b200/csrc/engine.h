@@ -267,7 +267,8 @@ struct KernelSet {
     void (*mood_rest)(const Batch&, int uin, int uout, cudaStream_t);
     // grids the launchers use: the pass-1 kernel of radius R, and the
     // largest grid of the other per-tile kernels (each capped at maxTiles)
-    void (*launch_info)(int R, int maxTiles, int* pass1_grid, int* tile_grid_max);
+    // grids of the batch's launch choices: pass 1 at radius R, the largest other tile kernel
+    void (*launch_info)(const Batch&, int R, int* pass1_grid, int* tile_grid_max);
     const ModuleOps* mod;
 };
 

@@ -106,8 +106,8 @@ class Engine {
     int riemann(int slot, int n, const double* uL, const double* uR, int dir, double* F);
     int eigenvecs(int slot, int n, const double* V, int dir, int cons, double* L, double* R);
 
-    // launch geometry of the kernels for radius R over this engine's tile capacity
-    void launch_info(int R, int* pass1_grid, int* tile_grid_max) const { K_->launch_info(R, maxTiles_, pass1_grid, tile_grid_max); }
+    // launch geometry of the kernels for radius R over this engine's tile capacity, as it is tuned now
+    void launch_info(int R, int* pass1_grid, int* tile_grid_max) const { K_->launch_info(batch(), R, pass1_grid, tile_grid_max); }
     int live_count() const;
     size_t instance_bytes(const hosono_params& p) const;
     const hosono_params& params(int slot) const { return slots_[slot].p; }

@@ -2358,46 +2358,31 @@ void launch_pass1_v(const Batch& B, int uin, cudaStream_t s) {
     lk(k_face_pass1<R, TMA, DYN, MINB, NBUF>, dim3((unsigned)pass1_grid<R, TMA, DYN, MINB, NBUF>(B.maxTiles)), kTile,
        (size_t)pass1_smem<R, NBUF>(), s, B, uin);
 }
-template <int R, int MINB, int NBUF>
-void launch_pass1_s(const Batch& B, int uin, cudaStream_t s) {  // staging and schedule
-    if (B.p1Tma) {
-        if (B.p1Dyn)
-            launch_pass1_v<R, true, true, MINB, NBUF>(B, uin, s);
-        else
-            launch_pass1_v<R, true, false, MINB, NBUF>(B, uin, s);
-    } else {
-        if (B.p1Dyn)
-            launch_pass1_v<R, false, true, MINB, NBUF>(B, uin, s);
-        else
-            launch_pass1_v<R, false, false, MINB, NBUF>(B, uin, s);
-    }
-}
 // the variant the tuning asks for: TMA staging and two boxes only with two
 // blocks per SM
+struct P1Form {
+    int (*grid)(int maxTiles);
+    void (*launch)(const Batch&, int uin, cudaStream_t);
+};
+template <int R, bool TMA, int MINB, int NBUF>
+P1Form pass1_form_v(bool dyn) {
+    return dyn ? P1Form{pass1_grid<R, TMA, true, MINB, NBUF>, launch_pass1_v<R, TMA, true, MINB, NBUF>}
+               : P1Form{pass1_grid<R, TMA, false, MINB, NBUF>, launch_pass1_v<R, TMA, false, MINB, NBUF>};
+}
 template <int R>
-void launch_pass1(const Batch& B, int uin, cudaStream_t s) {
-    if (B.p1Blocks == 3) {
-        if (B.p1Dyn)
-            launch_pass1_v<R, false, true, 3, 1>(B, uin, s);
-        else
-            launch_pass1_v<R, false, false, 3, 1>(B, uin, s);
-    } else if (B.p1Blocks == 4) {
-        if (B.p1Dyn)
-            launch_pass1_v<R, false, true, 4, 1>(B, uin, s);
-        else
-            launch_pass1_v<R, false, false, 4, 1>(B, uin, s);
-    } else if (B.p1Boxes == 1) {
-        launch_pass1_s<R, 2, 1>(B, uin, s);
-    } else {
-        launch_pass1_s<R, 2, 2>(B, uin, s);
-    }
+P1Form pass1_form(const Batch& B) {
+    const bool dyn = B.p1Dyn != 0;
+    if (B.p1Blocks == 3) return pass1_form_v<R, false, 3, 1>(dyn);
+    if (B.p1Blocks == 4) return pass1_form_v<R, false, 4, 1>(dyn);
+    if (B.p1Boxes == 1) return B.p1Tma ? pass1_form_v<R, true, 2, 1>(dyn) : pass1_form_v<R, false, 2, 1>(dyn);
+    return B.p1Tma ? pass1_form_v<R, true, 2, 2>(dyn) : pass1_form_v<R, false, 2, 2>(dyn);
 }
 // one launch per radius held (the kernels also skip radii the device's
 // tile list does not hold)
 void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
-    if (B.p1Radii & (1 << 2)) launch_pass1<2>(B, uin, s);
-    if (B.p1Radii & (1 << 1)) launch_pass1<1>(B, uin, s);
-    if (B.p1Radii & (1 << 3)) launch_pass1<3>(B, uin, s);
+    if (B.p1Radii & (1 << 2)) pass1_form<2>(B).launch(B, uin, s);
+    if (B.p1Radii & (1 << 1)) pass1_form<1>(B).launch(B, uin, s);
+    if (B.p1Radii & (1 << 3)) pass1_form<3>(B).launch(B, uin, s);
 }
 // One cluster per instance slot: 16 blocks (a non-portable size, taken where
 // the GPU can place one) for up to nine slots, which fills the GPU, else what
@@ -2531,10 +2516,9 @@ void l_mood_rest(const Batch& B, int uin, int uout, cudaStream_t s) {
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_mood_rest, B, uin, uout);
 }
-void l_launch_info(int R, int maxTiles, int* pass1, int* tile_grid_max) {
-    *pass1 = R == 1   ? pass1_grid<1, false, false, 2, 2>(maxTiles)
-             : R == 2 ? pass1_grid<2, false, false, 2, 2>(maxTiles)
-                      : pass1_grid<3, false, false, 2, 2>(maxTiles);
+void l_launch_info(const Batch& B, int R, int* pass1, int* tile_grid_max) {
+    const int maxTiles = B.maxTiles;
+    *pass1 = (R == 1 ? pass1_form<1>(B) : R == 2 ? pass1_form<2>(B) : pass1_form<3>(B)).grid(maxTiles);
     const void* tile_kernels[] = {(const void*)k_cfl_reduce,     (const void*)k_cascade_lower,
                                    (const void*)k_compact_next, (const void*)k_compact_post,
                                   (const void*)k_compact_dirty,  (const void*)k_ct_update_detect, (const void*)k_mood_flags,
