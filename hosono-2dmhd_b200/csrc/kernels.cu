@@ -303,9 +303,9 @@ __device__ __forceinline__ void p1_release(P1Ctl* ctl) {
 // one face (both sides, every quadrature point); returns the side verdict bits
 // (1 left, 2 right; P1_REST: the columns of the variables the mode leaves out
 // hold fluxes too, as an IEEE solve of a point gave them).
-// Points go in pairs: one sweep of GP sums gives both, the second's states wait
-// in this thread's column of shared memory (park[k * NTHREADS]) while the first
-// is solved.  The Gauss sum of the fluxes accumulates in another column
+// PARK: points go in pairs: one sweep of GP sums gives both, the second's states
+// wait in this thread's column of shared memory (park[k * NTHREADS]) while the
+// first is solved; else one by one.  The Gauss sum of the fluxes accumulates in another column
 // (acc[v * NTHREADS]), which keeps it out of the registers the Riemann solver
 // needs.  dir is a run-time value: the kernel holds one copy of the Riemann
 // solver for both face directions, which halves its instruction footprint; the
@@ -318,7 +318,7 @@ static __device__ __noinline__ void pass1_rest(double* Fo, long long sw, long lo
             Fo[v * plane + (v == MOMN || v == MAGN ? sw : v == MOMT || v == MAGT ? -sw : 0)] = acc[v * NTHREADS];
     if (!Solve<MODE>::var(MAGT)) *ct = acc[MAGT * NTHREADS];
 }
-template <int R, int MODE>
+template <int R, int MODE, bool PARK>
 __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __restrict__ sU,
                                               const double* __restrict__ sPv, int sx, int sy, int dir, bool needL,
                                               bool needR, bool doFlux, long long c, double* acc, double* park,
@@ -337,10 +337,10 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
     for (int v = 0; v < NCONS; v++)
         if (S::var(v)) acc[v * NTHREADS] = 0.0;
 #pragma unroll 1
-    for (int q0 = 0; q0 < NQ; q0 += 2) {
-        const bool pair = q0 + 1 < NQ;
+    for (int q0 = 0; q0 < NQ; q0 += PARK ? 2 : 1) {
+        const bool pair = PARK && q0 + 1 < NQ;
         double uL[NCONS], uR[NCONS];
-        if ((NQ & 1) && !pair) {
+        if (!PARK || ((NQ & 1) && !pair)) {
             double u[1][2][NCONS];
             if (x)
                 gp_face_s<R, MODE, true, 1>(base, swap, pvL + NS * q0, pvR + NS * q0, u);
@@ -367,7 +367,7 @@ __device__ __forceinline__ uint8_t pass1_face(const InstDev& d, const double* __
                 park[k++ * NTHREADS] = u[1][1][v];
             }
         }
-        if (last && q0 + 2 >= NQ) p1_release<R>(ctl);  // this thread's last read of the box
+        if (last && q0 + (PARK ? 2 : 1) >= NQ) p1_release<R>(ctl);  // this thread's last read of the box
 #pragma unroll 1
         for (int q = q0;;) {
             bool admL = true, admR = true;
@@ -438,7 +438,7 @@ struct P1Cell {
     int dir0, dir1;  // its faces: the x-face, the y-face or both
     int box, pv, acc, ctl;  // offsets in doubles (ctl: 0 where the block stages itself)
 };
-template <int R, int MODE>
+template <int R, int MODE, bool PARK>
 static __device__ __noinline__ void pass1_tile(P1Cell c) {
     extern __shared__ __align__(128) double smem[];
     using Box = P1Box<R>;
@@ -467,7 +467,7 @@ static __device__ __noinline__ void pass1_tile(P1Cell c) {
         const bool x = dir == XDIR;
         if (i >= clo && i <= cxhi + (x ? 1 : 0) && j >= clo && j <= cyhi + (x ? 0 : 1)) {
             const int a = x ? i : j, ahi = x ? cxhi : cyhi;
-            const uint8_t bits = pass1_face<R, MODE>(d, smem + c.box, smem + c.pv, sx, sy, dir, a - 1 >= clo, a <= ahi,
+            const uint8_t bits = pass1_face<R, MODE, PARK>(d, smem + c.box, smem + c.pv, sx, sy, dir, a - 1 >= clo, a <= ahi,
                                                      inF, cc, smem + c.acc, smem + c.acc + NCONS * NTHREADS, ctl,
                                                      dir == c.dir1);
             if (bits & 1) pass1_fail(d.fail, c.failList, &c.S->cFail, (int)(x ? cc - 1 : cc - G.pitch));
@@ -495,7 +495,7 @@ __device__ __forceinline__ bool rows_nonzero(const double* sU, int plane, int ro
 // u: the unit, of which a tile has 1 << sh.  Whole tiles (sh = 0): a warp takes
 // a row, its x-faces, then its y-faces.  Smaller units: a warp takes one
 // direction of a row, so a unit has 8 >> sh rows on twice as many warps.
-template <int R, bool SPEC>
+template <int R, bool SPEC, bool PARK>
 __device__ __forceinline__ void pass1_tile_any(const Batch& B, int u, int sh, const double* sU, int pv, int acc, int ctl) {
     extern __shared__ __align__(128) double smem[];
     static_assert(TILE_X == 32, "a tile row is a warp");
@@ -524,16 +524,16 @@ __device__ __forceinline__ void pass1_tile_any(const Batch& B, int u, int sh, co
     const bool z = !SPEC || rows_nonzero<R>(sU, MOMZ, c.row);
     if (d.phys.force_hydro) {
         if (rows_nonzero<R>(sU, MAGX, c.row) || rows_nonzero<R>(sU, MAGY, c.row) || rows_nonzero<R>(sU, MAGZ, c.row))
-            pass1_tile<R, SOLVE_HYDRO_FIELD>(c);
+            pass1_tile<R, SOLVE_HYDRO_FIELD, PARK>(c);
         else if (z)
-            pass1_tile<R, SOLVE_HYDRO>(c);
+            pass1_tile<R, SOLVE_HYDRO, PARK>(c);
         else if (SPEC)
-            pass1_tile<R, SOLVE_HYDRO_PLANAR>(c);
+            pass1_tile<R, SOLVE_HYDRO_PLANAR, PARK>(c);
     } else {
         if (z || rows_nonzero<R>(sU, MAGZ, c.row))
-            pass1_tile<R, SOLVE_MHD>(c);
+            pass1_tile<R, SOLVE_MHD, PARK>(c);
         else if (SPEC)
-            pass1_tile<R, SOLVE_MHD_PLANAR>(c);
+            pass1_tile<R, SOLVE_MHD_PLANAR, PARK>(c);
     }
 }
 
@@ -701,27 +701,31 @@ static __device__ __noinline__ void p1_refill(P1Ctl* ctl) {
 // 0.3 on the tile's barrier, 0.3 on instruction fetch.  Before the shared sweeps,
 // face coordinates and zero planes: 0.720 ms, 1,058 of 2,183 instructions.
 constexpr int P1_HALF = 2;             // half-tile units below this many whole tiles per block
-constexpr int P1_THREAD = 3 * NCONS;  // doubles of shared memory per thread: accumulators, parked face states
-template <int R>
+// The parked states take 32 KB a block, which only two blocks an SM with one box
+// each can spare: three or four blocks, or two boxes, keep the accumulators alone
+// (pairs gain 1.7 % at Orszag-Tang 1024^2 R=2; four blocks cut to two by them cost 25 %).
+constexpr bool p1_park(int minb, int nbuf) { return minb == 2 && nbuf == 1; }
+template <int R, int MINB, int NBUF>
 struct P1Smem {  // dynamic shared memory layout (doubles): boxes, per-thread columns, prediction vectors, mbarriers
-    static constexpr int box(int nbuf) { return nbuf * P1Box<R>::DOUBLES; }
-    static constexpr int bytes(int nbuf) {
-        return ctl(nbuf) * (int)sizeof(double) + (int)sizeof(P1Ctl);
-    }
-    static constexpr int ctl(int nbuf) {  // the control block, after the two mbarriers
-        return nbuf * P1Box<R>::DOUBLES + P1_THREAD * NTHREADS + nbuf * P1Box<R>::PVN + 2;
-    }
+    static constexpr int THREAD = (p1_park(MINB, NBUF) ? 3 : 1) * NCONS;  // accumulators, parked face states
+    static constexpr int BOX = NBUF * P1Box<R>::DOUBLES;
+    static constexpr int CTL = BOX + THREAD * NTHREADS + NBUF * P1Box<R>::PVN + 2;  // after the two mbarriers
+    static constexpr int BYTES = CTL * (int)sizeof(double) + (int)sizeof(P1Ctl);
+    // the blocks an SM's 228 KB hold, 1 KB of each block's own: MINB, but three of four at R = 3
+    static constexpr int BLOCKS = MINB < 228 * 1024 / (BYTES + 1024) ? MINB : 228 * 1024 / (BYTES + 1024);
+    static_assert(BLOCKS == (R == 3 && MINB == 4 ? 3 : MINB), "the blocks an SM is compiled for do not fit");
 };
 template <int R, bool TMA, bool DYN, int MINB, int NBUF>
 __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin) { PDL_ENTRY();
     static_assert(NBUF == 1 || NBUF == 2, "one or two stencil boxes");
-    constexpr bool SPEC = TMA && MINB == 2 && NBUF == 1;
+    constexpr bool PARK = p1_park(MINB, NBUF), SPEC = TMA && PARK;
+    using Smem = P1Smem<R, MINB, NBUF>;
     extern __shared__ __align__(128) double smem[];
     __shared__ int sTile;  // the dynamic schedule's tile, as thread 0 took it
     using Box = P1Box<R>;
     const int tid = threadIdx.y * TILE_X + threadIdx.x;
-    const int acc = P1Smem<R>::box(NBUF) + tid;
-    double* pvBuf = smem + P1Smem<R>::box(NBUF) + P1_THREAD * NTHREADS;  // NBUF prediction-vector buffers
+    const int acc = Smem::BOX + tid;
+    double* pvBuf = smem + Smem::BOX + Smem::THREAD * NTHREADS;  // NBUF prediction-vector buffers
     uint64_t* bars = reinterpret_cast<uint64_t*>(pvBuf + NBUF * Box::PVN);
     if (!(B.flags->radii & (1 << R))) return;  // no instance of this radius
     if (TMA) {
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             pass1_stage<R>(B, uin, t, smem, pvBuf, tid);
             cp_async_wait<0>();
             __syncthreads();  // tile t's box is in place for every thread
-            pass1_tile_any<R, SPEC>(B, t, 0, smem, (int)(pvBuf - smem), acc, 0);
+            pass1_tile_any<R, SPEC, PARK>(B, t, 0, smem, (int)(pvBuf - smem), acc, 0);
             __syncthreads();  // every read of this box is done before it is refilled
             t = next_tile(t + gridDim.x);
         }
@@ -762,7 +766,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
     if constexpr (NBUF == 1 && TMA) {  // one box, refilled by the last thread that reads it
         // A thread that finds the box of its turn in place knows that every
         // thread has released the one before: the copy needs no block barrier.
-        constexpr int CTL = P1Smem<R>::ctl(1);
+        constexpr int CTL = Smem::CTL;
         P1Ctl* ctl = reinterpret_cast<P1Ctl*>(smem + CTL);
         // Fewer tiles than two rounds of the grid: smaller units, so that more
         // SMs work and the last round is shorter (us per launch, whole tiles ->
@@ -788,7 +792,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             // the next turn's unit, before this thread releases the box
             if (tid == 0)
                 ctl->next[(turn + 1) & 1] = DYN ? pass1_take<R>(B, nu, sh) : pass1_next<R>(B, t + gridDim.x, nu, sh);
-            pass1_tile_any<R, SPEC>(B, t, sh, smem, (int)(pvBuf - smem), acc, CTL);
+            pass1_tile_any<R, SPEC, PARK>(B, t, sh, smem, (int)(pvBuf - smem), acc, CTL);
         }
     }
     int t = next_tile(B.p1First + blockIdx.x);
@@ -822,7 +826,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) k_face_pass1(Batch B, int uin)
             }
         }
         __syncthreads();  // tile t's box is in place for every thread
-        pass1_tile_any<R, SPEC>(B, t, 0, smem + buf * Box::DOUBLES, (int)(pvBuf - smem) + buf * Box::PVN, acc, 0);
+        pass1_tile_any<R, SPEC, PARK>(B, t, 0, smem + buf * Box::DOUBLES, (int)(pvBuf - smem) + buf * Box::PVN, acc, 0);
         __syncthreads();  // every read of this box is done before it is refilled
         buf ^= 1;
         t = tn;
@@ -2339,24 +2343,24 @@ void l_step_end(const Batch& B, cudaGraphConditionalHandle h, int turn, cudaStre
     lk(k_step_end, dim3(1), dim3(128), 0, s, B, h, (int)(h != 0), turn);
 }
 // dynamic shared memory of a pass-1 kernel variant
-template <int R, int NBUF>
+template <int R, int MINB, int NBUF>
 constexpr int pass1_smem() {
-    return P1Smem<R>::bytes(NBUF);
+    return P1Smem<R, MINB, NBUF>::BYTES;
 }
 template <int R, bool TMA, bool DYN, int MINB, int NBUF>
 int pass1_grid(int maxTiles) {
     static const bool attr =  // once per process (thread-safe static initialisation)
         cudaFuncSetAttribute((const void*)k_face_pass1<R, TMA, DYN, MINB, NBUF>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, pass1_smem<R, NBUF>()) == cudaSuccess;
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, pass1_smem<R, MINB, NBUF>()) == cudaSuccess;
     (void)attr;
-    const int r = resident_blocks((const void*)k_face_pass1<R, TMA, DYN, MINB, NBUF>, pass1_smem<R, NBUF>());
+    const int r = resident_blocks((const void*)k_face_pass1<R, TMA, DYN, MINB, NBUF>, pass1_smem<R, MINB, NBUF>());
     const int units = TMA && NBUF == 1 && maxTiles < r ? 4 * maxTiles : maxTiles;  // few tiles go in quarters
     return r < units ? r : units;
 }
 template <int R, bool TMA, bool DYN, int MINB, int NBUF>
 void launch_pass1_v(const Batch& B, int uin, cudaStream_t s) {
     lk(k_face_pass1<R, TMA, DYN, MINB, NBUF>, dim3((unsigned)pass1_grid<R, TMA, DYN, MINB, NBUF>(B.maxTiles)), kTile,
-       (size_t)pass1_smem<R, NBUF>(), s, B, uin);
+       (size_t)pass1_smem<R, MINB, NBUF>(), s, B, uin);
 }
 // the variant the tuning asks for: TMA staging and two boxes only with two
 // blocks per SM
