@@ -856,6 +856,7 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
         tr0 = tr1;
     }
     CUE(cudaGetLastError());
+    launches -= radii_held();  // counted with the graph's, which lacks this stage's pass 1
     CUE(cudaGraphLaunch(gAdvRest_, s_));
     if (int rc = check_errors()) return restore_v(rc);
     return download(slot, U, V, nullptr);

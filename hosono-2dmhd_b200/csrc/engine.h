@@ -103,7 +103,9 @@ struct InstState {
     int passes;      // MOOD passes in the current stage
     int passCap;     // pass limit of a stage (HOSONO_MOOD_CAP_DEFAULT, or set by the caller)
     int maxPasses, stages, cascadeIters, passesTotal;
-    int chainPasses, chainIters;  // of passesTotal / cascadeIters: those the kernel chain ran
+    // what the kernel chain ran: ends of pass 1, later passes, face cascades of
+    // pass 1, cascade iterations of pass 1 and of later passes
+    int chainStages, chainPasses, chainCasc, chainIters[2];
     long long innerTotal, detectTotal;
     unsigned long long cflbits[2];
 };

@@ -42,13 +42,20 @@ hosono_stats stats_delta(const InstState& a, const InstState& b) {
     return s;
 }
 
-// kernels one graph execution launched, from the work counters: per step the
-// step end and 3 RK kernels, per run 3 to begin its first step (a host dt
-// needs none); per stage the two cluster kernels, the update and one pass-1 kernel per GP radius held;
-// what the kernel chain ran: 4 per face-cascade iteration, 11 per pass.
-long long graph_launches(const InstState& a, const InstState& b, int steps, bool host_dt, int radii) {
-    return (long long)steps * 4 + (host_dt ? 0 : 3) + (3LL + radii) * (b.stages - a.stages) +
-           4LL * (b.chainIters - a.chainIters) + 11LL * (b.chainPasses - a.chainPasses);
+// kernels the step graphs launched from state a to b, from the work counters:
+// per step the step end and 3 RK kernels, 3 to begin a run's first step (a
+// profiled run's every step; a host dt needs none); per stage one pass-1 kernel
+// per GP radius held, the update and the two cluster kernels (the first alone
+// with the persistent later passes); what the kernel chain ran: per face cascade
+// of pass 1 three, per iteration of one four, per end of pass 1 three, per later
+// pass 11 (the persistent form: one for all of a stage's).
+long long graph_launches(Engine& e, const InstState& a, const InstState& b, int steps, int begins) {
+    const bool persistent = e.tuning().later_passes == HOSONO_LATER_PERSISTENT;
+    const int ends = b.chainStages - a.chainStages;
+    return 4LL * steps + 3LL * begins + (long long)(e.radii_held() + (persistent ? 2 : 3)) * (b.stages - a.stages) +
+           3LL * (b.chainCasc - a.chainCasc) + 4LL * (b.chainIters[0] - a.chainIters[0]) + 3LL * ends +
+           (persistent ? (long long)ends
+                       : 4LL * (b.chainIters[1] - a.chainIters[1]) + 11LL * (b.chainPasses - a.chainPasses));
 }
 
 }  // namespace
@@ -100,7 +107,7 @@ int hosono_gpu_advance(hosono_handle* h, double dt) {
     if (!rc) rc = h->eng.state(h->slot, &b);
     if (!rc) {
         h->stats = stats_delta(a, b);
-        if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(a, b, 1, true, h->eng.radii_held());
+        if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(h->eng, a, b, 1, 0);
     }
     return rc;
 }
@@ -138,7 +145,8 @@ int hosono_gpu_step(hosono_handle* h, int max_steps, double* t_out, int* nstep_o
     rc = h->eng.state(h->slot, &b);
     if (rc) return rc;
     h->stats = stats_delta(a, b);
-    if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(a, b, b.nstep - a.nstep, false, h->eng.radii_held());
+    const int steps = b.nstep - a.nstep;
+    if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(h->eng, a, b, steps, h->profile ? steps : 1);
     if (t_out) *t_out = b.t;
     if (nstep_out) *nstep_out = b.nstep;
     return HOSONO_OK;
@@ -159,7 +167,7 @@ int hosono_gpu_advance_host(hosono_handle* h, double dt, double* U, double* V) {
     if (!rc) rc = h->eng.state(h->slot, &b);
     if (!rc) {
         h->stats = stats_delta(a, b);
-        if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(a, b, 1, true, h->eng.radii_held());
+        if (h->eng.use_graphs && !h->eng.trace) h->eng.launches += graph_launches(h->eng, a, b, 1, 0);
     }
     return rc;
 }

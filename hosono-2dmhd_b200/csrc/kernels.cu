@@ -898,9 +898,10 @@ __device__ __forceinline__ void d_cascade_cond(const Batch& B, int tid, cudaGrap
         S.anyFail = 0;
         S.nextIter = in;
         if (in) {
+            if (S.passes == 0 && !S.cascaded) S.chainCasc++;
             S.cascaded = 1;
             S.cascadeIters++;
-            S.chainIters++;
+            S.chainIters[S.passes > 0]++;
             any = 1;
         }
     }
@@ -1868,7 +1869,10 @@ __device__ __forceinline__ void d_pass_end(const Batch& B, int tid, cudaGraphCon
         if (flip && pass_lowered(S)) S.schemeSel = 1 - S.schemeSel;  // k_mood_flags wrote the other buffer
         S.passes++;
         S.passesTotal++;
-        S.chainPasses++;
+        if (flip)
+            S.chainStages++;
+        else
+            S.chainPasses++;
         S.innerTotal += S.nInner;
         S.detectTotal += S.nDetect;
         S.lastInner = S.nInner;
