@@ -804,6 +804,9 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
             launches++;
             write_field(slot, &InstState::stepping, 0);
         }
+        // U may be pinned, and the caller's again: no copy of it is left
+        if (sCopy_) cudaStreamSynchronize(sCopy_);
+        cudaStreamSynchronize(s_);
         err = rc;
         msg = m;
         return rc;
