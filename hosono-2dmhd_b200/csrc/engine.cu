@@ -1084,9 +1084,9 @@ int Engine::record_chain(Rec& r, const Batch& B, int uin, int uout, Cascade& cas
 int Engine::record_begin(Rec& r) {
     const Batch B = batch();
     const KernelSet* K = K_;
-    TRYE(r.k([&](cudaStream_t s) { K->step_prepare(B, 0, s); }));
+    TRYE(r.k([&](cudaStream_t s) { K->step_prepare(B, s); }));
     TRYE(r.k([&](cudaStream_t s) { K->cfl_reduce(B, s); }));
-    return r.k([&](cudaStream_t s) { K->step_begin(B, 0, s); });
+    return r.k([&](cudaStream_t s) { K->step_begin(B, s); });
 }
 int Engine::record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_cond, bool profile, bool first_head) {
     const Batch B = batch();

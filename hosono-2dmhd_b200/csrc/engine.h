@@ -222,8 +222,8 @@ struct KernelSet {
     const char* name;
     // time loop: per-instance step begin (cfl -> validated dt) and end
     void (*cfl_reduce)(const Batch&, cudaStream_t);
-    void (*step_prepare)(const Batch&, int steps, cudaStream_t);
-    void (*step_begin)(const Batch&, int use_host_dt, cudaStream_t);
+    void (*step_prepare)(const Batch&, cudaStream_t);
+    void (*step_begin)(const Batch&, cudaStream_t);
     // turn: the next step begins here too (its CFL maxima came with rk_final)
     void (*step_end)(const Batch&, cudaGraphConditionalHandle run_cond, int turn, cudaStream_t);
     // forward-Euler stage

@@ -90,10 +90,6 @@ __device__ __forceinline__ int active_tile(const Batch& B, int v) { return range
     for (int v_ = blockIdx.x, nv_ = (B).actInfo[1], t = 0; v_ < nv_; v_ += gridDim.x)      \
         for (bool once_ = (t = active_tile((B), v_), true); once_; once_ = false)
 
-
-// the one thread per instance that owns cell (0,0) (every instance has a tile at its origin)
-__device__ __forceinline__ bool first_tile_thread(const Cell& c) { return c.i == 0 && c.j == 0; }
-
 // GP prediction at quadrature point q of face f of cell (i,j), radius RR:
 // sum_k pv(k,q,f,RR) * U(:, stencil_k), stencil order k=1..ns
 // (reconstruct.f90:109-124; stencil order of GP.f90:85-95).
@@ -2112,8 +2108,7 @@ __device__ __forceinline__ void step_begin(const InstDev& d, InstState& S) {
     S.dtdx = dt / d.geo.dx;
     S.dtdy = dt / d.geo.dy;
 }
-__global__ void k_step_begin(Batch B, int use_host_dt) { PDL_ENTRY();
-    if (use_host_dt) return;  // the host already stored dt
+__global__ void k_step_begin(Batch B) { PDL_ENTRY();
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
         if (!S.stepping) continue;
@@ -2125,7 +2120,7 @@ __global__ void k_step_begin(Batch B, int use_host_dt) { PDL_ENTRY();
 
 // Step start: which instances take part, fresh CFL accumulators.  (The step
 // budget flags->stepsLeft is set by the host before each run launch.)
-__global__ void k_step_prepare(Batch B, int /*unused*/) { PDL_ENTRY();
+__global__ void k_step_prepare(Batch B) { PDL_ENTRY();
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
         S.stepping = (S.live && !S.done && !B.hold[k]) ? 1 : 0;
@@ -2341,8 +2336,8 @@ void lk(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t
     lk(kern, dim3((unsigned)resident_blocks((const void*)kern)), dim3(256), 0, s, B, ##__VA_ARGS__)
 
 void l_cfl_reduce(const Batch& B, cudaStream_t s) { TILE_LAUNCH(k_cfl_reduce, B, s); }
-void l_step_prepare(const Batch& B, int steps, cudaStream_t s) { lk(k_step_prepare, dim3(1), dim3(128), 0, s, B, steps); }
-void l_step_begin(const Batch& B, int use_host_dt, cudaStream_t s) { lk(k_step_begin, dim3(1), dim3(128), 0, s, B, use_host_dt); }
+void l_step_prepare(const Batch& B, cudaStream_t s) { lk(k_step_prepare, dim3(1), dim3(128), 0, s, B); }
+void l_step_begin(const Batch& B, cudaStream_t s) { lk(k_step_begin, dim3(1), dim3(128), 0, s, B); }
 void l_step_end(const Batch& B, cudaGraphConditionalHandle h, int turn, cudaStream_t s) {
     lk(k_step_end, dim3(1), dim3(128), 0, s, B, h, (int)(h != 0), turn);
 }
