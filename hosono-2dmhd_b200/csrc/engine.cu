@@ -214,7 +214,7 @@ Engine::~Engine() {
     for (cudaEvent_t ev : bandEv_)
         if (ev) cudaEventDestroy(ev);
     if (sCopy_) cudaStreamDestroy(sCopy_);
-    for (void* p : {(void*)d_instTiles_, (void*)d_actRange_, (void*)d_actInfo_, (void*)d_casRange_,
+    for (void* p : {(void*)d_instTiles_, (void*)d_mcSlots_, (void*)d_actRange_, (void*)d_actInfo_, (void*)d_casRange_,
                     (void*)d_casInfo_, (void*)d_hold_, (void*)d_gbar_})
         if (p) cudaFree(p);
     for (void* p : {(void*)d_dev_, (void*)d_st_, (void*)d_tiles_, (void*)d_ntiles_, (void*)d_flags_, (void*)staging_,
@@ -240,6 +240,7 @@ int Engine::init(int max_inst, int max_tiles, int fp_mode) {
     CUE(cudaMalloc(&d_st_, sizeof(InstState) * maxInst_));
     CUE(cudaMalloc(&d_tiles_, sizeof(int4) * maxTiles_));
     CUE(cudaMalloc(&d_instTiles_, sizeof(int2) * maxInst_));
+    CUE(cudaMalloc(&d_mcSlots_, sizeof(int) * maxInst_));
     CUE(cudaMalloc(&d_actRange_, sizeof(int2) * maxInst_));
     CUE(cudaMalloc(&d_actInfo_, sizeof(int) * 2));
     CUE(cudaMalloc(&d_casRange_, sizeof(int2) * maxInst_));
@@ -252,6 +253,9 @@ int Engine::init(int max_inst, int max_tiles, int fp_mode) {
     CUE(cudaMemsetAsync(d_instTiles_, 0, sizeof(int2) * maxInst_, s_));
     CUE(cudaMemsetAsync(d_actInfo_, 0, sizeof(int) * 2, s_));
     instTiles_.assign(maxInst_, make_int2(0, 0));
+    mcSlots_.assign(maxInst_, -1);
+    CUE(cudaMemcpyAsync(d_mcSlots_, mcSlots_.data(), sizeof(int) * maxInst_, cudaMemcpyHostToDevice, s_));
+    mcCount_ = clusters_for(0, maxInst_);
     CUE(cudaMalloc(&d_ntiles_, sizeof(int)));
     CUE(cudaMalloc(&d_flags_, sizeof(BatchFlags)));
     lists_.cap = (long long)maxTiles_ * TILE_X * TILE_Y;
@@ -478,6 +482,8 @@ Batch Engine::batch() const {
     B.p1Init = 1;
     B.mcMax = trace || tune_.later_passes == HOSONO_LATER_PERSISTENT ? -1 : kClusterCells;
     B.mcBlocks = mcBlocks_;
+    B.mcCount = mcCount_;
+    B.mcSlots = mcCount_ < maxInst_ ? d_mcSlots_ : nullptr;
     B.ctStaged = tune_.update_staging == HOSONO_STAGE_TMA ? 1 : 0;
     B.dev = d_dev_;
     B.st = d_st_;
@@ -533,31 +539,40 @@ size_t Engine::instance_bytes(const hosono_params& p) const {
 int Engine::upload_tables() {
     tiles_.clear();
     radii_ = 0;
+    int live = 0;
     for (int k = 0; k < maxInst_; k++) {
         instTiles_[k] = make_int2((int)tiles_.size(), 0);
         if (!slots_[k].live) continue;
+        mcSlots_[live++] = k;
         const Geo& G = slots_[k].dev.geo;
         radii_ |= 1 << G.R;
         for (int y = 0; y < G.nyt; y += TILE_Y)
             for (int x = 0; x < G.nxt; x += TILE_X) tiles_.push_back(make_int4(k, x, y, 0));
         instTiles_[k].y = (int)tiles_.size() - instTiles_[k].x;
     }
+    std::fill(mcSlots_.begin() + live, mcSlots_.end(), -1);
     if ((int)tiles_.size() > maxTiles_) return fail(HOSONO_EINVAL, "tile capacity exceeded");
     const int n = (int)tiles_.size();
     if (n) CUE(cudaMemcpyAsync(d_tiles_, tiles_.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(d_ntiles_, &n, sizeof(int), cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(&d_flags_->radii, &radii_, sizeof(int), cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(d_instTiles_, instTiles_.data(), sizeof(int2) * maxInst_, cudaMemcpyHostToDevice, s_));
+    CUE(cudaMemcpyAsync(d_mcSlots_, mcSlots_.data(), sizeof(int) * maxInst_, cudaMemcpyHostToDevice, s_));
     CUE(cudaStreamSynchronize(s_));
     // the graphs launch pass 1 for the radii held when they were recorded:
     // a new radius needs new graphs
     if (radii_ & ~graphRadii_) drop_graphs();
-    // ... and so does another cluster size; a larger one waits until it would
-    // hold at twice the instances, so that a server's few admissions and
-    // retirements do not record graphs again and again
-    const int live = live_count(), want = cluster_blocks_for(live, sms_);
+    // ... and so does another cluster size or number; a larger size waits until
+    // it would hold at twice the instances, a smaller number until a quarter
+    // would do, so that a server's few admissions and retirements do not record
+    // graphs again and again
+    const int want = cluster_blocks_for(live, sms_), count = clusters_for(live, maxInst_);
     if (want < mcBlocks_ || cluster_blocks_for(2 * live, sms_) > mcBlocks_) {
         mcBlocks_ = want;
+        drop_graphs();
+    }
+    if (live > mcCount_ || 4 * count <= mcCount_) {
+        mcCount_ = count;
         drop_graphs();
     }
     return HOSONO_OK;

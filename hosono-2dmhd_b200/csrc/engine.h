@@ -168,6 +168,8 @@ struct Batch {
     int p1Init;          // pass 1 also resets the stage's MOOD planes (0: the autotuner's timing launches)
     int mcMax;           // most listed cells the cluster kernels take per instance (-1: everything to the chain)
     int mcBlocks;        // blocks of an instance's cluster where 16 are not taken
+    int mcCount;         // clusters of a launch, and the slots they take in turn (-1: none);
+    const int* mcSlots;  // null: a cluster a slot
     int maxTiles;        // capacity of the tile list
     int maxInst;         // capacity (slots)
     const int2* instTiles;  // per slot: first tile in the tile list, tile count (0: not live)
@@ -183,6 +185,8 @@ struct Batch {
     int2* casRange;
     int* casInfo;
 };
+
+__host__ __device__ inline int mc_clusters(const Batch& B) { return B.mcSlots ? B.mcCount : B.maxInst; }
 
 enum : int { MOOD_FLAGS_LISTS = 0, MOOD_FLAGS_DENSE = 1, MOOD_FLAGS_LISTS_CLEAR = 2 };
 

@@ -42,6 +42,14 @@ constexpr int kClusterCells = 800;
 // 4781; 128 of 128^2: 9423 / 8230 / 7876 / 7978 / 8914.
 inline int cluster_blocks_for(int live, int sms) { return 8 * live <= sms ? 8 : 4 * live <= sms ? 4 : 2; }
 
+// Clusters of a launch: a power of two, 16 at least, for the live instances
+// (a cluster a slot, and no list of them, where there are no more slots).
+inline int clusters_for(int live, int slots) {
+    int n = 16;
+    while (n < live) n *= 2;
+    return n < slots ? n : slots;
+}
+
 class Engine {
   public:
     Engine() = default;
@@ -196,12 +204,14 @@ class Engine {
     int maxInst_ = 0, maxTiles_ = 0;
     int sms_ = 148;
     int mcBlocks_ = 8;    // Batch::mcBlocks, for the instances of the committed tile list
+    int mcCount_ = 0;     // Batch::mcCount, likewise
     int radii_ = 0;       // BatchFlags::radii of the committed tile list
     int graphRadii_ = 0;  // radii_ when the step graphs were recorded (their pass-1 launches)
     InstDev* d_dev_ = nullptr;
     InstState* d_st_ = nullptr;
     int4* d_tiles_ = nullptr;
     int2* d_instTiles_ = nullptr;
+    int* d_mcSlots_ = nullptr;  // Batch::mcSlots
     int2* d_actRange_ = nullptr;
     int* d_actInfo_ = nullptr;
     int2* d_casRange_ = nullptr;
@@ -209,6 +219,7 @@ class Engine {
     int* d_hold_ = nullptr;
     unsigned* d_gbar_ = nullptr;
     std::vector<int2> instTiles_;
+    std::vector<int> mcSlots_;
     int* d_ntiles_ = nullptr;
     BatchFlags* d_flags_ = nullptr;
     Lists lists_{};

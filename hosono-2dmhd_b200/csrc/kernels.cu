@@ -2387,7 +2387,7 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
     if (B.p1Radii & (1 << 1)) pass1_form<1>(B).launch(B, uin, s);
     if (B.p1Radii & (1 << 3)) pass1_form<3>(B).launch(B, uin, s);
 }
-// One cluster per instance slot: 16 blocks (a non-portable size, taken where
+// One cluster per slot, or live one (Batch::mcSlots): 16 blocks (a non-portable size, taken where
 // the GPU can place one) for up to nine slots, which fills the GPU, else what
 // the engine chose for its live instances (kClusterCells in engine_host.h).
 // The shared memory a cluster kernel needs is static; 16 blocks take leave.
@@ -2431,7 +2431,7 @@ template <typename... KArgs, typename... Args>
 void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t s, Args... args) {
     pdl_take();  // a cluster launch is never programmatic itself
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(blocks * B.maxInst));
+    cfg.gridDim = dim3((unsigned)(blocks * mc_clusters(B)));
     cfg.blockDim = dim3(MC_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];

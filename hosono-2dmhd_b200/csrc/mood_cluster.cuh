@@ -673,6 +673,11 @@ __device__ __forceinline__ void mc_setup(const Batch& B, int k, int uin, int uou
     }
     __syncthreads();
 }
+// the cluster's slot (-1: none)
+__device__ __forceinline__ int mc_slot(const Batch& B) {
+    const int n = blockIdx.x / cluster_nctaid();
+    return B.mcSlots ? B.mcSlots[n] : n;
+}
 __device__ __forceinline__ McT mc_place() {
     McT t;
     const int rank = blockIdx.x % cluster_nctaid();
@@ -688,7 +693,7 @@ __device__ __forceinline__ McT mc_place() {
 __device__ __forceinline__ void mc_done(const Batch& B, bool left, int* out, cudaGraphConditionalHandle h, int set_handle) {
     if (left) atomicOr(&B.flags->mcBig, 1);
     __threadfence();
-    if (atomicAdd(&B.flags->mcDone, 1) + 1 == B.maxInst) {
+    if (atomicAdd(&B.flags->mcDone, 1) + 1 == mc_clusters(B)) {
         B.flags->mcDone = 0;
         const int any = atomicExch(&B.flags->mcBig, 0);
         *out = any;
@@ -703,12 +708,12 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_faces(Batch B, int uin, 
                                                             int set_handle) { PDL_ENTRY();
     __shared__ Mc m;
     const McT t = mc_place();
-    const int k = blockIdx.x / cluster_nctaid();
+    const int slot = mc_slot(B), k = max(slot, 0);
     InstState& S = B.st[k];
-    const bool on = S.stepping != 0;
+    const bool on = slot >= 0 && S.stepping != 0;
     const bool lead = t.lead;
     bool left = false;
-    if (lead && k == 0) {  // the chain's lists, pass 1's tile counters and the grid barrier start over
+    if (lead && blockIdx.x == 0) {  // the chain's lists, pass 1's tile counters and the grid barrier start over
         for (int w = 0; w < LIST_N; w++) B.L.counts[w] = 0;
         for (int r = 0; r < 4; r++) B.flags->p1Next[r] = 0;
         B.gbar[0] = 0;
@@ -764,9 +769,9 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mood_passes(Batch B, int uin,
     PDL_ENTRY();
     __shared__ Mc m;
     const McT t = mc_place();
-    const int k = blockIdx.x / cluster_nctaid();
+    const int slot = mc_slot(B), k = max(slot, 0);
     InstState& S = B.st[k];
-    const bool on = S.stepping != 0 && (!REST || S.hand);
+    const bool on = slot >= 0 && S.stepping != 0 && (!REST || S.hand);
     const bool lead = t.lead;
     bool left = false;
     if (on) {
