@@ -562,20 +562,26 @@ int Engine::upload_tables() {
     // the graphs launch pass 1 for the radii held when they were recorded:
     // a new radius needs new graphs
     if (radii_ & ~graphRadii_) drop_graphs();
-    // ... and so does another cluster size or number; a larger size waits until
-    // it would hold at twice the instances, a smaller number until a quarter
-    // would do, so that a server's few admissions and retirements do not record
-    // graphs again and again
-    const int want = cluster_blocks_for(live, sms_), count = clusters_for(live, maxInst_);
-    if (want < mcBlocks_ || cluster_blocks_for(2 * live, sms_) > mcBlocks_) {
+    live_ = live;
+    return HOSONO_OK;
+}
+
+// The clusters of the launches to come, for the instances of the committed
+// tile list (asked where they are launched or recorded, so that a server's
+// retirements and the admissions after them count once).  Another size or number
+// needs new graphs; a larger size waits until it would hold at twice the
+// instances, a smaller number until a quarter would do, so that a few instances
+// more or less do not record graphs again and again.
+void Engine::fit_clusters() {
+    const int want = cluster_blocks_for(live_, sms_), count = clusters_for(live_, maxInst_);
+    if (want < mcBlocks_ || cluster_blocks_for(2 * live_, sms_) > mcBlocks_) {
         mcBlocks_ = want;
         drop_graphs();
     }
-    if (live > mcCount_ || 4 * count <= mcCount_) {
+    if (live_ > mcCount_ || 4 * count <= mcCount_) {
         mcCount_ = count;
         drop_graphs();
     }
-    return HOSONO_OK;
 }
 
 // The instances' scalars at rest are mirrored in pinned host memory (h_st_):
@@ -1127,6 +1133,7 @@ int Engine::record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_co
 // blast 64^2, two driver steps of a new handle 11.1 -> 4.6 ms; Orszag-Tang
 // 1024^2 through host buffers 8.4 -> 5.6 ms; 2048^2, two steps 32.7 -> 21.4).
 int Engine::build_graph(cudaGraphExec_t Engine::*which) {
+    fit_clusters();
     if (this->*which) return HOSONO_OK;
     graphRadii_ = radii_;  // a subset of the radii of the graphs there are
     cudaGraph_t g;
@@ -1218,6 +1225,7 @@ int Engine::advance(int slot, double dt) {
         TRYE(build_graph(&Engine::gAdvance_));
         CUE(cudaGraphLaunch(gAdvance_, s_));  // check_errors waits for it
     } else {
+        fit_clusters();
         Rec r(this, nullptr);
         TRYE(record_step(r, STEP_HOST_DT, 0, false));
         CUE(cudaStreamSynchronize(s_));
@@ -1235,6 +1243,7 @@ int Engine::run(int max_steps) {
         TRYE(build_graph(&Engine::gRun_));
         CUE(cudaGraphLaunch(gRun_, s_));  // check_errors waits for it
     } else {
+        fit_clusters();
         Rec r(this, nullptr);
         CUE(cudaStreamSynchronize(s_));
         *h_flags_ = f;

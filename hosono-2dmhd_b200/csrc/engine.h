@@ -167,9 +167,7 @@ struct Batch {
     int ctStaged;        // the pass-1 update reads TMA-staged boxes (1) or the planes (0)
     int p1Init;          // pass 1 also resets the stage's MOOD planes (0: the autotuner's timing launches)
     int mcMax;           // most listed cells the cluster kernels take per instance (-1: everything to the chain)
-    int mcBlocks;        // blocks of an instance's cluster where 16 are not taken
-    int mcCount;         // clusters of a launch, and the slots they take in turn (-1: none);
-    const int* mcSlots;  // null: a cluster a slot
+    int mcBlocks;        // blocks of an instance's cluster (16: or 8, where the GPU cannot place 16)
     int maxTiles;        // capacity of the tile list
     int maxInst;         // capacity (slots)
     const int2* instTiles;  // per slot: first tile in the tile list, tile count (0: not live)
@@ -184,6 +182,10 @@ struct Batch {
     // (built by cascade_cond; the cascade kernels walk only these tiles)
     int2* casRange;
     int* casInfo;
+    // the slots the clusters of a launch take in turn (-1: none), mcCount of
+    // them; null: a cluster a slot
+    const int* mcSlots;
+    int mcCount;
 };
 
 __host__ __device__ inline int mc_clusters(const Batch& B) { return B.mcSlots ? B.mcCount : B.maxInst; }

@@ -33,14 +33,17 @@ struct DeviceAllocator {
 // / 92 / 92 ms.
 constexpr int kClusterCells = 800;
 
-// Blocks of a cluster: 8, or as few as 2 where more instances are live than
-// clusters of that size fit the GPU at once (a block takes an SM).  A pass of
+// Blocks of a cluster: 16 (where the GPU can place a cluster of this
+// non-portable size, else 8), or as few as 2 where more instances are live
+// than clusters of that size fit the GPU at once (a block takes an SM).  A pass of
 // few cells is latency, so a smaller cluster loses less time on it than a second
 // wave of clusters does.  us per step with 8 / 4 / 2 / 1 blocks / none, blasts of
 // 40^2 R=2: 18 of them 742 / 769 / 977 / 1432 / 1527, 36: 1177 / 966 / 1148 / 1617
 // / 1899, 74: 2199 / 1724 / 1475 / 1942 / 2428, 256: 6884 / 4973 / 4140 / 4094 /
 // 4781; 128 of 128^2: 9423 / 8230 / 7876 / 7978 / 8914.
-inline int cluster_blocks_for(int live, int sms) { return 8 * live <= sms ? 8 : 4 * live <= sms ? 4 : 2; }
+inline int cluster_blocks_for(int live, int sms) {
+    return 16 * live <= sms ? 16 : 8 * live <= sms ? 8 : 4 * live <= sms ? 4 : 2;
+}
 
 // Clusters of a launch: a power of two, 16 at least, for the live instances
 // (a cluster a slot, and no list of them, where there are no more slots).
@@ -173,6 +176,7 @@ class Engine {
 
     Batch batch() const;
     int upload_tables();
+    void fit_clusters();
     int write_state_field(int slot, size_t offset, const void* src, size_t n);
     int write_state(int slot, const InstState& st);
     template <typename T>
@@ -203,8 +207,9 @@ class Engine {
     cudaStream_t s_ = nullptr;
     int maxInst_ = 0, maxTiles_ = 0;
     int sms_ = 148;
-    int mcBlocks_ = 8;    // Batch::mcBlocks, for the instances of the committed tile list
-    int mcCount_ = 0;     // Batch::mcCount, likewise
+    int live_ = 0;        // instances of the committed tile list
+    int mcBlocks_ = 16;   // Batch::mcBlocks, Batch::mcCount: what fit_clusters took
+    int mcCount_ = 0;
     int radii_ = 0;       // BatchFlags::radii of the committed tile list
     int graphRadii_ = 0;  // radii_ when the step graphs were recorded (their pass-1 launches)
     InstDev* d_dev_ = nullptr;

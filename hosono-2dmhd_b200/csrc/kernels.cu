@@ -2387,10 +2387,10 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
     if (B.p1Radii & (1 << 1)) pass1_form<1>(B).launch(B, uin, s);
     if (B.p1Radii & (1 << 3)) pass1_form<3>(B).launch(B, uin, s);
 }
-// One cluster per slot, or live one (Batch::mcSlots): 16 blocks (a non-portable size, taken where
-// the GPU can place one) for up to nine slots, which fills the GPU, else what
-// the engine chose for its live instances (kClusterCells in engine_host.h).
-// The shared memory a cluster kernel needs is static; 16 blocks take leave.
+// One cluster per slot, or live one (Batch::mcSlots), of the size the engine
+// chose for its live instances (cluster_blocks_for in engine_host.h).  The shared
+// memory a cluster kernel needs is static; 16 blocks, a non-portable size, take
+// leave.
 template <typename K>
 bool cluster_sixteen(K kernel) {
     if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -2425,7 +2425,7 @@ int cluster_blocks(K kernel, const Batch& B) {
     const auto key = std::make_pair(dev, (const void*)kernel);
     auto it = known.find(key);
     if (it == known.end()) it = known.emplace(key, cluster_sixteen(kernel)).first;
-    return it->second && B.maxInst <= 9 ? 16 : B.mcBlocks;
+    return it->second || B.mcBlocks <= 8 ? B.mcBlocks : 8;
 }
 template <typename... KArgs, typename... Args>
 void lk_cluster(void (*kern)(KArgs...), int blocks, const Batch& B, cudaStream_t s, Args... args) {

@@ -53,6 +53,19 @@ def test_sparse_slots(keep, tmp_par_dir):
     b.close()
 
 
+def _per_step(m, par, tiles, slots):
+    b = m.Batch(slots, tiles)
+    k = b.add_par(par)
+    times = []
+    for _ in range(5):
+        b.set_time(k, 0.0, 1e30)
+        t = time.perf_counter()
+        b.run(max_steps=20)
+        times.append(time.perf_counter() - t)
+    b.close()
+    return statistics.median(times[1:])
+
+
 @pytest.mark.gpu
 def test_spare_slots_cost_little(tmp_par_dir):
     """A step of one small blast among 4,000 slots against one among 20: 1.09
@@ -60,16 +73,14 @@ def test_spare_slots_cost_little(tmp_par_dir):
     m = pkg.load()
     par = parfiles.make(tmp_par_dir, "spare", parfiles.blast(64, 2, p_ratio=100.0))
     tiles = m.Batch.tiles_for(m.par_load(par)[0])
+    assert _per_step(m, par, tiles, 4000) < 1.4 * _per_step(m, par, tiles, 20)
 
-    def per_step(slots):
-        b = m.Batch(slots, tiles)
-        k = b.add_par(par)
-        times = []
-        for _ in range(5):
-            b.set_time(k, 0.0, 1e30)
-            t = time.perf_counter()
-            b.run(max_steps=20)
-            times.append(time.perf_counter() - t)
-        b.close()
-        return statistics.median(times[1:])
-    assert per_step(4000) < 1.4 * per_step(20)
+
+@pytest.mark.gpu
+def test_a_lone_solve_has_the_cluster_of_its_own_handle(tmp_par_dir):
+    """A step of one small blast among 20 slots takes as long as one of a single
+    slot (1.32 times with clusters of eight blocks instead of sixteen)."""
+    m = pkg.load()
+    par = parfiles.make(tmp_par_dir, "lone", parfiles.blast(64, 2, p_ratio=100.0))
+    tiles = m.Batch.tiles_for(m.par_load(par)[0])
+    assert _per_step(m, par, tiles, 20) < 1.16 * _per_step(m, par, tiles, 1)
