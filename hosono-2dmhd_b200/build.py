@@ -19,8 +19,12 @@ LIB = os.path.join(PKG, "libhosono_gpu.so")
 INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# No -split-compile: it cuts the module in either of two ways, by its threads'
+# timing, so one source gave two libraries, whose pass 1 differed by 2 %
+# (Orszag-Tang 2048^2 19.7 or 20.15 ms for three steps, 19.55 without it) and whose fast
+# arithmetic differed in the last bits.  kernels.cu takes 100 s instead of 35.
 NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-I", CSRC,
-               "--expt-relaxed-constexpr", "-split-compile", "0"] + ARCH
+               "--expt-relaxed-constexpr"] + ARCH
 
 
 def nvcc():
