@@ -207,8 +207,7 @@ Engine::~Engine() {
         if (sl.modAlloc) cudaFree(sl.modAlloc);
     }
     if (sCopy_) cudaStreamSynchronize(sCopy_);
-    for (cudaGraphExec_t g : {gAdvance_, gRun_, gProf_, gAdvRest_})
-        if (g) cudaGraphExecDestroy(g);
+    drop_graphs();
     for (cudaEvent_t ev : profEv_)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : bandEv_)
@@ -253,9 +252,9 @@ int Engine::init(int max_inst, int max_tiles, int fp_mode) {
     CUE(cudaMemsetAsync(d_instTiles_, 0, sizeof(int2) * maxInst_, s_));
     CUE(cudaMemsetAsync(d_actInfo_, 0, sizeof(int) * 2, s_));
     instTiles_.assign(maxInst_, make_int2(0, 0));
-    mcSlots_.assign(maxInst_, -1);
-    CUE(cudaMemcpyAsync(d_mcSlots_, mcSlots_.data(), sizeof(int) * maxInst_, cudaMemcpyHostToDevice, s_));
-    mcCount_ = clusters_for(0, maxInst_);
+    CUE(cudaMemsetAsync(d_mcSlots_, 0xff, sizeof(int) * maxInst_, s_));
+    hold_.assign(maxInst_, 0);
+    fit_clusters(1);
     CUE(cudaMalloc(&d_ntiles_, sizeof(int)));
     CUE(cudaMalloc(&d_flags_, sizeof(BatchFlags)));
     lists_.cap = (long long)maxTiles_ * TILE_X * TILE_Y;
@@ -335,11 +334,12 @@ int Engine::encode_tmaps(InstDev& dev) {
 
 void Engine::drop_graphs() {
     if (s_) cudaStreamSynchronize(s_);
-    for (cudaGraphExec_t* g : {&gAdvance_, &gRun_, &gProf_, &gAdvRest_})
-        if (*g) {
-            cudaGraphExecDestroy(*g);
-            *g = nullptr;
-        }
+    for (StepGraphs& c : graphs_)
+        for (cudaGraphExec_t* g : {&c.advance, &c.run, &c.prof, &c.advRest})
+            if (*g) {
+                cudaGraphExecDestroy(*g);
+                *g = nullptr;
+            }
 }
 
 int Engine::set_tuning(const hosono_tuning& t) {
@@ -481,7 +481,7 @@ Batch Engine::batch() const {
     B.p1End = INT_MAX;
     B.p1Init = 1;
     B.mcMax = trace || tune_.later_passes == HOSONO_LATER_PERSISTENT ? -1 : kClusterCells;
-    B.mcBlocks = mcBlocks_;
+    B.mcBlocks = 16 >> mcClass_;
     B.mcCount = mcCount_;
     B.mcSlots = mcCount_ < maxInst_ ? d_mcSlots_ : nullptr;
     B.ctStaged = tune_.update_staging == HOSONO_STAGE_TMA ? 1 : 0;
@@ -539,49 +539,59 @@ size_t Engine::instance_bytes(const hosono_params& p) const {
 int Engine::upload_tables() {
     tiles_.clear();
     radii_ = 0;
-    int live = 0;
     for (int k = 0; k < maxInst_; k++) {
         instTiles_[k] = make_int2((int)tiles_.size(), 0);
         if (!slots_[k].live) continue;
-        mcSlots_[live++] = k;
         const Geo& G = slots_[k].dev.geo;
         radii_ |= 1 << G.R;
         for (int y = 0; y < G.nyt; y += TILE_Y)
             for (int x = 0; x < G.nxt; x += TILE_X) tiles_.push_back(make_int4(k, x, y, 0));
         instTiles_[k].y = (int)tiles_.size() - instTiles_[k].x;
     }
-    std::fill(mcSlots_.begin() + live, mcSlots_.end(), -1);
     if ((int)tiles_.size() > maxTiles_) return fail(HOSONO_EINVAL, "tile capacity exceeded");
     const int n = (int)tiles_.size();
     if (n) CUE(cudaMemcpyAsync(d_tiles_, tiles_.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(d_ntiles_, &n, sizeof(int), cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(&d_flags_->radii, &radii_, sizeof(int), cudaMemcpyHostToDevice, s_));
     CUE(cudaMemcpyAsync(d_instTiles_, instTiles_.data(), sizeof(int2) * maxInst_, cudaMemcpyHostToDevice, s_));
-    CUE(cudaMemcpyAsync(d_mcSlots_, mcSlots_.data(), sizeof(int) * maxInst_, cudaMemcpyHostToDevice, s_));
     CUE(cudaStreamSynchronize(s_));
     // the graphs launch pass 1 for the radii held when they were recorded:
     // a new radius needs new graphs
     if (radii_ & ~graphRadii_) drop_graphs();
-    live_ = live;
     return HOSONO_OK;
 }
 
-// The clusters of the launches to come, for the instances of the committed
-// tile list (asked where they are launched or recorded, so that a server's
-// retirements and the admissions after them count once).  Another size or number
-// needs new graphs; a larger size waits until it would hold at twice the
-// instances, a smaller number until a quarter would do, so that a few instances
-// more or less do not record graphs again and again.
-void Engine::fit_clusters() {
-    const int want = cluster_blocks_for(live_, sms_), count = clusters_for(live_, maxInst_);
-    if (want < mcBlocks_ || cluster_blocks_for(2 * live_, sms_) > mcBlocks_) {
-        mcBlocks_ = want;
+// The clusters of the launches to come, for the number of stepping instances.
+// Each class has its own graphs, so that going back and forth records none; the
+// last one's are for a number of clusters, and recorded anew for a larger or
+// where a quarter would do.
+void Engine::fit_clusters(int stepping) {
+    mcClass_ = cluster_class(stepping, sms_);
+    if (mcClass_ < kClusterClasses - 1) {
+        mcCount_ = std::min(cluster_room(mcClass_, sms_), maxInst_);
+        return;
+    }
+    const int want = clusters_for(stepping, maxInst_);
+    if (stepping > mcMany_ || 4 * want <= mcMany_) {
+        mcMany_ = want;
         drop_graphs();
     }
-    if (live_ > mcCount_ || 4 * count <= mcCount_) {
-        mcCount_ = count;
-        drop_graphs();
-    }
+    mcCount_ = mcMany_;
+}
+// ... for a step of one instance that the host starts
+int Engine::fit_one(int slot) {
+    fit_clusters(1);
+    if (mcCount_ == maxInst_) return HOSONO_OK;
+    std::vector<int> list(mcCount_, -1);
+    list[0] = slot;
+    CUE(cudaMemcpyAsync(d_mcSlots_, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, s_));
+    return HOSONO_OK;
+}
+// instances a run launch would step
+int Engine::going() const {
+    int n = 0;
+    for (int k = 0; k < maxInst_; k++) n += slots_[k].live && !h_st_[k].done && !hold_[k];
+    return n;
 }
 
 // The instances' scalars at rest are mirrored in pinned host memory (h_st_):
@@ -730,6 +740,7 @@ int Engine::add(const hosono_params& p, const double* pv, const double* qw, int*
     st.passCap = HOSONO_MOOD_CAP_DEFAULT(R, p.nx, p.ny);
     TRYE(write_state(k, st));
     CUE(cudaMemsetAsync(d_hold_ + k, 0, sizeof(int), s_));
+    hold_[k] = 0;
     sl.live = true;
     sl.ntiles = tiles_of(p);
     slots_[k] = sl;
@@ -849,7 +860,8 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     st.stepping = 1;
     st.error = 0;
     TRYE(write_state(slot, st));
-    TRYE(build_graph(&Engine::gAdvRest_));
+    TRYE(fit_one(slot));
+    TRYE(build_graph(&StepGraphs::advRest));
     // the copies start once everything before on the main stream is done with the staging buffer
     CUE(cudaEventRecord(bandEv_[HOSONO_UPLOAD_BANDS_MAX], s_));
     CUE(cudaStreamWaitEvent(sCopy_, bandEv_[HOSONO_UPLOAD_BANDS_MAX], 0));
@@ -881,7 +893,7 @@ int Engine::advance_host(int slot, double dt, double* U, double* V) {
     }
     CUE(cudaGetLastError());
     launches -= radii_held();  // counted with the graph's, which lacks this stage's pass 1
-    CUE(cudaGraphLaunch(gAdvRest_, s_));
+    CUE(cudaGraphLaunch(graphs_[mcClass_].advRest, s_));
     if (int rc = check_errors()) return restore_v(rc);
     return download(slot, U, V, nullptr);
 }
@@ -976,6 +988,7 @@ int Engine::download(int slot, double* U, double* V, int* scheme) {
 int Engine::set_holds(const int* holds) {
     CUE(cudaMemcpyAsync(d_hold_, holds, sizeof(int) * maxInst_, cudaMemcpyHostToDevice, s_));
     CUE(cudaStreamSynchronize(s_));
+    hold_.assign(holds, holds + maxInst_);
     return HOSONO_OK;
 }
 
@@ -1132,19 +1145,19 @@ int Engine::record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_co
 // one takes 1.1-1.6 ms of a new handle's first step (all four took 3-4.6 ms:
 // blast 64^2, two driver steps of a new handle 11.1 -> 4.6 ms; Orszag-Tang
 // 1024^2 through host buffers 8.4 -> 5.6 ms; 2048^2, two steps 32.7 -> 21.4).
-int Engine::build_graph(cudaGraphExec_t Engine::*which) {
-    fit_clusters();
-    if (this->*which) return HOSONO_OK;
+int Engine::build_graph(cudaGraphExec_t StepGraphs::*which) {
+    cudaGraphExec_t& exec = graphs_[mcClass_].*which;
+    if (exec) return HOSONO_OK;
     graphRadii_ = radii_;  // a subset of the radii of the graphs there are
     cudaGraph_t g;
     CUE(cudaGraphCreate(&g, 0));
     Rec r(this, g);
     int rc;
-    if (which == &Engine::gAdvance_) {
+    if (which == &StepGraphs::advance) {
         rc = record_step(r, STEP_HOST_DT, 0, false);
-    } else if (which == &Engine::gAdvRest_) {  // the banded upload ran the first stage's pass 1
+    } else if (which == &StepGraphs::advRest) {  // the banded upload ran the first stage's pass 1
         rc = record_step(r, STEP_HOST_DT, 0, false, false);
-    } else if (which == &Engine::gProf_) {
+    } else if (which == &StepGraphs::prof) {
         // one step at the graph's top level: event records are not allowed
         // inside conditional bodies, and pass 1 sits outside the MOOD loops
         rc = record_step(r, STEP_WHOLE, 0, true);
@@ -1161,10 +1174,10 @@ int Engine::build_graph(cudaGraphExec_t Engine::*which) {
         cudaGraphDestroy(g);
         return rc;
     }
-    cudaError_t e = cudaGraphInstantiate(&(this->*which), g, 0);
+    cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        this->*which = nullptr;
+        exec = nullptr;
         return fail(HOSONO_ECUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
     return HOSONO_OK;
@@ -1176,10 +1189,18 @@ int Engine::launch(cudaGraphExec_t g) {
     return HOSONO_OK;
 }
 
-int Engine::check_errors() {
+// what a launch left: the instances' scalars and the batch's flags
+int Engine::fetch() {
     CUE(cudaMemcpyAsync(h_st_, d_st_, sizeof(InstState) * maxInst_, cudaMemcpyDeviceToHost, s_));
     CUE(cudaMemcpyAsync(h_flags_, d_flags_, sizeof(BatchFlags), cudaMemcpyDeviceToHost, s_));
     CUE(cudaStreamSynchronize(s_));
+    return HOSONO_OK;
+}
+int Engine::check_errors() {
+    TRYE(fetch());
+    return errors();
+}
+int Engine::errors() {
     if (h_flags_->error) return fail(h_flags_->error, "a MOOD work list overflowed its capacity");
     if (!instance_errors_fatal) return HOSONO_OK;
     for (int k = 0; k < maxInst_; k++)
@@ -1221,11 +1242,11 @@ int Engine::advance(int slot, double dt) {
     st.stepping = 1;
     st.error = 0;
     TRYE(write_state(slot, st));
+    TRYE(fit_one(slot));
     if (use_graphs && !trace) {
-        TRYE(build_graph(&Engine::gAdvance_));
-        CUE(cudaGraphLaunch(gAdvance_, s_));  // check_errors waits for it
+        TRYE(build_graph(&StepGraphs::advance));
+        CUE(cudaGraphLaunch(graphs_[mcClass_].advance, s_));  // check_errors waits for it
     } else {
-        fit_clusters();
         Rec r(this, nullptr);
         TRYE(record_step(r, STEP_HOST_DT, 0, false));
         CUE(cudaStreamSynchronize(s_));
@@ -1238,21 +1259,31 @@ int Engine::run(int max_steps) {
     f.anyLive = 1;
     f.radii = radii_;
     f.stepsLeft = max_steps > 0 ? max_steps : INT_MAX;
-    CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
     if (use_graphs && !trace) {
-        TRYE(build_graph(&Engine::gRun_));
-        CUE(cudaGraphLaunch(gRun_, s_));  // check_errors waits for it
-    } else {
-        fit_clusters();
-        Rec r(this, nullptr);
-        CUE(cudaStreamSynchronize(s_));
-        *h_flags_ = f;
-        long long it = 0;
-        while (h_flags_->anyLive) {
-            if (++it > (long long)INT_MAX) break;
-            TRYE(record_step(r, STEP_WHOLE, 0, false));
-            TRYE(sync());
-        }
+        // one launch; but where instances are done and those still going are few
+        // enough for larger clusters, it ends and the next one goes on with those
+        // (64 blasts of 128^2 to 512^2 that end after 13 to 302 steps: 4.62 -> 2.86 s)
+        do {
+            fit_clusters(going());
+            f.pauseAt = mcClass_ ? cluster_room(mcClass_ - 1, sms_) : 0;
+            CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
+            TRYE(build_graph(&StepGraphs::run));
+            CUE(cudaGraphLaunch(graphs_[mcClass_].run, s_));
+            TRYE(fetch());  // waits for it
+            f.stepsLeft = h_flags_->stepsLeft;
+        } while (!h_flags_->error && h_flags_->going > 0 && f.stepsLeft > 0);
+        return errors();
+    }
+    fit_clusters(going());
+    CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
+    Rec r(this, nullptr);
+    CUE(cudaStreamSynchronize(s_));
+    *h_flags_ = f;
+    long long it = 0;
+    while (h_flags_->anyLive) {
+        if (++it > (long long)INT_MAX) break;
+        TRYE(record_step(r, STEP_WHOLE, 0, false));
+        TRYE(sync());
     }
     return check_errors();
 }
@@ -1263,8 +1294,9 @@ int Engine::run_profiled_step(double* pass1_ms, int* pass1_launches) {
     f.radii = radii_;
     f.stepsLeft = 1;
     CUE(cudaMemcpyAsync(d_flags_, &f, sizeof f, cudaMemcpyHostToDevice, s_));
-    TRYE(build_graph(&Engine::gProf_));
-    TRYE(launch(gProf_));
+    fit_clusters(going());
+    TRYE(build_graph(&StepGraphs::prof));
+    TRYE(launch(graphs_[mcClass_].prof));
     double ms = 0;
     for (int st = 0; st < 3; st++) {
         float t = 0.f;

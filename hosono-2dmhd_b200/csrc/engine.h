@@ -123,6 +123,8 @@ struct BatchFlags {
     int anyCasc;     // some instance's pass-1 face cascade is left to the kernel chain
     int anyMood;     // some instance's later passes are left to the kernel chain
     int mcDone, mcBig;  // clusters finished in the running cluster launch; whether one left work to the chain
+    int going;       // instances that have steps to make after the last step_end ...
+    int pauseAt;     // ... and how few of them end the run launch (larger clusters then take over)
 };
 
 // Roles of the three U buffers: the state lives in U[parity]; A in
@@ -182,9 +184,9 @@ struct Batch {
     // (built by cascade_cond; the cascade kernels walk only these tiles)
     int2* casRange;
     int* casInfo;
-    // the slots the clusters of a launch take in turn (-1: none), mcCount of
-    // them; null: a cluster a slot
-    const int* mcSlots;
+    // the stepping slots, which the clusters of a launch take in turn (-1: none),
+    // mcCount of them; null: a cluster a slot
+    int* mcSlots;
     int mcCount;
 };
 

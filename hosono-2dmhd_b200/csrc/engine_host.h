@@ -33,25 +33,34 @@ struct DeviceAllocator {
 // / 92 / 92 ms.
 constexpr int kClusterCells = 800;
 
-// Blocks of a cluster: 16 (where the GPU can place a cluster of this
-// non-portable size, else 8), or as few as 2 where more instances are live
-// than clusters of that size fit the GPU at once (a block takes an SM).  A pass of
-// few cells is latency, so a smaller cluster loses less time on it than a second
-// wave of clusters does.  us per step with 8 / 4 / 2 / 1 blocks / none, blasts of
-// 40^2 R=2: 18 of them 742 / 769 / 977 / 1432 / 1527, 36: 1177 / 966 / 1148 / 1617
-// / 1899, 74: 2199 / 1724 / 1475 / 1942 / 2428, 256: 6884 / 4973 / 4140 / 4094 /
-// 4781; 128 of 128^2: 9423 / 8230 / 7876 / 7978 / 8914.
-inline int cluster_blocks_for(int live, int sms) {
-    return 16 * live <= sms ? 16 : 8 * live <= sms ? 8 : 4 * live <= sms ? 4 : 2;
+// Blocks of a cluster: 16 >> class, 16 (where the GPU can place a cluster of this
+// non-portable size, else 8) down to 2 by the number of stepping instances: as
+// many as the GPU holds at once (a block takes an SM), half as many again at four.
+// A pass of few cells is latency, so a smaller cluster loses less time on it than
+// a second wave of clusters does.  us per step with 8 / 4 / 2 / 1 blocks / none,
+// blasts of 40^2 R=2: 18 of them 742 / 769 / 977 / 1432 / 1527, 36: 1177 / 966 / 1148 /
+// 1617 / 1899, 74: 2199 / 1724 / 1475 / 1942 / 2428, 256: 6884 / 4973 / 4140 / 4094 /
+// 4781; 128 of 128^2: 9423 / 8230 / 7876 / 7978 / 8914; with 4 / 2 blocks 40 of 128^2
+// to 512^2 10.3 / 12.6 ms, 64 of them 16.0 / 16.8, 64 of 64^2 2.35 / 2.21.
+constexpr int kClusterClasses = 4;
+inline int cluster_room(int cls, int sms) { return cls == 2 ? 3 * sms / 8 : sms / (16 >> cls); }
+inline int cluster_class(int stepping, int sms) {
+    int c = 0;
+    while (c < kClusterClasses - 1 && stepping > cluster_room(c, sms)) c++;
+    return c;
 }
 
-// Clusters of a launch: a power of two, 16 at least, for the live instances
-// (a cluster a slot, and no list of them, where there are no more slots).
-inline int clusters_for(int live, int slots) {
-    int n = 16;
-    while (n < live) n *= 2;
+// Clusters of a launch of the last class: a power of two (no more than slots).
+inline int clusters_for(int stepping, int slots) {
+    int n = 64;
+    while (n < stepping) n *= 2;
     return n < slots ? n : slots;
 }
+
+struct StepGraphs {
+    cudaGraphExec_t advance = nullptr, run = nullptr, prof = nullptr;
+    cudaGraphExec_t advRest = nullptr;  // advance without the first stage's set-up and pass 1
+};
 
 class Engine {
   public:
@@ -176,7 +185,9 @@ class Engine {
 
     Batch batch() const;
     int upload_tables();
-    void fit_clusters();
+    void fit_clusters(int stepping);
+    int fit_one(int slot);
+    int going() const;
     int write_state_field(int slot, size_t offset, const void* src, size_t n);
     int write_state(int slot, const InstState& st);
     template <typename T>
@@ -191,10 +202,12 @@ class Engine {
     enum StepForm { STEP_HOST_DT, STEP_WHOLE, STEP_TURN };
     int record_begin(Rec& r);
     int record_step(Rec& r, StepForm form, cudaGraphConditionalHandle run_cond, bool profile, bool first_head = true);
-    int build_graph(cudaGraphExec_t Engine::*which);
+    int build_graph(cudaGraphExec_t StepGraphs::*which);
     int launch(cudaGraphExec_t g);
     int sync();
+    int fetch();
     int check_errors();
+    int errors();
     int trace_before_pass();
     int trace_snapshot();
     int trace_after_pass();
@@ -207,9 +220,8 @@ class Engine {
     cudaStream_t s_ = nullptr;
     int maxInst_ = 0, maxTiles_ = 0;
     int sms_ = 148;
-    int live_ = 0;        // instances of the committed tile list
-    int mcBlocks_ = 16;   // Batch::mcBlocks, Batch::mcCount: what fit_clusters took
-    int mcCount_ = 0;
+    int mcClass_ = 0, mcCount_ = 0;  // the launches' cluster_class and number of clusters (fit_clusters)
+    int mcMany_ = 0;                 // the last class's number
     int radii_ = 0;       // BatchFlags::radii of the committed tile list
     int graphRadii_ = 0;  // radii_ when the step graphs were recorded (their pass-1 launches)
     InstDev* d_dev_ = nullptr;
@@ -224,7 +236,7 @@ class Engine {
     int* d_hold_ = nullptr;
     unsigned* d_gbar_ = nullptr;
     std::vector<int2> instTiles_;
-    std::vector<int> mcSlots_;
+    std::vector<int> hold_;  // d_hold_
     int* d_ntiles_ = nullptr;
     BatchFlags* d_flags_ = nullptr;
     Lists lists_{};
@@ -235,8 +247,7 @@ class Engine {
     int* schemeInt_ = nullptr;
     std::vector<Slot> slots_;
     std::vector<int4> tiles_;
-    cudaGraphExec_t gAdvance_ = nullptr, gRun_ = nullptr, gProf_ = nullptr;
-    cudaGraphExec_t gAdvRest_ = nullptr;  // gAdvance_ without the first stage's set-up and pass 1
+    StepGraphs graphs_[kClusterClasses];
     cudaStream_t sCopy_ = nullptr;        // the banded upload's copy stream
     cudaEvent_t bandEv_[HOSONO_UPLOAD_BANDS_MAX + 1] = {};
     cudaEvent_t profEv_[6] = {};

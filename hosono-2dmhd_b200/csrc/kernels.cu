@@ -2118,15 +2118,36 @@ __global__ void k_step_begin(Batch B) { PDL_ENTRY();
     }
 }
 
+// The clusters' list of stepping slots, by one block: each is listed, then the
+// rest of the list cleared (n: 0 before; the host launches clusters enough).
+__device__ __forceinline__ void list_stepping(const Batch& B, int k, int* n) {
+    if (!B.mcSlots) return;
+    const int at = atomicAdd(n, 1);
+    if (at < B.mcCount)
+        B.mcSlots[at] = k;
+    else
+        B.flags->error = HOSONO_EINVAL;
+}
+__device__ __forceinline__ void list_end(const Batch& B, const int* n) {
+    if (!B.mcSlots) return;
+    __syncthreads();
+    for (int e = *n + (int)threadIdx.x; e < B.mcCount; e += blockDim.x) B.mcSlots[e] = -1;
+}
+
 // Step start: which instances take part, fresh CFL accumulators.  (The step
 // budget flags->stepsLeft is set by the host before each run launch.)
 __global__ void k_step_prepare(Batch B) { PDL_ENTRY();
+    __shared__ int n;
+    if (threadIdx.x == 0) n = 0;
+    __syncthreads();
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
         S.stepping = (S.live && !S.done && !B.hold[k]) ? 1 : 0;
         S.cflbits[0] = 0;
         S.cflbits[1] = 0;
+        if (S.stepping) list_stepping(B, k, &n);
     }
+    list_end(B, &n);
 }
 
 // Step end: the new state is buffer A (parity flips), t += dt, nstep += 1,
@@ -2134,8 +2155,8 @@ __global__ void k_step_prepare(Batch B) { PDL_ENTRY();
 // the batch condition.  turn: the run goes on in the same launch, so the next
 // step begins here (its CFL maxima came with rk_final).
 __global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle, int turn) { PDL_ENTRY();
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
+    __shared__ int going, n;
+    if (threadIdx.x == 0) going = n = 0;
     __syncthreads();
     for (int k = threadIdx.x; k < B.maxInst; k += blockDim.x) {
         InstState& S = B.st[k];
@@ -2146,13 +2167,14 @@ __global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle
             if (!((S.t < S.tmax) && (S.nstep < S.nstepmax))) S.done = 1;
         }
         S.stepping = 0;  // at rest between launches; step_prepare picks the next participants
-        if (S.live && !S.done && !B.hold[k]) any = 1;
+        if (S.live && !S.done && !B.hold[k]) atomicAdd(&going, 1);
     }
     __syncthreads();
     __shared__ int go;
     if (threadIdx.x == 0) {
         const int left = --B.flags->stepsLeft;
-        go = any && left > 0;
+        go = going > B.flags->pauseAt && left > 0;
+        B.flags->going = going;
         B.flags->anyLive = go;
         if (set_handle) cudaGraphSetConditional(h, go ? 1u : 0u);
     }
@@ -2162,10 +2184,12 @@ __global__ void k_step_end(Batch B, cudaGraphConditionalHandle h, int set_handle
         if (turn && go && S.live && !S.done && !B.hold[k]) {
             S.stepping = 1;
             step_begin(B.dev[k], S);
+            list_stepping(B, k, &n);
         }
         S.cflbits[0] = 0;
         S.cflbits[1] = 0;
     }
+    if (turn && go) list_end(B, &n);
 }
 
 // ======================================================================
@@ -2387,8 +2411,8 @@ void l_face_pass1(const Batch& B, int uin, cudaStream_t s) {
     if (B.p1Radii & (1 << 1)) pass1_form<1>(B).launch(B, uin, s);
     if (B.p1Radii & (1 << 3)) pass1_form<3>(B).launch(B, uin, s);
 }
-// One cluster per slot, or live one (Batch::mcSlots), of the size the engine
-// chose for its live instances (cluster_blocks_for in engine_host.h).  The shared
+// One cluster per slot, or stepping one (Batch::mcSlots), of the size the engine
+// chose for their number (cluster_class in engine_host.h).  The shared
 // memory a cluster kernel needs is static; 16 blocks, a non-portable size, take
 // leave.
 template <typename K>

@@ -1,6 +1,5 @@
 """Engines with more slots than solves, as a server's is: the solves' clusters
 find their slots wherever they are, and empty slots cost no launches' time."""
-import statistics
 import time
 
 import numpy as np
@@ -63,7 +62,7 @@ def _per_step(m, par, tiles, slots):
         b.run(max_steps=20)
         times.append(time.perf_counter() - t)
     b.close()
-    return statistics.median(times[1:])
+    return min(times[1:])
 
 
 @pytest.mark.gpu
