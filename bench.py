@@ -588,7 +588,7 @@ def load_problems():
 
 def bench_batched(m, fp, torch, manifest="blast64_seed0.json", limit=None, eager=False, tune=True):
     """The 64-instance MHD-blast workload (uneven N in {128..512}) advanced to
-    t_end=0.02 as one batch (one graph launch for the whole run) and, for
+    t_end=0.02 as one batch (up to four graph launches for the whole run) and, for
     comparison, as 64 plain single solves one after the other.  Set-up (host
     initial state, GP tables, upload) and the first step of each (graph
     capture) are outside the timed regions; zone-updates count the timed steps."""

@@ -19,7 +19,8 @@
 //                          mood_passes for instances whose passes got short } }
 //
 // Each loop condition is set on the device by the kernel that ends the loop
-// body (cudaGraphSetConditional), so a whole run is one graph launch.
+// body (cudaGraphSetConditional), so a whole run is one graph launch
+// (a batch's: one for each cluster size it comes down to).
 
 #include "engine_host.h"
 

@@ -313,12 +313,12 @@ int hosono_gpu_stream(hosono_handle* h, void** stream);
 typedef struct hosono_tuning {
     int pass1_staging;        /* HOSONO_STAGE_* */
     int pass1_schedule;       /* HOSONO_SCHED_* */
-    int pass1_blocks_per_sm;  /* resident pass-1 blocks per SM the register budget aims at: 2 (0 = 2;
-                                 128 registers), 3 or 4 (80 / 64 registers, one stencil box per
-                                 block, cp.async staging only) */
+    int pass1_blocks_per_sm;  /* resident pass-1 blocks per SM: 2 (0 = 2; 128 registers), 3 or 4 (80 / 64
+                                 registers, one stencil box per block, cp.async staging only; at
+                                 R = 3 the shared memory holds three of four) */
     int later_passes;         /* HOSONO_LATER_*; the autotuner keeps the caller's choice */
     int pass1_boxes;          /* stencil boxes per pass-1 block at two blocks per SM: 1 (0 = 1; load,
-                                 compute, load the next; the shared memory saved goes to L1) or 2 (the
+                                 compute, load the next; face states of two quadrature points a sweep) or 2 (the
                                  next tile's box loads while the current one is computed) */
     int upload_bands;         /* hosono_gpu_advance_host: row bands of the overlapped upload (0 = by size:
                                  16 from 2048 array rows, 8 from 1024, else 1; 1 = upload, then step;
@@ -336,7 +336,7 @@ int hosono_gpu_get_tuning(hosono_handle* h, hosono_tuning* t);
 
 /* Autotuner.  Times every candidate hosono_tuning on the instances the
  * handle or batch holds now -- `trials` launches of the MOOD pass-1 kernels
- * (83 % of a time step; they only write scratch that every stage rewrites,
+ * (three quarters of a time step; they only write scratch that every stage rewrites,
  * so the solution is untouched) per candidate, after one untimed launch --
  * and applies the fastest.  The choice is kept in a process-wide cache keyed
  * by (arithmetic mode, GP radii present, size class = floor(log2(interior
